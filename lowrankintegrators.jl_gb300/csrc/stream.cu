@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "../../include/lri.h"
+#include "burgers_flow.h"
 #include "core_svd.h"
 #include "engine.cuh"
 #include "tc_kr.h"
@@ -1483,384 +1484,6 @@ __global__ void s_stage_finish(int R, const int32_t* __restrict__ rank, int nz, 
   }
 }
 
-// ---------------------------------------------------------------------------
-// Fused RK stages of the Burgers flows for small active widths (ka <= 32).
-// At low rank each stage of the K, L and S substep flows is row-local work
-// on an n x ka panel plus small matrices (N_nu, A_xx, Z) and the packed flow
-// tensor T' (np x ka, np = ka (ka + 1) / 2 pairs), all of which fit in shared
-// memory; one kernel per stage replaces the stencil, panel product,
-// Khatri-Rao and combine launches above (same arithmetic per entry, sums in
-// a different order).  One CTA per FUSED_BMH rows (K and S flows, with one
-// periodic halo row on each side for the stencils and the Dx of the
-// quadratic term: 32 rows of Khatri-Rao work, one per thread and column
-// group) or FUSED_BML rows (L flow).  The tensor sits pair-major in shared
-// memory, tpt[p kpp + c] with kpp = ka rounded up to 4, plus 4: one 16-byte
-// load (a broadcast across the warp) serves four columns.
-// ---------------------------------------------------------------------------
-constexpr int FUSED_BMH = 30;
-constexpr int FUSED_BML = 64;
-constexpr int FUSED_KMAX = 32;
-
-// Four consecutive columns c0 .. c0 + 3 of one row of
-//   sum_{a <= b} KR(P, Q)_ab T'[p(a,b), c],  KR(P, Q)_ab = (P_a Q_b + P_b Q_a) / 2
-// (SAME: P == Q, KR = P_a P_b); P, Q: the row's ka <= 32 values; T'
-// pair-major in shared memory, tpt[p kpp + c], zero beyond the active
-// columns.  Each 16-byte tensor load serves 4 (8) multiply-adds and is the
-// loop's only shared-memory read; a warp's threads share c0, so the tensor
-// reads are broadcasts.
-template <typename T, int KMAX, bool SAME>
-__device__ __forceinline__ void kr_row4_k(int ka, int kpp, const T* P, const T* Q, const T* tpt, int c0,
-                                          T (&acc)[4]) {
-  // the row's values in registers (zero beyond ka); loops unrolled over the
-  // KMAX x KMAX triangle, pairs beyond ka skipped (ka is uniform)
-  T qv[KMAX], pv[SAME ? 1 : KMAX];
-#pragma unroll
-  for (int k = 0; k < KMAX; ++k) {
-    qv[k] = (k < ka) ? Q[k] : T(0);
-    if (!SAME) pv[SAME ? 0 : k] = (k < ka) ? P[k] : T(0);
-  }
-  const T* tp = tpt + c0;
-#pragma unroll
-  for (int a = 0; a < KMAX; ++a) {
-    if (a < ka) {
-      T g1[4] = {T(0), T(0), T(0), T(0)}, g2[4] = {T(0), T(0), T(0), T(0)};
-#pragma unroll
-      for (int b = a; b < KMAX; ++b) {
-        if (b < ka) {
-          T t[4];
-          ld_vec<4>(tp, t);
-          tp += kpp;
-#pragma unroll
-          for (int v = 0; v < 4; ++v) {
-            g1[v] = fma(qv[b], t[v], g1[v]);
-            if (!SAME) g2[v] = fma(pv[SAME ? 0 : b], t[v], g2[v]);
-          }
-        }
-      }
-#pragma unroll
-      for (int v = 0; v < 4; ++v) {
-        if (SAME) acc[v] = fma(qv[a], g1[v], acc[v]);
-        else acc[v] = fma(T(0.5), fma(pv[SAME ? 0 : a], g1[v], qv[a] * g2[v]), acc[v]);
-      }
-    }
-  }
-}
-template <typename T, bool SAME>
-__device__ __forceinline__ void kr_row4(int ka, int kpp, const T* P, const T* Q, const T* tpt, int c0, T (&acc)[4]) {
-  if (ka <= 16) kr_row4_k<T, 16, SAME>(ka, kpp, P, Q, tpt, c0, acc);
-  else kr_row4_k<T, 32, SAME>(ka, kpp, P, Q, tpt, c0, acc);
-}
-
-// row stride of the pair-major tensor in shared memory
-__host__ __device__ constexpr int tensor_kpp(int kap) { return kap + 4; }
-
-// the packed tensor's active block, pair-major: tpt[p kpp + c] = Tp[p + c PP]
-// for c < ka, zero for ka <= c < kpp (kap = ka rounded up to 4); global
-// reads run along the pairs (coalesced)
-template <typename T>
-__device__ __forceinline__ void load_tensor(int ka, int kap, const T* __restrict__ Tp, int PP, T* tpt) {
-  const int np = ka * (ka + 1) / 2, kpp = tensor_kpp(kap), total = np * kpp;
-  constexpr int U = 8;  // loads in flight per thread
-  for (int e0 = threadIdx.x; e0 < total; e0 += U * blockDim.x) {
-    T v[U];
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int e = e0 + u * blockDim.x;
-      const int pp = e % np, c = e / np;
-      v[u] = (e < total && c < ka) ? Tp[pp + (int64_t)c * PP] : T(0);
-    }
-#pragma unroll
-    for (int u = 0; u < U; ++u) {
-      const int e = e0 + u * blockDim.x;
-      if (e < total) tpt[(e % np) * kpp + e / np] = v[u];
-    }
-  }
-}
-
-// Per-row arrays in shared memory have an odd row stride (ka | 1), and
-// threads run along the rows, so a warp touches 32 distinct banks and its
-// global accesses to a column are coalesced.
-
-// K substep stage: v = (ih2 Dxx Z) N_nu + alpha KR(Dx Z, Z) T'_V + beta Dx(KR(Z, Z) T'_V),
-// Dx = ihx (shift - shift) on the active columns (zero elsewhere), then the RK update.
-template <typename T>
-__global__ void __launch_bounds__(256) burgers_k_stage(int N, int R, const int32_t* __restrict__ rank,
-                                                       const T* __restrict__ Z, const double* __restrict__ Nnu,
-                                                       const T* __restrict__ Tp, int PP, double ih2, double ihx,
-                                                       double alpha, double beta, uint32_t* status, RkStage<T> rk) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int ka = min(R, (int)*rank);
-  if (ka > FUSED_KMAX) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(status, ST_BAD_SHAPE);
-    return;
-  }
-  const int np = ka * (ka + 1) / 2, ld = ka | 1, kap = (ka + 3) & ~3, ncg = kap / 4;
-  const bool nonlin = (alpha != 0.0 || beta != 0.0);
-  T* tpt = reinterpret_cast<T*>(smraw);            // np x kpp
-  T* zs = tpt + (nonlin ? np * tensor_kpp(kap) : 0);  // (BM + 2) x ld: rows i0 - 1 .. i0 + BM
-  T* ks = zs + (FUSED_BMH + 2) * ld;                 // (BM + 2) x ld: KR(Z, Z) T' (kap columns used)
-  T* ns = ks + (FUSED_BMH + 2) * (kap | 1);          // ka x ka: N_nu
-  T* d1 = ns + ka * ka;                             // BM x ld: Dx Z
-  const int ldk = kap | 1;
-  const int i0 = blockIdx.x * FUSED_BMH;
-  if (nonlin) load_tensor(ka, kap, Tp, PP, tpt);
-  for (int e = threadIdx.x; e < (FUSED_BMH + 2) * ka; e += blockDim.x) {
-    const int ii = e % (FUSED_BMH + 2), a = e / (FUSED_BMH + 2);
-    int g = i0 - 1 + ii;
-    g = (g < 0) ? g + N : ((g >= N) ? g - N : g);
-    zs[ii * ld + a] = Z[g + (int64_t)a * N];
-  }
-  for (int e = threadIdx.x; e < ka * ka; e += blockDim.x) ns[e] = T(Nnu[(e % ka) + (int64_t)(e / ka) * R]);
-  __syncthreads();
-  if (beta != 0.0)
-    for (int e = threadIdx.x; e < (FUSED_BMH + 2) * ncg; e += blockDim.x) {
-      const int ii = e % (FUSED_BMH + 2), c0 = 4 * (e / (FUSED_BMH + 2));
-      T acc[4] = {T(0), T(0), T(0), T(0)};
-      kr_row4<T, true>(ka, tensor_kpp(kap), zs + ii * ld, zs + ii * ld, tpt, c0, acc);
-#pragma unroll
-      for (int v = 0; v < 4; ++v) ks[ii * ldk + c0 + v] = acc[v];
-    }
-  for (int e = threadIdx.x; e < FUSED_BMH * ka; e += blockDim.x) {
-    const int ii = e % FUSED_BMH, a = e / FUSED_BMH;
-    d1[ii * ld + a] = T(ihx) * (zs[(ii + 2) * ld + a] - zs[ii * ld + a]);
-  }
-  __syncthreads();
-  const int rows = min(FUSED_BMH, N - i0);
-  for (int e = threadIdx.x; e < FUSED_BMH * ncg; e += blockDim.x) {  // active column groups
-    const int ii = e % FUSED_BMH, c0 = 4 * (e / FUSED_BMH);
-    if (ii >= rows) continue;
-    T v[4] = {T(0), T(0), T(0), T(0)};
-    const T* zm = zs + ii * ld;
-    const T* z0 = zm + ld;
-    const T* zp = z0 + ld;
-    for (int a = 0; a < ka; ++a) {
-      const T d2 = T(ih2) * ((zm[a] + zp[a]) - T(2) * z0[a]);
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (c0 + q < ka) v[q] = fma(d2, ns[a + (c0 + q) * ka], v[q]);
-    }
-    if (alpha != 0.0) {
-      T k1[4] = {T(0), T(0), T(0), T(0)};
-      kr_row4<T, false>(ka, tensor_kpp(kap), d1 + ii * ld, z0, tpt, c0, k1);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = fma(T(alpha), k1[q], v[q]);
-    }
-    if (beta != 0.0)
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] = fma(T(beta * ihx), ks[(ii + 2) * ldk + c0 + q] - ks[ii * ldk + c0 + q], v[q]);
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = c0 + q;
-      if (c < R) rk_apply(rk, (int64_t)(i0 + ii) + (int64_t)c * N, (c < ka) ? v[q] : T(0));
-    }
-  }
-  for (int e = threadIdx.x; e < FUSED_BMH * (R - kap); e += blockDim.x) {  // inactive columns: zero rate
-    const int ii = e % FUSED_BMH, c = kap + e / FUSED_BMH;
-    if (ii < rows) rk_apply(rk, (int64_t)(i0 + ii) + (int64_t)c * N, T(0));
-  }
-}
-
-// L substep stage: v[j, c] = nu_j (Z A_xx)[j, c] + KR(Z, Z)_j T'_L[:, c], then the RK update.
-template <typename T>
-__global__ void __launch_bounds__(256) burgers_l_stage(int M, int R, const int32_t* __restrict__ rank,
-                                                       const T* __restrict__ Z, const T* __restrict__ nu,
-                                                       const double* __restrict__ Axx, const T* __restrict__ Tp,
-                                                       int PP, int nonlin, uint32_t* status, RkStage<T> rk) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int ka = min(R, (int)*rank);
-  if (ka > FUSED_KMAX) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(status, ST_BAD_SHAPE);
-    return;
-  }
-  const int np = ka * (ka + 1) / 2, ld = ka | 1, kap = (ka + 3) & ~3;
-  T* tpt = reinterpret_cast<T*>(smraw);
-  T* zs = tpt + (nonlin ? np * tensor_kpp(kap) : 0);  // BM x ld
-  T* as = zs + FUSED_BML * ld;              // ka x ka: A_xx
-  const int j0 = blockIdx.x * FUSED_BML;
-  const int rows = min(FUSED_BML, M - j0);
-  if (nonlin) load_tensor(ka, kap, Tp, PP, tpt);
-  for (int e = threadIdx.x; e < FUSED_BML * ka; e += blockDim.x) {
-    const int jj = e % FUSED_BML, a = e / FUSED_BML;
-    zs[jj * ld + a] = (jj < rows) ? Z[(j0 + jj) + (int64_t)a * M] : T(0);
-  }
-  for (int e = threadIdx.x; e < ka * ka; e += blockDim.x) as[e] = T(Axx[(e % ka) + (int64_t)(e / ka) * R]);
-  __syncthreads();
-  const int ncg = kap / 4;
-  for (int e = threadIdx.x; e < FUSED_BML * ncg; e += blockDim.x) {  // active column groups
-    const int jj = e % FUSED_BML, c0 = 4 * (e / FUSED_BML);
-    if (jj >= rows) continue;
-    T v[4] = {T(0), T(0), T(0), T(0)};
-    const T* z = zs + jj * ld;
-    T lin[4] = {T(0), T(0), T(0), T(0)};
-    for (int a = 0; a < ka; ++a)
-#pragma unroll
-      for (int q = 0; q < 4; ++q)
-        if (c0 + q < ka) lin[q] = fma(z[a], as[a + (c0 + q) * ka], lin[q]);
-    const T nj = nu[j0 + jj];
-#pragma unroll
-    for (int q = 0; q < 4; ++q) v[q] = nj * lin[q];
-    if (nonlin) {
-      T k[4] = {T(0), T(0), T(0), T(0)};
-      kr_row4<T, true>(ka, tensor_kpp(kap), z, z, tpt, c0, k);
-#pragma unroll
-      for (int q = 0; q < 4; ++q) v[q] += k[q];
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) {
-      const int c = c0 + q;
-      if (c < R) rk_apply(rk, (int64_t)(j0 + jj) + (int64_t)c * M, (c < ka) ? v[q] : T(0));
-    }
-  }
-  for (int e = threadIdx.x; e < FUSED_BML * (R - kap); e += blockDim.x) {  // inactive columns: zero rate
-    const int jj = e % FUSED_BML, c = kap + e / FUSED_BML;
-    if (jj < rows) rk_apply(rk, (int64_t)(j0 + jj) + (int64_t)c * M, T(0));
-  }
-}
-
-// S substep stage, row part: with A = Uhat Z (N x ka on the active columns
-// of the augmented panel), P2 = alpha KR(Dx A, A) T'_h + beta Dx(KR(A, A) T'_h)
-// and this CTA's partial of Uhat^T P2 (ka x ka, FP64 at the active indices
-// of part[blockIdx.x], ld 2R).  s_stage_finish_warp adds the partials.
-template <typename T>
-__global__ void __launch_bounds__(256) burgers_s_rows(int N, int R, const int32_t* __restrict__ rank,
-                                                      const T* __restrict__ Uh, const double* __restrict__ Zs,
-                                                      const T* __restrict__ Tp, int PP, double ihx, double alpha,
-                                                      double beta, uint32_t* status, double* __restrict__ part,
-                                                      const double* __restrict__ Nnu, const double* __restrict__ Axx,
-                                                      double* __restrict__ C) {
-  extern __shared__ __align__(16) unsigned char smraw[];
-  const int r = min(R, (int)*rank), ka = 2 * r, w = 2 * R;
-  if (ka > FUSED_KMAX) {
-    if (threadIdx.x == 0 && blockIdx.x == 0) atomicOr(status, ST_BAD_SHAPE);
-    return;
-  }
-  const int np = ka * (ka + 1) / 2, ld = ka | 1, kap = (ka + 3) & ~3, ncg = kap / 4, ldk = kap | 1;
-  T* tpt = reinterpret_cast<T*>(smraw);        // np x kpp
-  T* us = tpt + np * tensor_kpp(kap);          // (BM + 2) x ld: Uhat rows i0 - 1 .. i0 + BM
-  T* zm = us + (FUSED_BMH + 2) * ld;            // ka x ka: Z, row-major (zm[k ka + c] = Z[k, c])
-  T* as = zm + ka * ka;                        // (BM + 2) x ld: A rows
-  T* ks = as + (FUSED_BMH + 2) * ld;            // (BM + 2) x ldk: KR(A, A) T'
-  T* d1 = ks + (FUSED_BMH + 2) * ldk;           // BM x ld: Dx A
-  T* p2 = d1 + FUSED_BMH * ld;                  // BM x ldk: P2
-  const int i0 = blockIdx.x * FUSED_BMH;
-  const int rows = min(FUSED_BMH, N - i0);
-  load_tensor(ka, kap, Tp, PP, tpt);
-  for (int e = threadIdx.x; e < (FUSED_BMH + 2) * ka; e += blockDim.x) {
-    const int ii = e % (FUSED_BMH + 2), a = e / (FUSED_BMH + 2);
-    int g = i0 - 1 + ii;
-    g = (g < 0) ? g + N : ((g >= N) ? g - N : g);
-    us[ii * ld + a] = Uh[g + (int64_t)act_col(a, r, R) * N];
-  }
-  for (int e = threadIdx.x; e < ka * ka; e += blockDim.x) {
-    const int k = e % ka, c = e / ka;
-    zm[k * ka + c] = T(Zs[act_col(k, r, R) + (int64_t)act_col(c, r, R) * w]);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < (FUSED_BMH + 2) * ka; e += blockDim.x) {  // A = Uhat Z
-    const int ii = e % (FUSED_BMH + 2), c = e / (FUSED_BMH + 2);
-    T acc = T(0);
-    for (int k = 0; k < ka; ++k) acc = fma(us[ii * ld + k], zm[k * ka + c], acc);
-    as[ii * ld + c] = acc;
-  }
-  __syncthreads();
-  if (beta != 0.0)
-    for (int e = threadIdx.x; e < (FUSED_BMH + 2) * ncg; e += blockDim.x) {
-      const int ii = e % (FUSED_BMH + 2), c0 = 4 * (e / (FUSED_BMH + 2));
-      T acc[4] = {T(0), T(0), T(0), T(0)};
-      kr_row4<T, true>(ka, tensor_kpp(kap), as + ii * ld, as + ii * ld, tpt, c0, acc);
-#pragma unroll
-      for (int v = 0; v < 4; ++v) ks[ii * ldk + c0 + v] = acc[v];
-    }
-  for (int e = threadIdx.x; e < FUSED_BMH * ka; e += blockDim.x) {
-    const int ii = e % FUSED_BMH, c = e / FUSED_BMH;
-    d1[ii * ld + c] = T(ihx) * (as[(ii + 2) * ld + c] - as[ii * ld + c]);
-  }
-  __syncthreads();
-  for (int e = threadIdx.x; e < FUSED_BMH * ncg; e += blockDim.x) {
-    const int ii = e % FUSED_BMH, c0 = 4 * (e / FUSED_BMH);
-    T v[4] = {T(0), T(0), T(0), T(0)};
-    if (ii < rows) {
-      if (alpha != 0.0) {
-        T k1[4] = {T(0), T(0), T(0), T(0)};
-        kr_row4<T, false>(ka, tensor_kpp(kap), d1 + ii * ld, as + (ii + 1) * ld, tpt, c0, k1);
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = fma(T(alpha), k1[q], v[q]);
-      }
-      if (beta != 0.0)
-#pragma unroll
-        for (int q = 0; q < 4; ++q) v[q] = fma(T(beta * ihx), ks[(ii + 2) * ldk + c0 + q] - ks[ii * ldk + c0 + q], v[q]);
-    }
-#pragma unroll
-    for (int q = 0; q < 4; ++q) p2[ii * ldk + c0 + q] = v[q];
-  }
-  __syncthreads();
-  double* dst = part + (int64_t)blockIdx.x * w * w;
-  for (int e = threadIdx.x; e < ka * ka; e += blockDim.x) {  // Uhat^T P2 over the tile's rows
-    const int a = e % ka, c = e / ka;
-    T acc = T(0);
-    for (int ii = 0; ii < rows; ++ii) acc = fma(us[(ii + 1) * ld + a], p2[ii * ldk + c], acc);
-    dst[act_col(a, r, R) + (int64_t)act_col(c, r, R) * w] = (double)acc;
-  }
-  if (blockIdx.x == 0) {
-    // the linear part of the stage, C = A_xx Z N_nu on the active block
-    // (T1 = Z N_nu first), in the tensor's area once every thread is past it
-    __syncthreads();
-    T* nn = tpt;           // N_nu, row-major
-    T* ax = nn + ka * ka;  // A_xx, row-major
-    T* t1 = ax + ka * ka;  // Z N_nu, row-major
-    for (int e = threadIdx.x; e < ka * ka; e += blockDim.x) {
-      const int k = e / ka, c = e % ka;
-      const int64_t g = act_col(k, r, R) + (int64_t)act_col(c, r, R) * w;
-      nn[e] = T(Nnu[g]);
-      ax[e] = T(Axx[g]);
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < ka * ka; e += blockDim.x) {
-      const int i = e / ka, c = e % ka;
-      T acc = T(0);
-      for (int k = 0; k < ka; ++k) acc = fma(zm[i * ka + k], nn[k * ka + c], acc);
-      t1[e] = acc;
-    }
-    __syncthreads();
-    for (int e = threadIdx.x; e < ka * ka; e += blockDim.x) {
-      const int i = e % ka, c = e / ka;
-      T acc = T(0);
-      for (int k = 0; k < ka; ++k) acc = fma(ax[i * ka + k], t1[k * ka + c], acc);
-      C[act_col(i, r, R) + (int64_t)act_col(c, r, R) * w] = (double)acc;
-    }
-  }
-}
-
-// S-flow stage of the fused path: v[a, c] = C[a, c] + sum_z part[z][a, c] on
-// the active block, one warp per entry (lane-strided partials, a fixed
-// shuffle tree: deterministic), then the RK update of the FP64 stage arrays.
-__global__ void __launch_bounds__(256) s_stage_finish_warp(int R, const int32_t* __restrict__ rank, int nz,
-                                                           const double* __restrict__ part,
-                                                           const double* __restrict__ C, RkStage<double> rk) {
-  const int r = min(R, (int)*rank), ka = 2 * r, w = 2 * R;
-  const int lane = threadIdx.x & 31;
-  const int64_t len = (int64_t)ka * ka;
-  for (int64_t o = (blockIdx.x * (int64_t)blockDim.x + threadIdx.x) >> 5; o < len;
-       o += ((int64_t)gridDim.x * blockDim.x) >> 5) {
-    const int64_t idx = act_col((int)(o % ka), r, R) + (int64_t)act_col((int)(o / ka), r, R) * w;
-    double v = 0.0;
-    for (int z = lane; z < nz; z += 32) v += part[z * (int64_t)w * w + idx];
-#pragma unroll
-    for (int off = 16; off > 0; off >>= 1) v += __shfl_xor_sync(0xffffffffu, v, off);
-    if (lane == 0) rk_apply(rk, idx, C[idx] + v);
-  }
-}
-
-// dynamic shared memory of the fused stages at the largest width (FUSED_KMAX)
-template <typename T>
-size_t fused_smem(int which) {
-  const size_t K = FUSED_KMAX, np = K * (K + 1) / 2, KP = tensor_kpp(FUSED_KMAX);
-  const size_t L = K | 1;  // padded row stride
-  if (which == 0) return sizeof(T) * (np * KP + 2 * (FUSED_BMH + 2) * L + K * K + FUSED_BMH * L);
-  if (which == 1) return sizeof(T) * (np * KP + FUSED_BML * L + K * K);
-  return sizeof(T) * (np * KP + 3 * (FUSED_BMH + 2) * L + K * K + 2 * FUSED_BMH * L);
-}
-
 // small FP64 helpers of the S step: X (R x R, T, ld R) -> Y (FP64, ld R), optionally transposed
 template <typename T>
 __global__ void small_to_f64(int R, const T* __restrict__ X, int trans, double* __restrict__ Y) {
@@ -1992,6 +1615,7 @@ struct lri_stream {
   void* tv = nullptr;   // flow tensors T'_V, T'_L, T'_Vhat: PP x 2R each (PP = 2R (2R + 1) / 2 pairs)
   void* tl = nullptr;
   void* th = nullptr;
+  void* tw = nullptr;   // W' of Uhat (the S flow on the core)
   void* kgp = nullptr;  // split partials of the tensor sums (ceil(max(n, m) / KR_ROWS) x PP x 2R) and of gram_act
   void* kap = nullptr;  // pair-split partials of the Khatri-Rao products: 2 x kZmax x max(n, m) x 2R
   void* pw = nullptr;   // 3 work panels of max(n, m) x 2R
@@ -2013,14 +1637,13 @@ struct lri_stream {
   double graph_dt[3] = {0.0, 0.0, 0.0};
   bool class_seen[3] = {false, false, false};
   double last_dt[3] = {0.0, 0.0, 0.0};  // dt of the class's previous step (a repeat of it is captured)
-  // fused RK-stage kernels for the current rank: 0 none (rank > 32), 1 the K
-  // and L stages (rank <= 32), 2 also the S stage (rank <= 16)
+  // flow kernels for the current rank (burgers_flow.cu): 0 none (rank > 32),
+  // 1 the K and L flows (rank <= 32), 2 also the S flow (rank <= 16)
   int fused = 0;
   // FP32 Burgers engines: the Khatri-Rao products of the unfused flows
   // (active width above 32) on the tensor cores (tc_kr.cu)
   bool kr_ok = false, use_kr = false;
   lri::TcKr kr;
-  double* fgp = nullptr;  // the fused S stage's per-tile partials: ceil(n / FUSED_BMH) x (2R)^2 FP64
 };
 
 
@@ -2147,6 +1770,8 @@ struct StreamOps {
   }
 
   // Burgers flow helpers (see the kernels' notes)
+  // bound of the active width in the K and L flow kernels
+  int flow_kmax() const { return s->fused >= 2 ? FLOW_KMAX / 2 : FLOW_KMAX; }
   int64_t pairs_max() const { return (2 * s->R) * (2 * s->R + 1) / 2; }
   // Tout (+)= coef * (packed tensor of KR(P,Q)^T Y over N rows)
   cudaError_t tensor(int N, int aug, const T* P, const T* Q, const T* Y, double coef, int acc, T* Tout) const {
@@ -2292,21 +1917,15 @@ struct StreamOps {
     return cudaSuccess;
   }
 
-  // one fused L-flow stage on this object's stream
-  cudaError_t l_stage_fused(const T* Z, const double* Axx, bool nonlin, const RkStage<T>& rk) const {
-    const int m = (int)s->m, R = (int)s->R;
-    burgers_l_stage<T><<<(m + FUSED_BML - 1) / FUSED_BML, 256, fused_smem<T>(1), st>>>(
-        m, R, s->d_rank, Z, static_cast<const T*>(s->nu), Axx, tp(s->tl), (int)pairs_max(), nonlin ? 1 : 0,
-        s->d_status, rk);
-    return cudaGetLastError();
-  }
-  // the whole L substep flow (Lp holds L0 and its RK panels): the fused
-  // stages, or the product panel, the Khatri-Rao partials and the combine
-  // (with the side stream's own panel and partials for scratch set 1)
+  // the whole L substep flow (Lp holds L0 and its RK panels): one launch up
+  // to rank FLOW_KMAX, else per stage the product panel, the Khatri-Rao
+  // partials and the combine (with the side stream's own panel and partials
+  // for scratch set 1)
   cudaError_t l_flow(T* Lp, const double* Axx, bool nonlin) const {
     if (s->fused >= 1)
-      return rk_panel((int64_t)s->m * s->R, Lp,
-                      [&](const T* Z, const RkStage<T>& rk) { return l_stage_fused(Z, Axx, nonlin, rk); });
+      return burgers_l_flow<T>(flow_kmax(), (int)s->m, (int)s->R, s->d_rank, Lp, static_cast<const T*>(s->nu), Axx,
+                               tp(s->tl), (int)pairs_max(), nonlin ? 1 : 0, s->sc, s->bh_dt / s->sc.nsub,
+                               s->d_status, st);
     const int m = (int)s->m, R = (int)s->R, w = 2 * R;
     const int64_t nm = std::max(s->n, s->m);
     T* P2 = sid ? tp(s->pw2) : tp(s->pw) + 2 * nm * w;
@@ -2345,12 +1964,6 @@ struct StreamOps {
     const int g = 304;
     cudaError_t e = refresh();
     if (e != cudaSuccess) return e;
-    if (s->fused) {
-      static std::atomic<uint64_t> a0{0}, a1{0}, a2{0};
-      if ((e = set_smem_limit(burgers_k_stage<T>, (int)fused_smem<T>(0), a0)) != cudaSuccess) return e;
-      if ((e = set_smem_limit(burgers_l_stage<T>, (int)fused_smem<T>(1), a1)) != cudaSuccess) return e;
-      if ((e = set_smem_limit(burgers_s_rows<T>, (int)fused_smem<T>(2), a2)) != cudaSuccess) return e;
-    }
     small_to_f64<T><<<16, 256, 0, st>>>(R, S, 0, blk(16));
     small_to_f64<T><<<16, 256, 0, st>>>(R, S, 1, blk(17));
     // operators of the K substep (V0 fixed): N_nu = V0^T diag(nu) V0, T'_V
@@ -2385,12 +1998,10 @@ struct StreamOps {
       if (el == cudaSuccess) el = ej;
     }
     const int zk = kz(n, 0);
-    e = rk_panel((int64_t)n * R, Kp, [&](const T* Z, const RkStage<T>& rk) {
-      if (s->fused >= 1) {
-        burgers_k_stage<T><<<(n + FUSED_BMH - 1) / FUSED_BMH, 256, fused_smem<T>(0), st>>>(
-            n, R, s->d_rank, Z, Nnu, tp(s->tv), (int)pairs_max(), ih2, ihx, ba, bb, s->d_status, rk);
-        return cudaGetLastError();
-      }
+    if (s->fused >= 1)
+      e = burgers_k_flow<T>(flow_kmax(), n, R, s->d_rank, Kp, Kp + (int64_t)n * R, Nnu, tp(s->tv), (int)pairs_max(),
+                            ih2, ihx, ba, bb, s->sc, s->bh_dt / s->sc.nsub, s->sms, s->d_status, st);
+    else e = rk_panel((int64_t)n * R, Kp, [&](const T* Z, const RkStage<T>& rk) {
       stencil_panel<T><<<g, 256, 0, st>>>(n, R, 0, s->d_rank, Z, ih2, P0, ihx, ba != 0.0 ? P1 : nullptr);
       panel_mul_act<T><<<dim3((n + 31) / 32, (R + 63) / 64), 256, 0, st>>>(n, R, 0, s->d_rank, P0, Nnu, R, P2);
       cudaError_t e2 = cudaGetLastError();
@@ -2416,8 +2027,12 @@ struct StreamOps {
     double* Axxh = blk(15);
     double* Nnuh = blk(23);
     double* Stmp = blk(22);
-    stencil_panel<T><<<g, 256, 0, st>>>(n, R, 1, s->d_rank, Uh, ih2, P0, 0.0, nullptr);
+    const bool sflow = s->fused >= 2;
+    stencil_panel<T><<<g, 256, 0, st>>>(n, R, 1, s->d_rank, Uh, ih2, P0, ihx, sflow ? P1 : nullptr);
     if ((e = gram(n, w, w, Uh, n, P0, n, 1.0, 0.0, Axxh, w)) != cudaSuccess) return e;
+    // the S flow on the core: W' of Uhat, as T'_L of U0 above
+    if (sflow && ba != 0.0 && (e = tensor(n, 1, P1, Uh, Uh, ba, 0, tp(s->tw))) != cudaSuccess) return e;
+    if (sflow && bb != 0.0 && (e = tensor(n, 1, Uh, Uh, P1, -bb, ba != 0.0, tp(s->tw))) != cudaSuccess) return e;
     scale_rows<T><<<g, 256, 0, st>>>(m, w, Vh, nu, P0);
     if ((e = gram(m, w, w, Vh, m, P0, m, 1.0, 0.0, Nnuh, w)) != cudaSuccess) return e;
     if (nonlin && (e = tensor(m, 1, Vh, Vh, Vh, 1.0, 0, tp(s->th))) != cudaSuccess) return e;
@@ -2425,7 +2040,11 @@ struct StreamOps {
     // S step on the augmented bases from S~0 = Mh S0 Nh^T (FP64 w x w):
     // S' = A_xx S N_nu + Uhat^T [alpha KR(Dx A, A) T'_Vhat + beta Dx(KR(A, A) T'_Vhat)], A = Uhat S
     small_msn<<<1, 1024, 0, st>>>(w, R, blk(3), blk(16), blk(4), Stmp, blk(18));
-    {
+    if (sflow) {
+      e = burgers_s_flow<T>(R, s->d_rank, blk(18), Nnuh, Axxh, tp(s->th), tp(s->tw), (int)pairs_max(),
+                            nonlin ? 1 : 0, s->sc, s->bh_dt / s->sc.nsub, s->d_status, st);
+      if (e != cudaSuccess) return e;
+    } else {
       const Scheme& sc = s->sc;
       const double h = s->bh_dt / sc.nsub;
       double* Sy = blk(18);
@@ -2441,16 +2060,6 @@ struct StreamOps {
           const double* Z = (st_ == 0) ? Sy : Sz;
           const bool last = (st_ + 1 == sc.nstages);
           const RkStage<double> rk{sc.b[st_], last ? 0.0 : h * sc.a[st_ + 1], h, st_ == 0, last, Sy, Sz, Sa};
-          if (nonlin && s->fused >= 2) {
-            // burgers_s_rows also forms C = A_xx Z N_nu (its first CTA)
-            const int nzf = (n + FUSED_BMH - 1) / FUSED_BMH;
-            burgers_s_rows<T><<<nzf, 256, fused_smem<T>(2), st>>>(n, R, s->d_rank, Uh, Z, tp(s->th),
-                                                                   (int)pairs_max(), ihx, ba, bb, s->d_status, s->fgp,
-                                                                   Nnuh, Axxh, Sk);
-            s_stage_finish_warp<<<128, 256, 0, st>>>(R, s->d_rank, nzf, s->fgp, Sk, rk);
-            e = cudaGetLastError();
-            continue;
-          }
           small_gemm_act<T><<<gsm, 256, 0, st>>>(R, s->d_rank, Z, Nnuh, Stmp);
           small_gemm_act<T><<<gsm, 256, 0, st>>>(R, s->d_rank, Axxh, Stmp, Sk);
           if (nonlin) {
@@ -2635,7 +2244,7 @@ static cudaError_t fused_class(lri_stream* s, cudaStream_t st, int* cls) {
   if (e == cudaSuccess) e = cudaStreamSynchronize(st);
   if (e != cudaSuccess) return e;
   const int ra = std::min<int>((int)s->R, r);
-  *cls = (2 * ra <= lri::FUSED_KMAX) ? 2 : (ra <= lri::FUSED_KMAX ? 1 : 0);
+  *cls = (2 * ra <= lri::FLOW_KMAX) ? 2 : (ra <= lri::FLOW_KMAX ? 1 : 0);
   return cudaSuccess;
 }
 
@@ -2742,7 +2351,8 @@ lri_status lri_burgers_create(lri_stream** out, int32_t dtype, int64_t n, int64_
   alloc(&s->pw, s->es * 3 * nm * 2 * R);
   alloc(&s->pw2, s->es * nm * 2 * R);
   alloc(&s->kap2nd, s->es * kZmax * nm * 2 * R);
-  alloc((void**)&s->fgp, sizeof(double) * ((n + lri::FUSED_BMH - 1) / lri::FUSED_BMH) * 4 * R * R);
+  // (the S flow's tensor of Uhat: ranks up to FLOW_KMAX / 2)
+  alloc(&s->tw, s->es * PP * std::min<int64_t>(2 * R, lri::FLOW_KMAX));
   if (e == cudaSuccess && dtype == LRI_F32 && lri::tc_kr_supported((int)R)) {
     e = lri::tc_kr_init(&s->kr, (int)R);
     s->kr_ok = s->use_kr = (e == cudaSuccess);
@@ -2810,7 +2420,7 @@ lri_status lri_stream_destroy(lri_stream* s) {
   cudaFree(s->pw);
   cudaFree(s->pw2);
   cudaFree(s->kap2nd);
-  cudaFree(s->fgp);
+  cudaFree(s->tw);
   cudaFree(s->d_rank);
   cudaFree(s->d_status);
   cudaFree(s->Uh);

@@ -91,3 +91,30 @@ def test_burgers_large_padded_exact_rank_matches_oracle(lri, oracle, precision, 
         assert err <= tol, f"step {k}: {err:.3e} (ranks {yg.S.shape[0]} / {yo.S.shape[0]})"
         U = np.asarray(yg.U, np.float64)
         assert np.abs(U.T @ U - np.eye(U.shape[1])).max() <= (1e-12 if precision == "fp64" else 1e-5)
+
+
+# (n, m, r, scheme, substeps, alpha, beta): panels shorter than a tile and with
+# remainders, odd and even launch counts of the K flow (4 RK4 or 8 Heun
+# substeps each), both widths of the flow kernels (ranks <= 16 and 17..32),
+# either quadratic term and both; the S flow on the core up to rank 16
+FLOW_EDGES = [(40, 37, 3, "RK4", 5, 0.0, -0.5), (97, 130, 16, "RK4", 3, -1.0, 0.0), (128, 64, 8, "Heun", 17, -0.3, -0.2),
+              (129, 65, 17, "RK4", 2, 0.0, -0.5), (100, 191, 32, "RK4", 4, -0.5, -0.25), (66, 65, 5, "Euler", 3, 0.0, 0.0)]
+
+
+@pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("fp32", 1e-5)])
+@pytest.mark.parametrize("n,m,r,scheme,nsub,alpha,beta", FLOW_EDGES)
+def test_burgers_flow_kernel_edges(lri, oracle, n, m, r, scheme, nsub, alpha, beta, precision, tol):
+    h, nu, X0d = workloads.burgers_uq(n, m, seed=4)
+    X0d = X0d + 1e-2 * np.random.default_rng(5).standard_normal(X0d.shape)
+    Y0 = oracle.truncated_svd(X0d, r=r)
+    dt, T = 1e-4, 2e-4
+    pg = lri.MatrixDEProblem(lri.BurgersOperator(h, nu, alpha=alpha, beta=beta),
+                             lri.SVDLikeRepresentation(Y0.U, Y0.S, Y0.V), (0.0, T))
+    po = oracle.MatrixDEProblem(oracle.BurgersOp(n, h, nu, alpha=alpha, beta=beta), Y0, (0.0, T))
+    ag = lri.RankAdaptiveUnconventionalAlgorithm(1e-8, rmax=r, K_alg=getattr(lri, scheme)(nsub), rmin=r)
+    ao = oracle.RankAdaptiveUnconventionalAlgorithm(1e-8, rmax=r, K_alg=getattr(oracle, scheme)(nsub), rmin=r)
+    sg = lri.solve_burgers_large(pg, ag, dt, precision=precision, save_everystep=True)
+    so = oracle.solve(po, ao, dt)
+    for k, (yg, yo) in enumerate(zip(sg.Y, so.Y)):
+        err = oracle.rel_fro_err(yg.full(), yo.full())
+        assert err <= tol, f"step {k}: {err:.3e}"
