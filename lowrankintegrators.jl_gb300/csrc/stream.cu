@@ -35,6 +35,7 @@
 #include <vector>
 
 #include "../../include/lri.h"
+#include "burgers_core.h"
 #include "burgers_flow.h"
 #include "core_svd.h"
 #include "engine.cuh"
@@ -1644,6 +1645,8 @@ struct lri_stream {
   // (active width above 32) on the tensor cores (tc_kr.cu)
   bool kr_ok = false, use_kr = false;
   lri::TcKr kr;
+  bool core_ok = false;  // the S flow on the core (burgers_core.cu) at ranks above FLOW_KMAX / 2
+  lri::SCore score;
 };
 
 
@@ -2027,22 +2030,30 @@ struct StreamOps {
     double* Axxh = blk(15);
     double* Nnuh = blk(23);
     double* Stmp = blk(22);
+    // S flow on the core: one cluster up to rank 16, tensor cores above (FP32)
     const bool sflow = s->fused >= 2;
-    stencil_panel<T><<<g, 256, 0, st>>>(n, R, 1, s->d_rank, Uh, ih2, P0, ihx, sflow ? P1 : nullptr);
+    const bool scoref = !sflow && nonlin && std::is_same<T, float>::value && s->core_ok;
+    const bool wten = sflow || scoref;
+    stencil_panel<T><<<g, 256, 0, st>>>(n, R, 1, s->d_rank, Uh, ih2, P0, ihx, wten ? P1 : nullptr);
     if ((e = gram(n, w, w, Uh, n, P0, n, 1.0, 0.0, Axxh, w)) != cudaSuccess) return e;
     // the S flow on the core: W' of Uhat, as T'_L of U0 above
-    if (sflow && ba != 0.0 && (e = tensor(n, 1, P1, Uh, Uh, ba, 0, tp(s->tw))) != cudaSuccess) return e;
-    if (sflow && bb != 0.0 && (e = tensor(n, 1, Uh, Uh, P1, -bb, ba != 0.0, tp(s->tw))) != cudaSuccess) return e;
+    if (wten && ba != 0.0 && (e = tensor(n, 1, P1, Uh, Uh, ba, 0, tp(s->tw))) != cudaSuccess) return e;
+    if (wten && bb != 0.0 && (e = tensor(n, 1, Uh, Uh, P1, -bb, ba != 0.0, tp(s->tw))) != cudaSuccess) return e;
     scale_rows<T><<<g, 256, 0, st>>>(m, w, Vh, nu, P0);
     if ((e = gram(m, w, w, Vh, m, P0, m, 1.0, 0.0, Nnuh, w)) != cudaSuccess) return e;
     if (nonlin && (e = tensor(m, 1, Vh, Vh, Vh, 1.0, 0, tp(s->th))) != cudaSuccess) return e;
-    if (nonlin && kr_tc() && (e = kr_split(2, tp(s->th), 1)) != cudaSuccess) return e;
+    if (nonlin && !wten && kr_tc() && (e = kr_split(2, tp(s->th), 1)) != cudaSuccess) return e;
     // S step on the augmented bases from S~0 = Mh S0 Nh^T (FP64 w x w):
     // S' = A_xx S N_nu + Uhat^T [alpha KR(Dx A, A) T'_Vhat + beta Dx(KR(A, A) T'_Vhat)], A = Uhat S
     small_msn<<<1, 1024, 0, st>>>(w, R, blk(3), blk(16), blk(4), Stmp, blk(18));
     if (sflow) {
       e = burgers_s_flow<T>(R, s->d_rank, blk(18), Nnuh, Axxh, tp(s->th), tp(s->tw), (int)pairs_max(),
                             nonlin ? 1 : 0, s->sc, s->bh_dt / s->sc.nsub, s->d_status, st);
+      if (e != cudaSuccess) return e;
+    } else if (scoref) {
+      if constexpr (std::is_same<T, float>::value)
+        e = s_core_flow(s->score, s->d_rank, blk(18), blk(21), Nnuh, Axxh, tp(s->th), tp(s->tw), (int)pairs_max(),
+                        s->sc, s->bh_dt / s->sc.nsub, s->d_status, st);
       if (e != cudaSuccess) return e;
     } else {
       const Scheme& sc = s->sc;
@@ -2351,8 +2362,12 @@ lri_status lri_burgers_create(lri_stream** out, int32_t dtype, int64_t n, int64_
   alloc(&s->pw, s->es * 3 * nm * 2 * R);
   alloc(&s->pw2, s->es * nm * 2 * R);
   alloc(&s->kap2nd, s->es * kZmax * nm * 2 * R);
-  // (the S flow's tensor of Uhat: ranks up to FLOW_KMAX / 2)
-  alloc(&s->tw, s->es * PP * std::min<int64_t>(2 * R, lri::FLOW_KMAX));
+  if (e == cudaSuccess && dtype == LRI_F32 && 2 * R > lri::FLOW_KMAX && lri::s_core_supported((int)R)) {
+    e = lri::s_core_init(&s->score, (int)R);
+    s->core_ok = (e == cudaSuccess);
+  }
+  // the S flow's tensor of Uhat
+  alloc(&s->tw, s->es * PP * (s->core_ok ? 2 * R : std::min<int64_t>(2 * R, lri::FLOW_KMAX)));
   if (e == cudaSuccess && dtype == LRI_F32 && lri::tc_kr_supported((int)R)) {
     e = lri::tc_kr_init(&s->kr, (int)R);
     s->kr_ok = s->use_kr = (e == cudaSuccess);
@@ -2429,6 +2444,7 @@ lri_status lri_stream_destroy(lri_stream* s) {
   cudaFree(s->Xl);
   cudaFree(s->Zp);
   lri::tc_kr_free(&s->kr);
+  lri::s_core_free(&s->score);
   cudaFree(s->part);
   cudaFree(s->part2);
   cudaFree(s->small2);

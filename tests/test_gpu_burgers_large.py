@@ -98,7 +98,9 @@ def test_burgers_large_padded_exact_rank_matches_oracle(lri, oracle, precision, 
 # substeps each), both widths of the flow kernels (ranks <= 16 and 17..32),
 # either quadratic term and both; the S flow on the core up to rank 16
 FLOW_EDGES = [(40, 37, 3, "RK4", 5, 0.0, -0.5), (97, 130, 16, "RK4", 3, -1.0, 0.0), (128, 64, 8, "Heun", 17, -0.3, -0.2),
-              (129, 65, 17, "RK4", 2, 0.0, -0.5), (100, 191, 32, "RK4", 4, -0.5, -0.25), (66, 65, 5, "Euler", 3, 0.0, 0.0)]
+              (129, 65, 17, "RK4", 2, 0.0, -0.5), (100, 191, 32, "RK4", 4, -0.5, -0.25), (66, 65, 5, "Euler", 3, 0.0, 0.0),
+              # the S flow's tensor-core form: two, three and four 32-column chunks of the core
+              (160, 150, 33, "RK4", 1, -1.0, 0.0), (131, 140, 49, "Heun", 2, 0.0, -0.5), (140, 129, 64, "RK4", 1, -0.4, -0.3)]
 
 
 @pytest.mark.parametrize("precision,tol", [("fp64", 1e-10), ("fp32", 1e-5)])
