@@ -53,6 +53,7 @@ struct lri_batch {
   const void* opB = nullptr;
   bool bound = false;
   bool data_ready = false;
+  lri::WidePlan wide;       // clusters of small FP64 BUG batches (C = 0: the step kernel)
   int32_t ctas_per_sm = 3;  // register budget of the step kernel (lri_batch_set_occupancy)
   // discrete adjoint (allocated by lri_batch_adjoint_prepare)
   double* d_adj_work = nullptr;
@@ -140,6 +141,7 @@ cudaError_t launch_one(const lri_batch* b, double t, double dt, const void* Ynex
     if (e != cudaSuccess) return e;
     return lri::launch_step<lri::dfloat>(make_args<lri::dfloat>(b, t, dt, Ynext), count, st, b->ctas_per_sm);
   }
+  if (b->wide.C) return lri::launch_wide_step(make_args<double>(b, t, dt, Ynext), count, b->wide, st);
   return lri::launch_step<double>(make_args<double>(b, t, dt, Ynext), count, st);
 }
 
@@ -282,6 +284,14 @@ lri_status lri_batch_create(lri_batch** out, const lri_batch_desc* desc, const l
     b->totSmall += lri::kSmallBlocks * al(w * w);  // blocks padded to 4 elements (see Inst::blk)
     d.offY = b->totY;
     if (desc->op == LRI_OP_DATA || alg->kind == LRI_ALG_GREEDY) b->totY += n * m;
+  }
+  // small FP64 BUG batches run on clusters (engine_wide.cu)
+  if (desc->dtype == LRI_F64 && alg->kind == LRI_ALG_BUG &&
+      (desc->op == LRI_OP_SYLVESTER_TRIDIAG || desc->op == LRI_OP_DATA)) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) == cudaSuccess &&
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
+      b->wide = lri::wide_plan(count, b->n.data(), b->m.data(), b->rcap.data(), sms);
   }
   // longest-processing-time-first launch order: CTAs start in block order
   b->order.resize(count);
@@ -523,7 +533,7 @@ int32_t lri_batch_launches_per_step(const lri_batch* b) {
   // one engine launch; double-float batches add the three write-back
   // conversions (and one snapshot conversion for data problems) per call
   if (b->desc.dtype == LRI_DF) return 4 + (b->totY > 0 ? 1 : 0);
-  return 1;
+  return b->wide.C ? 2 : 1;  // clusters: the sides, then the core
 }
 
 }  // extern "C"

@@ -111,6 +111,17 @@ inline cudaError_t launch_step(const StepArgs<T>& g, int count, cudaStream_t str
   }
 }
 
+// FP64 BUG steps of small batches on clusters (engine_wide.cu): CTAs per
+// cluster (0: the batch takes the step kernel) and the shared memory of the
+// two launches.
+constexpr size_t kWideSmemMax = 226 * 1024;
+struct WidePlan {
+  int C = 0;
+  size_t side_smem = 0, core_smem = 0;
+};
+WidePlan wide_plan(int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms);
+cudaError_t launch_wide_step(const StepArgs<double>& g, int count, const WidePlan& p, cudaStream_t st);
+
 // double <-> double-float conversions of n elements (dfloat storage is a
 // pair of floats, 8 bytes per element)
 cudaError_t convert_f64_to_df(const double* in, void* out, int64_t n, cudaStream_t stream);

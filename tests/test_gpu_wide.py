@@ -1,0 +1,85 @@
+"""FP64 BUG steps of small batches on thread-block clusters (the rows of each
+side split over a cluster, the core's columns over another) against the
+oracle: factors, not only Y (both use Householder's signs), at row counts
+with remainders, empty CTAs and fewer rows than columns per CTA, one-column
+to 64-column cores, batches of uneven members, data streams."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+# FP64 factors of cores with condition number 2^(r/4) <= 2^16 over three
+# steps: rounding grows to about 1e-16 * 2^16 * sqrt(n r) < 1e-9
+TOL = 1e-9
+
+
+def instance(seed, n, m, r):
+    g = np.random.default_rng(seed)
+    A = (g.uniform(0.5, 1, n), -2 - g.uniform(0, 1, n), g.uniform(0.5, 1, n))
+    B = (g.uniform(0.5, 1, m), -2 - g.uniform(0, 1, m), g.uniform(0.5, 1, m))
+    U, V = (np.linalg.qr(g.standard_normal((k, r)))[0] for k in (n, m))
+    return A, B, U, np.diag(2.0 ** (-np.arange(1, r + 1) / 4.0)), V
+
+
+def close(a, b):
+    return np.linalg.norm(a - b) <= TOL * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("scheme,nsub", [("RK4", 2), ("Heun", 1), ("Euler", 3)])
+@pytest.mark.parametrize("shapes", [[(8, 9, 1)], [(33, 17, 5)], [(17, 130, 16)], [(300, 257, 32)], [(64, 70, 64)],
+                                    [(100, 64, 33)], [(512, 40, 7), (31, 300, 20), (64, 64, 3)],
+                                    [(40 + 3 * i, 60 - i, 2 + i % 5) for i in range(21)]])
+def test_wide_step_matches_oracle(lri, oracle, shapes, scheme, nsub):
+    dt, k = 1e-2, 3
+    ins = [instance(10 + i, *s) for i, s in enumerate(shapes)]
+    probs = [lri.MatrixDEProblem(lri.SylvesterTridiagOperator(A, B), lri.SVDLikeRepresentation(U, S, V), (0.0, k * dt))
+             for A, B, U, S, V in ins]
+    got = lri.solve_ensemble(probs, lri.UnconventionalAlgorithm(getattr(lri, scheme)(nsub)), dt, precision="fp64")
+    for (A, B, U, S, V), y in zip(ins, got):
+        po = oracle.MatrixDEProblem(oracle.SylvesterTridiagOp(A, B), oracle.SVDLikeRepresentation(U, S, V), (0.0, k * dt))
+        yo = oracle.solve(po, oracle.UnconventionalAlgorithm(getattr(oracle, scheme)(nsub)), dt).Y[-1]
+        assert close(y.U, yo.U) and close(y.S, yo.S) and close(y.V, yo.V)
+
+
+def test_wide_step_full_gram_form(lri, oracle):
+    """A basis that is not orthonormal to 2^-36 takes the full Gram product."""
+    A, B, U, S, V = instance(3, 120, 90, 6)
+    U = U * (1 + 1e-6 * np.arange(6))
+    V = V @ (np.eye(6) + 1e-4 * np.ones((6, 6)))
+    po = oracle.MatrixDEProblem(oracle.SylvesterTridiagOp(A, B), oracle.SVDLikeRepresentation(U, S, V), (0.0, 0.02))
+    pg = lri.MatrixDEProblem(lri.SylvesterTridiagOperator(A, B), lri.SVDLikeRepresentation(U, S, V), (0.0, 0.02))
+    y = lri.solve(pg, lri.UnconventionalAlgorithm(lri.RK4(2)), 0.01).Y[-1]
+    yo = oracle.solve(po, oracle.UnconventionalAlgorithm(oracle.RK4(2)), 0.01).Y[-1]
+    assert close(y.U, yo.U) and close(y.S, yo.S) and close(y.V, yo.V)
+
+
+@pytest.mark.parametrize("n,m,r", [(100, 100, 12), (8, 70, 3), (131, 33, 32), (200, 210, 64)])
+def test_wide_data_step_matches_oracle(lri, oracle, n, m, r):
+    g = np.random.default_rng(n)
+    _, _, U, S, V = instance(n, n, m, r)
+    snaps = [U @ S @ V.T]
+    for _ in range(3):
+        snaps.append(snaps[-1] + 0.05 * g.standard_normal((n, m)))
+    sg = lri.solve(lri.MatrixDataProblem(snaps, lri.SVDLikeRepresentation(U, S, V)), lri.UnconventionalAlgorithm())
+    so = oracle.solve(oracle.MatrixDataProblem(snaps, oracle.SVDLikeRepresentation(U, S, V)),
+                      oracle.UnconventionalAlgorithm())
+    for y, yo in zip(sg.Y, so.Y):
+        assert close(y.U, yo.U) and close(y.S, yo.S) and close(y.V, yo.V)
+
+
+def test_wide_graph_and_single_steps_agree(lri):
+    """One five-step call (a captured graph) and five calls give the same bits,
+    also after binding new factors."""
+    A, B, U, S, V = instance(5, 210, 190, 9)
+    b = lri.Batch([210], [190], [9], lri.UnconventionalAlgorithm(lri.RK4(1)), lri.SylvesterTridiagOperator.kind, "fp64")
+    out = []
+    for multi in (True, False):
+        b.upload([lri.SVDLikeRepresentation(U, S, V)], [lri.SylvesterTridiagOperator(A, B)])
+        if multi:
+            b.step(0.0, 0.01, 5)
+        else:
+            for j in range(5):
+                b.step(0.01 * j, 0.01)
+        b.check_status()
+        out.append(b.download()[0])
+    assert np.array_equal(out[0].U, out[1].U) and np.array_equal(out[0].S, out[1].S) and np.array_equal(out[0].V, out[1].V)
