@@ -17,6 +17,7 @@
 #include <cooperative_groups.h>
 
 #include "engine_impl.cuh"
+#include "wide.cuh"
 
 namespace cg = cooperative_groups;
 
@@ -512,6 +513,681 @@ __global__ void __launch_bounds__(NT, 3) adjoint_step_kernel(AdjArgs g) {
   }
 }
 
+// ---------------------------------------------------------------------------
+// The same reversal of small batches on thread-block clusters (wide.cuh): four
+// launches, the phases above.  adj_fwd, adj_rev and adj_out give each side of
+// an instance a cluster whose CTAs split its rows (panels in shared memory,
+// the stage inputs in the workspace); adj_core splits the core's entries over
+// one cluster.  The products (T z) G use G = I + E with E applied in FP32
+// while max|E| <= 2^-36, as the forward steps do.  One reverse step at n = m =
+// 2048, r = 32: 37.0 ms on a 2-CTA pair, 2.0 ms here (adj_fwd 0.66, adj_core
+// 0.17, adj_rev 1.03, adj_out 0.15), bound by FP64 issue on 32 SMs.
+// ---------------------------------------------------------------------------
+using wide::load_rows;
+using wide::load_rows_halo;
+using wide::outputs;
+using wide::push_halos;
+using wide::QrSmem;
+using wide::reduce_parts;
+using wide::Team;
+using wide::Tri;
+using wide::WT;
+
+// One side of an instance and its workspace (the layout of adjoint_step_kernel).
+struct WideAdj {
+  int n, m, r, W, N, No;
+  bool kside;
+  const double* X0;   // this side's input basis
+  const double* Xo;   // the other side's
+  const double* S0;
+  double* Xb;         // the adjoint of this side's basis (in: output's, out: input's)
+  double* Sb;
+  double* thb;
+  const double* tri;
+  const double* trio;
+  double* small;
+  double* small1;
+  double* Z;          // stage inputs
+  double* Q;
+  double* xb;
+};
+
+__device__ void wide_adj(const AdjArgs& g, int inst, bool kside, WideAdj& s) {
+  const InstDesc d = g.inst[inst];
+  const int n = d.n, m = d.m, r = d.rcap;
+  s.n = n; s.m = m; s.r = s.W = r; s.kside = kside;
+  s.N = kside ? n : m;
+  s.No = kside ? m : n;
+  s.X0 = kside ? g.U0 + d.offU : g.V0 + d.offV;
+  s.Xo = kside ? g.V0 + d.offV : g.U0 + d.offU;
+  s.S0 = g.S0 + d.offS;
+  s.Xb = kside ? g.Ub + d.offU : g.Vb + d.offV;
+  s.Sb = g.Sb + d.offS;
+  s.thb = g.thb + g.th_off[inst];
+  s.tri = kside ? g.opA + d.offA : g.opB + d.offB;
+  s.trio = kside ? g.opB + d.offB : g.opA + d.offA;
+  double* w = g.work + g.adj_off[inst];
+  s.small = w;
+  s.small1 = w + (int64_t)A_COUNT * r * r;
+  w += 2 * (int64_t)A_COUNT * r * r;
+  const int64_t lenK = (int64_t)n * r, nsK = g.sK.nstages * g.sK.nsub, nsL = g.sL.nstages * g.sL.nsub;
+  if (!kside) w += 3 * (int64_t)n + (nsK + P_COUNT) * lenK;
+  w += 3 * (int64_t)s.N;
+  s.Z = w;
+  const int64_t len = (int64_t)s.N * r;
+  w += (kside ? nsK : nsL) * len;
+  s.Q = w + P_Q * len;
+  s.xb = w + P_XB * len;
+}
+
+// shared memory in doubles: panels, then the small matrices
+__host__ __device__ inline size_t adj_ld(int N, int C) { return (size_t)((((N + C - 1) / C) + 2) | 1); }
+__host__ __device__ inline size_t adj_misc(int N, int r, int C) {
+  const size_t R0 = (N + C - 1) / C, rr = (size_t)r * r;
+  return 4 * rr + (rr + 1) / 2 + (size_t)r * R0 / 2 + 1;  // P, three partials, E, the FP32 copy
+}
+__host__ inline size_t adj_fwd_doubles(int N, int r, int C) {
+  return 4 * adj_ld(N, C) * r + adj_misc(N, r, C) + QrSmem::doubles(C, r);
+}
+__host__ inline size_t adj_rev_doubles(int N, int r, int C) { return 5 * adj_ld(N, C) * r + adj_misc(N, r, C) + r; }
+
+// C E-form operands: Ps[k r + c] = P(c, k) (or P(k, c) with pt), Es = G - I (or
+// its transpose with gt); true when the full product is needed
+__device__ bool load_ep(int r, int W, const double* G, const double* P, bool gt, bool pt, double* Ps, float* Es) {
+  int full = 0;
+  for (int e = threadIdx.x; e < r * r; e += WT) {
+    const int k = e / r, c = e % r;
+    Ps[e] = pt ? P[k + (int64_t)c * W] : P[c + (int64_t)k * W];
+    const double ev = (gt ? G[c + (int64_t)k * W] : G[k + (int64_t)c * W]) - ((k == c) ? 1.0 : 0.0);
+    Es[e] = (float)ev;
+    if (!(fabs(ev) <= 0x1p-36)) full = 1;  // NaN included
+  }
+  return __syncthreads_or(full) != 0;
+}
+
+__global__ void __launch_bounds__(WT, 1) adj_fwd(const __grid_constant__ AdjArgs g, int C) {
+  extern __shared__ __align__(16) double dsm[];
+  Team tm{cg::this_cluster(), (int)cg::this_cluster().block_rank(), C};
+  const int ci = blockIdx.x / C, tid = threadIdx.x;
+  WideAdj s;
+  wide_adj(g, ci >> 1, (ci & 1) == 0, s);
+  const int r = s.r, W = s.W, N = s.N, No = s.No, rr = r * r;
+  const int R0 = tm.rows_per(N), lo = tm.lo(N), rows = tm.hi(N) - lo, ld = (int)adj_ld(N, C);
+  const int64_t len = (int64_t)N * r;
+  const Tri T{s.tri, N, lo};
+  double* p0 = dsm;
+  double* p1 = p0 + (size_t)r * ld;
+  double* y = p1 + (size_t)r * ld;
+  double* acc = y + (size_t)r * ld;
+  double* misc = acc + (size_t)r * ld;
+  const QrSmem qs = QrSmem::carve(misc + adj_misc(N, r, C), C, r);
+  double* Gg = blkp(s.small, W, s.kside ? A_GV : A_GU);  // G, then P
+  tm.cl.sync();  // every CTA runs before any distributed access
+  {
+    // projections of the other input basis, in blocks of at most R0 rows
+    const int lo2 = tm.lo(No), hi2 = tm.hi(No);
+    double* part = misc;
+    for (int e = tid; e < 2 * rr; e += WT) part[e] = 0.0;
+    for (int b = lo2; b < hi2; b += R0) {
+      const int nb = min(R0, hi2 - b);
+      __syncthreads();
+      load_rows_halo(s.Xo, No, b, nb, r, p0, ld);
+      __syncthreads();
+      const Tri To{s.trio, No, b};
+      for (int e = tid; e < nb * r; e += WT) p1[(e / nb) * ld + 1 + e % nb] = To.mul(p0, ld, e % nb, e / nb);
+      __syncthreads();
+      for (int o = tid; o < 2 * rr; o += WT) {
+        const int a = o % r, c = (o / r) % r;
+        if (o < rr && a > c) continue;  // G is symmetric
+        const double* x = (o < rr) ? p0 : p1;
+        double v = part[o];
+        for (int i = 1; i <= nb; ++i) v = fma(p0[a * ld + i], x[c * ld + i], v);
+        part[o] = v;
+      }
+    }
+    __syncthreads();
+    reduce_parts(tm, part, 2 * rr, [&](int e, double v) {
+      const int a = e % r, c = (e / r) % r;
+      if (e >= rr) Gg[(int64_t)W * W + a + (int64_t)c * W] = v;
+      else if (a <= c) Gg[a + (int64_t)c * W] = Gg[c + (int64_t)a * W] = v;
+    });
+  }
+  // zero halo rows at the ends of the domain (never pushed to)
+  for (int e = tid; e < 2 * r; e += WT) {
+    double* p = (e < r) ? p0 : p1;
+    const int k = e % r;
+    p[k * ld] = 0.0;
+    p[k * ld + 1 + R0] = 0.0;
+    if (rows < R0) p[k * ld + 1 + rows] = 0.0;
+  }
+  // K0 = U0 S0 (L0 = V0 S0^T)
+  double* Ps = misc;
+  for (int e = tid; e < rr; e += WT) {
+    const int k = e / r, c = e % r;
+    Ps[e] = s.kside ? s.S0[k + (int64_t)c * r] : s.S0[c + (int64_t)k * r];
+  }
+  load_rows(s.X0, N, lo, rows, r, p1, ld);
+  __syncthreads();
+  for (int e = tid; e < rows * r; e += WT) {
+    const int i = e % rows, c = e / rows;
+    double v = 0.0;
+    for (int k = 0; k < r; ++k) v = fma(p1[k * ld + 1 + i], Ps[k * r + c], v);
+    p0[c * ld + 1 + i] = y[c * ld + 1 + i] = v;
+    s.Z[lo + i + (int64_t)c * N] = v;
+  }
+  __syncthreads();
+  float* Es = reinterpret_cast<float*>(misc + 4 * rr);
+  float* tf = reinterpret_cast<float*>(misc + 4 * rr + (rr + 1) / 2);
+  const bool full = load_ep(r, W, Gg, Gg + (int64_t)W * W, false, false, Ps, Es);
+  tm.cl.sync();  // the zero halo rows of every CTA are set
+  push_halos(tm, N, rows, r, p0, ld);
+  tm.cl.sync();
+  // stage-form RK of y' = T y G + y P^T, every stage input to the workspace
+  const Scheme& sc = s.kside ? g.sK : g.sL;
+  const double h = g.dt / sc.nsub;
+  double* win = p0;
+  double* wout = p1;
+  for (int sub = 0; sub < sc.nsub; ++sub)
+    for (int st = 0; st < sc.nstages; ++st) {
+      int big = full;
+      if (!full) {
+        for (int e = tid; e < rows * r; e += WT) {
+          const int i = e % rows, k = e / rows;
+          const double tw = T.mul(win, ld, i, k);
+          wout[k * ld + 1 + i] = tw;
+          tf[e] = (float)tw;
+          big |= !(fabs(tw) < 0x1p100);
+        }
+        big = __syncthreads_or(big);
+      }
+      const bool last = st + 1 == sc.nstages, end = last && sub + 1 == sc.nsub;
+      const double bs = sc.b[st], ha = last ? 0.0 : h * sc.a[st + 1];
+      double* Zn = s.Z + (int64_t)(sub * sc.nstages + st + 1) * len;
+      for (int e = tid; e < rows * r; e += WT) {
+        const int i = e % rows, c = e / rows, o = c * ld + 1 + i;
+        double v;
+        if (!big) {
+          float ef = 0.0f;
+          for (int k = 0; k < r; ++k) ef = fmaf(tf[k * rows + i], Es[k * r + c], ef);
+          v = wout[o] + (double)ef;
+        } else {
+          v = 0.0;
+          for (int k = 0; k < r; ++k) v = fma(T.mul(win, ld, i, k), Gg[k + (int64_t)c * W], v);
+        }
+        for (int k = 0; k < r; ++k) v = fma(win[k * ld + 1 + i], Ps[k * r + c], v);
+        const double a = (st == 0) ? bs * v : fma(bs, v, acc[o]);
+        acc[o] = a;
+        double z;
+        if (last) y[o] = z = fma(h, a, y[o]);
+        else z = fma(ha, v, y[o]);
+        wout[o] = z;
+        if (!end) Zn[lo + i + (int64_t)c * N] = z;
+        if (i == 0 && tm.q > 0) tm.at(wout, tm.q - 1)[c * ld + 1 + R0] = z;
+        if (i == rows - 1 && tm.q + 1 < C && lo + rows < N) tm.at(wout, tm.q + 1)[c * ld] = z;
+      }
+      tm.cl.sync();
+      double* t = win;
+      win = wout;
+      wout = t;
+    }
+  wide::qr(tm, N, lo, rows, r, win + 1, ld, wout + 1, blkp(s.small, W, s.kside ? A_RK : A_RL), W, qs);
+  // M = Q^T X0 and the projections of Q
+  double* Q = wout;
+  double* part = misc;
+  load_rows(s.X0, N, lo, rows, r, win, ld);
+  push_halos(tm, N, rows, r, Q, ld);
+  tm.cl.sync();
+  for (int e = tid; e < rows * r; e += WT) {
+    const int i = e % rows, k = e / rows;
+    y[k * ld + 1 + i] = T.mul(Q, ld, i, k);
+    s.Q[lo + i + (int64_t)k * N] = Q[k * ld + 1 + i];
+  }
+  __syncthreads();
+  outputs(3 * rr, [&](int o, int l, int L) {
+    const int a = o % r, c = (o / r) % r, w = o / rr;
+    if (w == 1 && a > c) return 0.0;
+    const double* x = (w == 0) ? win : (w == 1 ? Q : y);
+    double v = 0.0;
+    for (int i = 1 + l; i <= rows; i += L) v = fma(Q[a * ld + i], x[c * ld + i], v);
+    return v;
+  }, [&](int o, double v) { part[o] = v; });
+  double* Mo = blkp(s.small, W, s.kside ? A_M : A_N);
+  double* Gn = blkp(s.small, W, s.kside ? A_GU1 : A_GV1);
+  double* Pn = blkp(s.small, W, s.kside ? A_PU1 : A_PV1);
+  reduce_parts(tm, part, 3 * rr, [&](int e, double v) {
+    const int a = e % r, c = (e / r) % r, w = e / rr;
+    if (w == 0) Mo[a + (int64_t)c * W] = v;
+    else if (w == 2) Pn[a + (int64_t)c * W] = v;
+    else if (a <= c) Gn[a + (int64_t)c * W] = Gn[c + (int64_t)a * W] = v;
+  });
+}
+
+// C = alpha op(A) op(B) over this CTA's share of the entries (r x r, ld W);
+// fin(entry offset, value) stores it
+template <class F>
+__device__ __forceinline__ void dgemm(const Team& tm, int r, int W, const double* A, bool ta, const double* B, bool tb,
+                                      const F& fin) {
+  const int per = (r * r + tm.C - 1) / tm.C, e0 = tm.q * per, e1 = min(r * r, e0 + per);
+  outputs(max(0, e1 - e0), [&](int o, int l, int L) {
+    const int i = (e0 + o) % r, j = (e0 + o) / r;
+    double v = 0.0;
+    for (int k = l; k < r; k += L)
+      v = fma(ta ? A[k + (int64_t)i * W] : A[i + (int64_t)k * W], tb ? B[j + (int64_t)k * W] : B[k + (int64_t)j * W], v);
+    return v;
+  }, [&](int o, double v) { fin((e0 + o) % r + (int64_t)((e0 + o) / r) * W, v); });
+}
+
+// Phase 2: the S step forward and reversed; entries split over one cluster,
+// intermediates in the scratch blocks, a cluster barrier after each group of
+// independent products.
+__global__ void __launch_bounds__(WT, 1) adj_core(const __grid_constant__ AdjArgs g, int C) {
+  Team tm{cg::this_cluster(), (int)cg::this_cluster().block_rank(), C};
+  WideAdj s;
+  wide_adj(g, blockIdx.x / C, true, s);
+  const int r = s.r, W = s.W;
+  auto B = [&](int i) { return blkp(s.small, W, i); };
+  auto t = [&](int i) { return blkp(s.small1, W, A_SST + i); };  // the L side's copy: scratch here
+  auto put = [](double* d) { return [d](int64_t e, double v) { d[e] = v; }; };
+  const double* S0 = s.S0;  // ld r = W
+  const Scheme& sc = g.sS;
+  const int ns = sc.nstages;
+  const double h = g.dt / sc.nsub;
+  dgemm(tm, r, W, S0, false, B(A_N), true, put(t(0)));
+  tm.sync();
+  dgemm(tm, r, W, B(A_M), false, t(0), false, put(B(A_SST)));
+  tm.sync();
+  double* acc = B(A_SACC);
+  for (int sub = 0; sub < sc.nsub; ++sub) {
+    const double* y = B(A_SST + sub * ns);
+    for (int st = 0; st < ns; ++st) {
+      const double* z = B(A_SST + sub * ns + st);
+      dgemm(tm, r, W, B(A_PU1), false, z, false, put(t(0)));
+      dgemm(tm, r, W, B(A_GU1), false, z, false, put(t(1)));
+      tm.sync();
+      double* k1 = t(2);
+      dgemm(tm, r, W, t(0), false, B(A_GV1), false, put(k1));
+      __syncthreads();  // k1's entries may be another thread's of this CTA
+      dgemm(tm, r, W, t(1), false, B(A_PV1), true, [&](int64_t e, double v) {
+        v += k1[e];
+        const double a = (st == 0) ? sc.b[0] * v : fma(sc.b[st], v, acc[e]);
+        acc[e] = a;
+        if (st + 1 < ns) B(A_SST + sub * ns + st + 1)[e] = fma(h * sc.a[st + 1], v, y[e]);
+        else if (sub + 1 < sc.nsub) B(A_SST + (sub + 1) * ns)[e] = fma(h, a, y[e]);
+      });
+      tm.sync();
+    }
+  }
+  // reversed: Sbar = S1_bar -> S~0_bar, coefficient gradients
+  double* Sbar = B(A_SB);
+  double* ybn = B(A_SYB);
+  double* kb = B(A_SKB);
+  double* zb = B(A_SZB);
+  const int per = (r * r + C - 1) / C, e0 = tm.q * per, e1 = min(r * r, e0 + per);
+  for (int o = e0 + threadIdx.x; o < e1; o += WT) {
+    const int64_t e = o % r + (int64_t)(o / r) * W;
+    Sbar[e] = s.Sb[e];
+    for (int b = A_CPU; b <= A_CPV; ++b) B(b)[e] = 0.0;
+  }
+  __syncthreads();
+  for (int sub = sc.nsub - 1; sub >= 0; --sub) {
+    for (int st = ns - 1; st >= 0; --st) {
+      const double* z = B(A_SST + sub * ns + st);
+      for (int o = e0 + threadIdx.x; o < e1; o += WT) {
+        const int64_t e = o % r + (int64_t)(o / r) * W;
+        if (st == ns - 1) ybn[e] = Sbar[e];
+        kb[e] = h * sc.b[st] * ybn[e] + ((st + 1 < ns) ? h * sc.a[st + 1] * zb[e] : 0.0);
+      }
+      tm.sync();
+      dgemm(tm, r, W, kb, false, B(A_GV1), true, put(t(0)));
+      dgemm(tm, r, W, B(A_PU1), false, z, false, put(t(1)));
+      dgemm(tm, r, W, kb, false, B(A_PV1), false, put(t(2)));
+      dgemm(tm, r, W, B(A_GU1), false, z, false, put(t(3)));
+      dgemm(tm, r, W, B(A_PU1), true, kb, false, put(t(4)));
+      dgemm(tm, r, W, B(A_GU1), true, kb, false, put(t(5)));
+      tm.sync();
+      auto add = [](double* d) { return [d](int64_t e, double v) { d[e] += v; }; };
+      dgemm(tm, r, W, t(0), false, z, true, add(B(A_CPU)));
+      dgemm(tm, r, W, t(1), true, kb, false, add(B(A_CGV)));
+      dgemm(tm, r, W, t(2), false, z, true, add(B(A_CGU)));
+      dgemm(tm, r, W, kb, true, t(3), false, add(B(A_CPV)));
+      dgemm(tm, r, W, t(4), false, B(A_GV1), true, put(t(6)));
+      __syncthreads();
+      dgemm(tm, r, W, t(5), false, B(A_PV1), false, [&](int64_t e, double v) {
+        v += t(6)[e];
+        zb[e] = v;
+        Sbar[e] += v;
+      });
+      tm.sync();  // kb is rewritten next
+    }
+  }
+  // S~0 = M S0 N^T:  Mb = St0b N S0^T, Nb = St0b^T M S0, S0b = M^T St0b N
+  dgemm(tm, r, W, B(A_N), false, S0, true, put(t(0)));
+  dgemm(tm, r, W, B(A_M), false, S0, false, put(t(1)));
+  dgemm(tm, r, W, Sbar, false, B(A_N), false, put(t(2)));
+  tm.sync();
+  dgemm(tm, r, W, Sbar, false, t(0), false, put(B(A_MB)));
+  dgemm(tm, r, W, Sbar, true, t(1), false, put(B(A_NB)));
+  dgemm(tm, r, W, B(A_M), true, t(2), false, put(B(A_S0B)));
+}
+
+// out(i, c) of this CTA's rows: x + sum_k [T X](i, k) C1(c, k) + X(i, k) C2(k, c) +
+// [T^T X](i, k) C1(k, c), the adjoint of G = X^T X (C2 = Gbar + Gbar^T) and P = X^T T X
+// (C1 = Pbar); C1s, C2s at k r + c
+__device__ __forceinline__ double proj_adj(const double* X, const double* TX, const double* TtX, int ld, int r, int i,
+                                           int c, const double* C1s, const double* C2s, double x) {
+  for (int k = 0; k < r; ++k) {
+    const int o = k * ld + 1 + i;
+    x = fma(TX[o], C1s[c * r + k], x);
+    x = fma(X[o], C2s[k * r + c], x);
+    x = fma(TtX[o], C1s[k * r + c], x);
+  }
+  return x;
+}
+
+// theta_bar[lo + i] += sum_c X(i, c) sum_k X(i, k) C1(c, k)
+__device__ void theta_proj(const Team& tm, int rows, int lo, int r, const double* X, int ld, const double* C1s,
+                           double* scr, double* thb) {
+  for (int e = threadIdx.x; e < rows * r; e += WT) {
+    const int i = e % rows, c = e / rows;
+    double v = 0.0;
+    for (int k = 0; k < r; ++k) v = fma(X[k * ld + 1 + i], C1s[c * r + k], v);
+    scr[c * ld + 1 + i] = v * X[c * ld + 1 + i];
+  }
+  __syncthreads();
+  outputs(rows, [&](int i, int l, int L) {
+    double v = 0.0;
+    for (int c = l; c < r; c += L) v += scr[c * ld + 1 + i];
+    return v;
+  }, [&](int i, double v) { thb[lo + i] += v; });
+  __syncthreads();
+}
+
+// small matrix (ld W) to Ms[k r + c]; sym: M + M^T
+__device__ __forceinline__ void load_small(int r, int W, const double* M, bool sym, double* Ms) {
+  for (int e = threadIdx.x; e < r * r; e += WT) {
+    const int k = e / r, c = e % r;
+    Ms[e] = M[k + (int64_t)c * W] + (sym ? M[c + (int64_t)k * W] : 0.0);
+  }
+}
+
+__global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs g, int C) {
+  extern __shared__ __align__(16) double dsm[];
+  Team tm{cg::this_cluster(), (int)cg::this_cluster().block_rank(), C};
+  const int ci = blockIdx.x / C, tid = threadIdx.x;
+  WideAdj s;
+  wide_adj(g, ci >> 1, (ci & 1) == 0, s);
+  const int r = s.r, W = s.W, N = s.N, rr = r * r;
+  const int lo = tm.lo(N), rows = tm.hi(N) - lo, ld = (int)adj_ld(N, C);
+  const int64_t len = (int64_t)N * r;
+  const Tri T{s.tri, N, lo};
+  double* p0 = dsm;
+  double* p1 = p0 + (size_t)r * ld;
+  double* yb = p1 + (size_t)r * ld;
+  double* p3 = yb + (size_t)r * ld;
+  double* p4 = p3 + (size_t)r * ld;
+  double* misc = p4 + (size_t)r * ld;
+  double* inv = misc + adj_misc(N, r, C);
+  tm.cl.sync();
+  // Q_bar = output's adjoint + X0 Mb^T + adjoint of the projections of Q; the
+  // first part of X0_bar: Q Mb
+  double* Mb = misc;
+  double* C1s = misc + rr;
+  double* C2s = misc + 2 * rr;
+  load_small(r, W, blkp(s.small, W, s.kside ? A_MB : A_NB), false, Mb);
+  load_small(r, W, blkp(s.small, W, s.kside ? A_CPU : A_CPV), false, C1s);
+  load_small(r, W, blkp(s.small, W, s.kside ? A_CGU : A_CGV), true, C2s);
+  load_rows_halo(s.Q, N, lo, rows, r, p0, ld);
+  load_rows(s.X0, N, lo, rows, r, p1, ld);
+  __syncthreads();
+  for (int e = tid; e < rows * r; e += WT) {
+    const int i = e % rows, k = e / rows;
+    p3[k * ld + 1 + i] = T.mul(p0, ld, i, k);
+    p4[k * ld + 1 + i] = T.mul_t(p0, ld, i, k);
+  }
+  __syncthreads();
+  for (int e = tid; e < rows * r; e += WT) {
+    const int i = e % rows, c = e / rows;
+    double v = s.Xb[lo + i + (int64_t)c * N], x = 0.0;
+    for (int k = 0; k < r; ++k) {
+      v = fma(p1[k * ld + 1 + i], Mb[c * r + k], v);
+      x = fma(p0[k * ld + 1 + i], Mb[k * r + c], x);
+    }
+    yb[c * ld + 1 + i] = proj_adj(p0, p3, p4, ld, r, i, c, C1s, C2s, v);
+    s.xb[lo + i + (int64_t)c * N] = x;
+  }
+  __syncthreads();
+  if (s.kside) theta_proj(tm, rows, lo, r, p0, ld, C1s, p1, s.thb);
+  // QR adjoint: yb <- (yb + Q copyltu(-yb^T Q)) R^-T
+  {
+    double* part = misc + 2 * rr;
+    __syncthreads();
+    outputs(rr, [&](int o, int l, int L) {
+      const int a = o % r, c = o / r;
+      double v = 0.0;
+      for (int i = 1 + l; i <= rows; i += L) v = fma(-yb[a * ld + i], p0[c * ld + i], v);
+      return v;
+    }, [&](int o, double v) { part[o] = v; });
+    double* Mx = blkp(s.kside ? s.small : s.small1, W, A_T1);
+    reduce_parts(tm, part, rr, [&](int e, double v) { Mx[e % r + (int64_t)(e / r) * W] = v; });
+    const double* R = blkp(s.small, W, s.kside ? A_RK : A_RL);
+    double* Cl = misc;
+    double* Rs = misc + rr;  // Rs[k r + j] = R(k, j)
+    for (int e = tid; e < rr; e += WT) {
+      const int k = e / r, c = e % r;
+      Cl[e] = (k >= c) ? Mx[k + (int64_t)c * W] : Mx[c + (int64_t)k * W];
+      Rs[e] = R[k + (int64_t)c * W];
+    }
+    if (tid < r) inv[tid] = 1.0 / R[tid + (int64_t)tid * W];
+    __syncthreads();
+    for (int e = tid; e < rows * r; e += WT) {
+      const int i = e % rows, c = e / rows;
+      double v = yb[c * ld + 1 + i];
+      for (int k = 0; k < r; ++k) v = fma(p0[k * ld + 1 + i], Cl[k * r + c], v);
+      yb[c * ld + 1 + i] = v;
+    }
+    __syncthreads();
+    // back substitution along each row, two lanes per row
+    for (int i0 = 0; i0 < rows; i0 += WT / 2) {
+      const int i = i0 + (tid >> 1), l = tid & 1;
+      const bool in = i < rows;
+      for (int k = r - 1; k >= 0; --k) {
+        double v = 0.0;
+        if (in)
+          for (int j = k + 1 + l; j < r; j += 2) v = fma(yb[j * ld + 1 + i], Rs[k * r + j], v);
+        v += __shfl_xor_sync(0xffffffffu, v, 1);
+        if (in && l == 0) yb[k * ld + 1 + i] = (yb[k * ld + 1 + i] - v) * inv[k];
+        __syncwarp();
+      }
+    }
+    __syncthreads();
+  }
+  // RK reversal: kb = h b_s yb' + h a_{s+1} zb_{s+1}; Gbar += (T z)^T kb,
+  // Pbar += kb^T z, theta_bar += kb . (z G); zb = T^T kb G^T + kb P; yb += zb
+  const double* Gg = blkp(s.small, W, s.kside ? A_GV : A_GU);
+  double* Ps = misc;
+  double* part = misc + rr;
+  float* Es = reinterpret_cast<float*>(misc + 4 * rr);
+  float* tf = reinterpret_cast<float*>(misc + 4 * rr + (rr + 1) / 2);
+  const bool full = load_ep(r, W, Gg, Gg + (int64_t)W * W, true, true, Ps, Es);
+  for (int e = tid; e < 3 * rr; e += WT) part[e] = 0.0;
+  const Scheme& sc = s.kside ? g.sK : g.sL;
+  const double h = g.dt / sc.nsub;
+  double* kb = p0;
+  double* ybn = p1;
+  double* z = p4;
+  // kb's halo rows: zero at the ends of the domain (no neighbour pushes there)
+  tm.cl.sync();  // every CTA is past its reads of Q's halo rows
+  for (int e = tid; e < r; e += WT) {
+    kb[e * ld] = 0.0;
+    kb[e * ld + 1 + tm.rows_per(N)] = 0.0;
+    kb[e * ld + 1 + rows] = 0.0;
+  }
+  tm.cl.sync();
+  for (int sub = sc.nsub - 1; sub >= 0; --sub) {
+    for (int e = tid; e < rows * r; e += WT) {
+      const int o = (e / rows) * ld + 1 + e % rows;
+      ybn[o] = yb[o];
+    }
+    for (int st = sc.nstages - 1; st >= 0; --st) {
+      const double hb = h * sc.b[st], ha = (st + 1 < sc.nstages) ? h * sc.a[st + 1] : 0.0;
+      for (int e = tid; e < rows * r; e += WT) {  // every thread its own entries
+        const int o = (e / rows) * ld + 1 + e % rows;
+        kb[o] = (st + 1 < sc.nstages) ? fma(ha, p3[o], hb * ybn[o]) : hb * ybn[o];
+      }
+      load_rows_halo(s.Z + (int64_t)(sub * sc.nstages + st) * len, N, lo, rows, r, z, ld);
+      __syncthreads();
+      push_halos(tm, N, rows, r, kb, ld);
+      int zbig = full;
+      for (int e = tid; e < rows * r; e += WT) {
+        const int o = (e / rows) * ld + 1 + e % rows;
+        p3[o] = T.mul(z, ld, e % rows, e / rows);
+        zbig |= !(fabs(z[o]) < 0x1p100);
+      }
+      tm.cl.sync();
+      outputs(2 * rr, [&](int o, int l, int L) {
+        const int a = o % r, c = (o / r) % r;
+        const double* x = (o < rr) ? p3 : kb;
+        const double* y = (o < rr) ? kb : z;
+        double v = 0.0;
+        for (int i = 1 + l; i <= rows; i += L) v = fma(x[a * ld + i], y[c * ld + i], v);
+        return v;
+      }, [&](int o, double v) { part[o] += v; });
+      zbig = __syncthreads_or(zbig);  // T z is consumed
+      if (s.kside) {
+        for (int e = tid; e < rows * r; e += WT) {
+          const int i = e % rows, c = e / rows;
+          double v;
+          if (!zbig) {
+            float ef = 0.0f;  // Es holds the transpose of G - I
+            for (int k = 0; k < r; ++k) ef = fmaf((float)z[k * ld + 1 + i], Es[c * r + k], ef);
+            v = z[c * ld + 1 + i] + (double)ef;
+          } else {
+            v = 0.0;
+            for (int k = 0; k < r; ++k) v = fma(z[k * ld + 1 + i], Gg[k + (int64_t)c * W], v);
+          }
+          p3[c * ld + 1 + i] = v * kb[c * ld + 1 + i];
+        }
+        __syncthreads();
+        outputs(rows, [&](int i, int l, int L) {
+          double v = 0.0;
+          for (int c = l; c < r; c += L) v += p3[c * ld + 1 + i];
+          return v;
+        }, [&](int i, double v) { s.thb[lo + i] += v; });
+        __syncthreads();
+      }
+      int big = full;
+      if (!full) {
+        for (int e = tid; e < rows * r; e += WT) {
+          const int i = e % rows, k = e / rows;
+          const double tk = T.mul_t(kb, ld, i, k);
+          p3[k * ld + 1 + i] = tk;
+          tf[e] = (float)tk;
+          big |= !(fabs(tk) < 0x1p100);
+        }
+        big = __syncthreads_or(big);
+      }
+      for (int e = tid; e < rows * r; e += WT) {
+        const int i = e % rows, c = e / rows, o = c * ld + 1 + i;
+        double v;
+        if (!big) {
+          float ef = 0.0f;
+          for (int k = 0; k < r; ++k) ef = fmaf(tf[k * rows + i], Es[k * r + c], ef);
+          v = p3[o] + (double)ef;
+        } else {
+          v = 0.0;
+          for (int k = 0; k < r; ++k) v = fma(T.mul_t(kb, ld, i, k), Gg[c + (int64_t)k * W], v);
+        }
+        for (int k = 0; k < r; ++k) v = fma(kb[k * ld + 1 + i], Ps[k * r + c], v);
+        p3[o] = v;
+        yb[o] += v;
+      }
+      tm.cl.sync();  // kb and its halo rows are rewritten next
+    }
+  }
+  // X0_bar += y0_bar S0^T (K) or S0 (L); S0_bar's part: X0^T y0_bar (K) or its transpose
+  for (int e = tid; e < rr; e += WT) {
+    const int k = e / r, c = e % r;
+    Ps[e] = s.kside ? s.S0[c + (int64_t)k * r] : s.S0[k + (int64_t)c * r];
+  }
+  load_rows(s.X0, N, lo, rows, r, p4, ld);
+  __syncthreads();
+  for (int e = tid; e < rows * r; e += WT) {
+    const int i = e % rows, c = e / rows;
+    double v = s.xb[lo + i + (int64_t)c * N];
+    for (int k = 0; k < r; ++k) v = fma(yb[k * ld + 1 + i], Ps[k * r + c], v);
+    s.xb[lo + i + (int64_t)c * N] = v;
+  }
+  outputs(rr, [&](int o, int l, int L) {
+    const int a = o % r, c = o / r;
+    const double* x = s.kside ? p4 : yb;
+    const double* y = s.kside ? yb : p4;
+    double v = 0.0;
+    for (int i = 1 + l; i <= rows; i += L) v = fma(x[a * ld + i], y[c * ld + i], v);
+    return v;
+  }, [&](int o, double v) { part[2 * rr + o] = v; });
+  double* Gb = blkp(s.small, W, s.kside ? A_KG : A_LG);
+  double* Pb = blkp(s.small, W, s.kside ? A_KP : A_LP);
+  double* S0b = s.kside ? blkp(s.small, W, A_S0B) : blkp(s.small1, W, A_S0B);
+  reduce_parts(tm, part, 3 * rr, [&](int e, double v) {
+    const int64_t o = e % r + (int64_t)((e / r) % r) * W;
+    if (e < rr) Gb[o] = v;
+    else if (e < 2 * rr) Pb[o] = v;
+    else S0b[o] = s.kside ? S0b[o] + v : v;
+  });
+}
+
+__global__ void __launch_bounds__(WT, 1) adj_out(const __grid_constant__ AdjArgs g, int C) {
+  extern __shared__ __align__(16) double dsm[];
+  Team tm{cg::this_cluster(), (int)cg::this_cluster().block_rank(), C};
+  const int ci = blockIdx.x / C, tid = threadIdx.x;
+  WideAdj s;
+  wide_adj(g, ci >> 1, (ci & 1) == 0, s);
+  const int r = s.r, W = s.W, N = s.N, rr = r * r;
+  const int lo = tm.lo(N), rows = tm.hi(N) - lo, ld = (int)adj_ld(N, C);
+  const Tri T{s.tri, N, lo};
+  double* p0 = dsm;
+  double* p3 = p0 + (size_t)r * ld;
+  double* p4 = p3 + (size_t)r * ld;
+  double* C1s = p4 + (size_t)r * ld;
+  double* C2s = C1s + rr;
+  // adjoint of the other side's projections of this side's input basis
+  load_small(r, W, blkp(s.small, W, s.kside ? A_LP : A_KP), false, C1s);
+  load_small(r, W, blkp(s.small, W, s.kside ? A_LG : A_KG), true, C2s);
+  load_rows_halo(s.X0, N, lo, rows, r, p0, ld);
+  __syncthreads();
+  for (int e = tid; e < rows * r; e += WT) {
+    const int i = e % rows, k = e / rows;
+    p3[k * ld + 1 + i] = T.mul(p0, ld, i, k);
+    p4[k * ld + 1 + i] = T.mul_t(p0, ld, i, k);
+  }
+  __syncthreads();
+  for (int e = tid; e < rows * r; e += WT) {
+    const int i = e % rows, c = e / rows;
+    const int64_t o = lo + i + (int64_t)c * N;
+    s.Xb[o] = proj_adj(p0, p3, p4, ld, r, i, c, C1s, C2s, s.xb[o]);
+  }
+  __syncthreads();
+  if (s.kside) theta_proj(tm, rows, lo, r, p0, ld, C1s, p3, s.thb);
+  if (!s.kside) {
+    const double* a = blkp(s.small, W, A_S0B);
+    const double* b = blkp(s.small1, W, A_S0B);
+    for (int e = tm.q * WT + tid; e < rr; e += C * WT) {
+      const int64_t o = e % r + (int64_t)(e / r) * W;
+      s.Sb[o] = a[o] + b[o];
+    }
+  }
+}
+
+cudaError_t adj_launch(void (*kern)(const AdjArgs, int), const AdjArgs& g, int blocks, int C, size_t smem,
+                       std::atomic<uint64_t>& done, cudaStream_t st) {
+  cudaError_t e = wide::cluster_attributes(kern, done);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  wide::cluster_config(cfg, attr, blocks, C, smem, st);
+  return cudaLaunchKernelEx(&cfg, kern, g, C);
+}
+
 }  // namespace
 
 size_t adjoint_work_elems(int64_t n, int64_t m, int64_t r, int ns_k, int ns_l) {
@@ -521,11 +1197,36 @@ size_t adjoint_work_elems(int64_t n, int64_t m, int64_t r, int ns_k, int ns_l) {
 
 int adjoint_max_stages() { return kAdjMaxStages; }
 
+WidePlan adjoint_plan(const WidePlan& step, int count, const int64_t* n, const int64_t* m, const int64_t* r) {
+  WidePlan p;
+  p.C = step.C;
+  for (int i = 0; i < count && p.C; ++i)
+    for (int64_t N : {n[i], m[i]}) {
+      const int ri = (int)r[i];
+      p.side_smem = std::max(p.side_smem, sizeof(double) * adj_fwd_doubles((int)N, ri, p.C));
+      p.core_smem = std::max(p.core_smem, sizeof(double) * adj_rev_doubles((int)N, ri, p.C));
+    }
+  if (p.side_smem > kWideSmemMax || p.core_smem > kWideSmemMax) return WidePlan{};
+  p.side_smem = std::max(p.side_smem, (size_t)120 * 1024);  // a CTA per SM
+  p.core_smem = std::max(p.core_smem, (size_t)120 * 1024);
+  return p;
+}
+
 cudaError_t launch_adjoint_step(const InstDesc* inst, const int64_t* adj_off, const int64_t* th_off, int count,
                                 const double* U0, const double* S0, const double* V0, double* Ub, double* Sb,
                                 double* Vb, double* thb, const double* opA, const double* opB, double* work,
-                                const Scheme& sK, const Scheme& sL, const Scheme& sS, double dt, cudaStream_t st) {
+                                const Scheme& sK, const Scheme& sL, const Scheme& sS, double dt, const WidePlan& plan,
+                                cudaStream_t st) {
   AdjArgs g{inst, adj_off, th_off, U0, S0, V0, Ub, Sb, Vb, thb, opA, opB, work, sK, sL, sS, dt, 0};
+  if (plan.C) {
+    static std::atomic<uint64_t> d0{0}, d1{0}, d2{0}, d3{0};
+    const int C = plan.C;
+    cudaError_t e = adj_launch(adj_fwd, g, 2 * C * count, C, plan.side_smem, d0, st);
+    if (e == cudaSuccess) e = adj_launch(adj_core, g, C * count, C, 0, d1, st);
+    if (e == cudaSuccess) e = adj_launch(adj_rev, g, 2 * C * count, C, plan.core_smem, d2, st);
+    if (e == cudaSuccess) e = adj_launch(adj_out, g, 2 * C * count, C, plan.core_smem, d3, st);
+    return e != cudaSuccess ? e : cudaGetLastError();
+  }
   const size_t smem = sizeof(Smem<double>);
   // Batches small enough that every instance can have two SMs run the K and
   // L sides on a 2-CTA cluster each.  Its CTAs ask for more shared memory

@@ -53,6 +53,7 @@ struct lri_batch {
   const void* opB = nullptr;
   bool bound = false;
   bool data_ready = false;
+  lri::WidePlan adj_wide;   // the same for the adjoint step
   lri::WidePlan wide;       // clusters of small FP64 BUG batches (C = 0: the step kernel)
   int32_t ctas_per_sm = 3;  // register budget of the step kernel (lri_batch_set_occupancy)
   // discrete adjoint (allocated by lri_batch_adjoint_prepare)
@@ -292,6 +293,7 @@ lri_status lri_batch_create(lri_batch** out, const lri_batch_desc* desc, const l
     if (cudaGetDevice(&dev) == cudaSuccess &&
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
       b->wide = lri::wide_plan(count, b->n.data(), b->m.data(), b->rcap.data(), sms);
+    b->adj_wide = lri::adjoint_plan(b->wide, count, b->n.data(), b->m.data(), b->rcap.data());
   }
   // longest-processing-time-first launch order: CTAs start in block order
   b->order.resize(count);
@@ -598,7 +600,7 @@ lri_status lri_batch_adjoint_step(lri_batch* b, double dt, const void* U0, const
       static_cast<const double*>(V0), static_cast<double*>(Ubar), static_cast<double*>(Sbar),
       static_cast<double*>(Vbar), static_cast<double*>(theta_bar), static_cast<const double*>(b->opA),
       static_cast<const double*>(b->opB), b->d_adj_work, to_scheme(b->alg.K_alg), to_scheme(b->alg.L_alg),
-      to_scheme(b->alg.S_alg), dt, (cudaStream_t)stream));
+      to_scheme(b->alg.S_alg), dt, b->adj_wide, (cudaStream_t)stream));
 }
 
 // ---------------------------------------------------------------------------

@@ -136,6 +136,10 @@ int adjoint_max_stages();
 cudaError_t launch_adjoint_step(const InstDesc* inst, const int64_t* adj_off, const int64_t* th_off, int count,
                                 const double* U0, const double* S0, const double* V0, double* Ub, double* Sb,
                                 double* Vb, double* thb, const double* opA, const double* opB, double* work,
-                                const Scheme& sK, const Scheme& sL, const Scheme& sS, double dt, cudaStream_t st);
+                                const Scheme& sK, const Scheme& sL, const Scheme& sS, double dt, const WidePlan& plan,
+                                cudaStream_t st);
+// the adjoint's plan on clusters for a batch whose steps take `step` (side_smem:
+// the forward recomputation, core_smem: the reversal); C = 0 where it does not fit
+WidePlan adjoint_plan(const WidePlan& step, int count, const int64_t* n, const int64_t* m, const int64_t* r);
 
 }  // namespace lri

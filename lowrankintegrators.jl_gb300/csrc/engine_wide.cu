@@ -25,10 +25,13 @@
 namespace lri {
 namespace {
 
+using wide::load_rows;
 using wide::outputs;
+using wide::push_halos;
 using wide::QrSmem;
 using wide::reduce_parts;
 using wide::Team;
+using wide::Tri;
 using wide::WT;
 
 // small-scratch block indices shared with the instance engine
@@ -87,16 +90,10 @@ __device__ void wide_horner(const Scheme& sc, double gam[5]) {
   }
 }
 
-// The cluster's rows of one side in shared memory: panels p[k ld + 1 + i] with
-// a halo row on each side (i = -1 and i = R0).
-struct SideSmem {
-  int ld;
-  double* p0;
-  double* p1;
-  double* p2;
-  double* misc;  // P, C, E (float) and the FP32 copy of T w; later the Gram partials
-  QrSmem qr;
-};
+// Shared memory of wide_sides: three panels of the cluster's rows, p[k ld + 1 +
+// i] with a halo row on each side (i = -1 and i = R0), the small matrices and
+// the FP32 copy of T w (later the Gram partials, or a data step's chunks), the
+// QR's scratch.
 __host__ __device__ inline size_t misc_doubles(int R0, int r) {
   const size_t sub = (size_t)r * R0 / 2 + 1 + 2 * (size_t)r * r + ((size_t)r * r + 1) / 2, gram = 3 * (size_t)r * r;
   const size_t data = 32 * (size_t)(R0 + r);  // data steps: a 32-column chunk of dY and of the other basis
@@ -106,40 +103,6 @@ __host__ __device__ inline size_t side_doubles(int N, int r, int C) {
   const int R0 = (N + C - 1) / C, ld = (R0 + 2) | 1;
   return 3 * (size_t)r * ld + misc_doubles(R0, r) + QrSmem::doubles(C, r);
 }
-
-// rows [lo, lo + rows) of a global panel (ld N) into a smem panel
-__device__ void load_rows(const double* X, int N, int lo, int rows, int r, double* p, int ld) {
-  for (int e = threadIdx.x; e < rows * r; e += WT) {
-    const int i = e % rows, k = e / rows;
-    p[k * ld + 1 + i] = X[lo + i + (int64_t)k * N];
-  }
-}
-
-// pushes this CTA's first and last rows into the neighbours' halo rows
-// (panel at the same shared address in every CTA); the cluster must
-// synchronise before they are read
-__device__ void push_halos(const Team& tm, int N, int rows, int r, double* p, int ld) {
-  if (rows == 0) return;
-  const int R0 = tm.rows_per(N);
-  const bool up = tm.q > 0, dn = tm.q + 1 < tm.C && tm.lo(N) + rows < N;
-  for (int e = threadIdx.x; e < 2 * r; e += WT) {
-    const int k = e >> 1;
-    if (!(e & 1) && up) tm.at(p, tm.q - 1)[k * ld + 1 + R0] = p[k * ld + 1];
-    if ((e & 1) && dn) tm.at(p, tm.q + 1)[k * ld] = p[k * ld + rows];
-  }
-}
-
-// T w at (row i, column k) of a smem panel
-struct Tri {
-  const double* tri;
-  int N, lo;
-  __device__ double mul(const double* p, int ld, int i, int k) const {
-    const int gi = lo + i;
-    const double cd = tri[N + gi], cs = gi > 0 ? tri[gi] : 0.0, cp = gi + 1 < N ? tri[2 * N + gi] : 0.0;
-    const double* w = p + k * ld + i;
-    return fma(cs, w[0], fma(cp, w[2], cd * w[1]));
-  }
-};
 
 __global__ void __launch_bounds__(WT, 1) wide_sides(const __grid_constant__ StepArgs<double> g, int C) {
   extern __shared__ __align__(16) double dsm[];
@@ -525,28 +488,11 @@ __global__ void __launch_bounds__(WT, 1) wide_core(const __grid_constant__ StepA
 
 cudaError_t cluster_launch(void (*kern)(const StepArgs<double>, int), const StepArgs<double>& g, int blocks, int C,
                            size_t smem, std::atomic<uint64_t>& done, cudaStream_t st) {
-  int dev = 0;
-  cudaError_t e = cudaGetDevice(&dev);
+  cudaError_t e = wide::cluster_attributes(kern, done);
   if (e != cudaSuccess) return e;
-  const uint64_t bit = (dev < 64) ? (uint64_t(1) << dev) : 0;
-  if (!bit || !(done.load(std::memory_order_acquire) & bit)) {
-    e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
-    if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, kWideSmemMax);
-    if (e != cudaSuccess) return e;
-    if (bit) done.fetch_or(bit, std::memory_order_acq_rel);
-  }
   cudaLaunchConfig_t cfg = {};
-  cfg.gridDim = dim3(blocks, 1, 1);
-  cfg.blockDim = dim3(WT, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = st;
   cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = C;
-  attr[0].val.clusterDim.y = 1;
-  attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
+  wide::cluster_config(cfg, attr, blocks, C, smem, st);
   return cudaLaunchKernelEx(&cfg, kern, g, C);
 }
 

@@ -15,7 +15,10 @@
 #include <cooperative_groups.h>
 #include <cuda_runtime.h>
 
+#include <atomic>
 #include <cstdint>
+
+#include "engine_api.h"
 
 namespace lri {
 namespace wide {
@@ -25,6 +28,34 @@ namespace cg = cooperative_groups;
 constexpr int WT = 256;          // threads per CTA
 constexpr int WC_MAX = 16;       // CTAs per cluster (above 8: opt-in)
 constexpr int WR_MAX = 64;       // widest panel
+
+// Launch attributes of a cluster kernel: clusters above 8 CTAs and the largest
+// dynamic shared memory (once per device, as set_smem_limit).
+template <typename F>
+inline cudaError_t cluster_attributes(F* kern, std::atomic<uint64_t>& done) {
+  int dev = 0;
+  cudaError_t e = cudaGetDevice(&dev);
+  if (e != cudaSuccess) return e;
+  const uint64_t bit = (dev < 64) ? (uint64_t(1) << dev) : 0;
+  if (bit && (done.load(std::memory_order_acquire) & bit)) return cudaSuccess;
+  e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
+  if (e == cudaSuccess) e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)kWideSmemMax);
+  if (e == cudaSuccess && bit) done.fetch_or(bit, std::memory_order_acq_rel);
+  return e;
+}
+inline void cluster_config(cudaLaunchConfig_t& cfg, cudaLaunchAttribute* attr, int blocks, int C, size_t smem,
+                           cudaStream_t st) {
+  cfg.gridDim = dim3(blocks, 1, 1);
+  cfg.blockDim = dim3(WT, 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = st;
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = C;
+  attr[0].val.clusterDim.y = 1;
+  attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = 1;
+}
 
 // This CTA's part of a cluster.
 struct Team {
@@ -74,6 +105,54 @@ __device__ void reduce_parts(const Team& tm, double* part, int len, const D& don
   }
   tm.sync();
 }
+
+// rows [lo, lo + rows) of a global panel (ld N) into a smem panel
+static __device__ void load_rows(const double* X, int N, int lo, int rows, int r, double* p, int ld) {
+  for (int e = threadIdx.x; e < rows * r; e += WT) {
+    const int i = e % rows, k = e / rows;
+    p[k * ld + 1 + i] = X[lo + i + (int64_t)k * N];
+  }
+}
+
+// pushes this CTA's first and last rows into the neighbours' halo rows
+// (panel at the same shared address in every CTA); the cluster must
+// synchronise before they are read
+static __device__ void push_halos(const Team& tm, int N, int rows, int r, double* p, int ld) {
+  if (rows == 0) return;
+  const int R0 = tm.rows_per(N);
+  const bool up = tm.q > 0, dn = tm.q + 1 < tm.C && tm.lo(N) + rows < N;
+  for (int e = threadIdx.x; e < 2 * r; e += WT) {
+    const int k = e >> 1;
+    if (!(e & 1) && up) tm.at(p, tm.q - 1)[k * ld + 1 + R0] = p[k * ld + 1];
+    if ((e & 1) && dn) tm.at(p, tm.q + 1)[k * ld] = p[k * ld + rows];
+  }
+}
+
+// the same with the halo rows from memory (zero outside [0, N))
+static __device__ void load_rows_halo(const double* X, int N, int lo, int rows, int r, double* p, int ld) {
+  for (int e = threadIdx.x; e < (rows + 2) * r; e += WT) {
+    const int i = e % (rows + 2), k = e / (rows + 2), g = lo - 1 + i;
+    p[k * ld + i] = (g >= 0 && g < N) ? X[g + (int64_t)k * N] : 0.0;
+  }
+}
+
+// T w (or T^T w) at row i, column k of a smem panel, T = [sub | dia | sup]
+struct Tri {
+  const double* tri;
+  int N, lo;
+  __device__ double mul(const double* p, int ld, int i, int k) const {
+    const int gi = lo + i;
+    const double cd = tri[N + gi], cs = gi > 0 ? tri[gi] : 0.0, cp = gi + 1 < N ? tri[2 * N + gi] : 0.0;
+    const double* w = p + k * ld + i;
+    return fma(cs, w[0], fma(cp, w[2], cd * w[1]));
+  }
+  __device__ double mul_t(const double* p, int ld, int i, int k) const {
+    const int gi = lo + i;
+    const double cd = tri[N + gi], cs = gi > 0 ? tri[2 * N + gi - 1] : 0.0, cp = gi + 1 < N ? tri[gi + 1] : 0.0;
+    const double* w = p + k * ld + i;
+    return fma(cs, w[0], fma(cp, w[2], cd * w[1]));
+  }
+};
 
 // Shared scratch of the distributed QR, carved from dynamic memory.
 struct QrSmem {

@@ -83,3 +83,30 @@ def test_wide_graph_and_single_steps_agree(lri):
         b.check_status()
         out.append(b.download()[0])
     assert np.array_equal(out[0].U, out[1].U) and np.array_equal(out[0].S, out[1].S) and np.array_equal(out[0].V, out[1].V)
+
+
+@pytest.mark.parametrize("n,m,r,scheme,nsub,steps", [(24, 20, 3, "RK4", 1, 3), (65, 40, 5, "Heun", 3, 2),
+                                                      (17, 130, 9, "Euler", 2, 3), (257, 130, 32, "RK4", 2, 2),
+                                                      (70, 64, 48, "RK4", 1, 1)])
+def test_wide_gradient_matches_cpu_adjoint(lri, oracle, n, m, r, scheme, nsub, steps):
+    """Loss gradient through the clusters' reverse steps against the NumPy
+    adjoint: theta and all three input factors."""
+    from oracle import lri_adjoint as AD
+    g = np.random.default_rng(n + m)
+    dt = 0.02
+    A0 = (np.ones(n), -2.0 * np.ones(n), np.ones(n))
+    B = (g.uniform(0.5, 1, m), -2.0 - g.uniform(0, 1, m), g.uniform(0.5, 1, m))
+    theta = g.normal(0.0, 0.1, n)
+    _, _, U, S, V = instance(n, n, m, r)
+    S = S + 0.01 * g.standard_normal((r, r))
+    P, Q = (np.linalg.qr(g.standard_normal((k, 6)))[0] for k in (n, m))
+    d = 2.0 ** (-np.arange(1, 7) / 4.0)
+    k = lri.n_steps((0.0, steps * dt), dt)
+    _, tc, uc, sc, vc = AD.loss_and_grad(U, S, V, A0, theta, B, getattr(oracle, scheme)(nsub), dt, k, (P, d, Q),
+                                         checkpoint_every=2)
+    prob = lri.MatrixDEProblem(lri.SylvesterTridiagOperator(A0, B, theta), lri.SVDLikeRepresentation(U, S, V),
+                               (0.0, steps * dt))
+    _, tg, gr = lri.bug_gradient(prob, lri.UnconventionalAlgorithm(getattr(lri, scheme)(nsub)), dt,
+                                 lri.SVDLikeRepresentation(P, np.diag(d), Q), checkpoint_every=2)
+    for a, b in ((tg, tc), (gr.U, uc), (gr.S, sc), (gr.V, vc)):
+        assert close(a, b)
