@@ -1,8 +1,8 @@
 """Builds the in-tree CUDA library ``_build/liblri_gb300.so`` for sm_103a.
 
-Fifteen translation units (FP32, FP64 and double-float engines, the FP32 and
+Sixteen translation units (FP32, FP64 and double-float engines, the FP32 and
 double-float engines sized for two CTAs per SM, the FP64 steps of small batches
-on clusters, host C ABI,
+on clusters, the BUG steps by sides, host C ABI,
 the allocation-free entry point, the discrete adjoint, the large-stream
 engine, its tensor-core snapshot passes, its cluster core SVD, the large
 Burgers engine's tensor-core Khatri-Rao products and its flow kernels
@@ -25,7 +25,7 @@ HEADER = os.path.join(os.path.dirname(HERE), "include", "lri.h")
 
 SOURCES = ["engine_f32.cu", "engine_f64.cu", "engine_df.cu", "engine_f32_occ2.cu", "engine_df_occ2.cu", "api.cpp",
            "noalloc.cu", "adjoint.cu", "stream.cu", "tc_pass.cu", "core_svd.cu", "tc_kr.cu", "burgers_flow.cu",
-           "burgers_core.cu", "engine_wide.cu"]
+           "burgers_core.cu", "engine_wide.cu", "engine_sides.cu"]
 ARCH_FLAGS = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]
 

@@ -587,7 +587,7 @@ __host__ __device__ inline size_t adj_misc(int N, int r, int C) {
   return 4 * rr + (rr + 1) / 2 + (size_t)r * R0 / 2 + 1;  // P, three partials, E, the FP32 copy
 }
 __host__ inline size_t adj_fwd_doubles(int N, int r, int C) {
-  return 4 * adj_ld(N, C) * r + adj_misc(N, r, C) + QrSmem::doubles(C, r);
+  return 4 * adj_ld(N, C) * r + adj_misc(N, r, C) + QrSmem<double>::elems(C, r);
 }
 __host__ inline size_t adj_rev_doubles(int N, int r, int C) { return 5 * adj_ld(N, C) * r + adj_misc(N, r, C) + r; }
 
@@ -620,7 +620,7 @@ __global__ void __launch_bounds__(WT, 1) adj_fwd(const __grid_constant__ AdjArgs
   double* y = p1 + (size_t)r * ld;
   double* acc = y + (size_t)r * ld;
   double* misc = acc + (size_t)r * ld;
-  const QrSmem qs = QrSmem::carve(misc + adj_misc(N, r, C), C, r);
+  const QrSmem<double> qs = QrSmem<double>::carve(misc + adj_misc(N, r, C), C, r);
   double* Gg = blkp(s.small, W, s.kside ? A_GV : A_GU);  // G, then P
   tm.cl.sync();  // every CTA runs before any distributed access
   {
@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(WT, 1) adj_fwd(const __grid_constant__ AdjArgs
       win = wout;
       wout = t;
     }
-  wide::qr(tm, N, lo, rows, r, win + 1, ld, wout + 1, blkp(s.small, W, s.kside ? A_RK : A_RL), W, qs);
+  wide::qr<double>(tm, N, lo, rows, r, win + 1, ld, wout + 1, blkp(s.small, W, s.kside ? A_RK : A_RL), W, qs);
   // M = Q^T X0 and the projections of Q
   double* Q = wout;
   double* part = misc;

@@ -53,6 +53,13 @@ struct lri_batch {
   const void* opB = nullptr;
   bool bound = false;
   bool data_ready = false;
+  // double-float BUG steps by sides (nclass = 0: the step kernel), the
+  // work list, and streams of their own for the classes after the first
+  lri::SidesPlan sides;
+  int32_t* d_items = nullptr;
+  cudaStream_t side_st[lri::SidesPlan::kMaxClass] = {};
+  cudaEvent_t side_ev[lri::SidesPlan::kMaxClass] = {};
+  cudaEvent_t fork_ev = nullptr;
   lri::WidePlan adj_wide;   // the same for the adjoint step
   lri::WidePlan wide;       // clusters of small FP64 BUG batches (C = 0: the step kernel)
   int32_t ctas_per_sm = 3;  // register budget of the step kernel (lri_batch_set_occupancy)
@@ -132,8 +139,31 @@ StepArgs<T> make_args(const lri_batch* b, double t, double dt, const void* Ynext
   return g;
 }
 
+// One BUG step by sides: the classes beside each other (forked from and joined
+// to st by events, also while st is captured: the joins happen on errors too),
+// then the cores.
+cudaError_t launch_sides(const lri_batch* b, const StepArgs<lri::dfloat>& g, cudaStream_t st) {
+  const int nc = b->sides.nclass;
+  cudaError_t e = nc > 1 ? cudaEventRecord(b->fork_ev, st) : cudaSuccess;
+  int forked = 1;
+  for (; forked < nc && e == cudaSuccess; ++forked) {
+    cudaStream_t s = b->side_st[forked];
+    if ((e = cudaStreamWaitEvent(s, b->fork_ev, 0)) != cudaSuccess) break;
+    e = lri::launch_sides_class(g, b->sides, forked, b->d_items, s);
+    const cudaError_t er = cudaEventRecord(b->side_ev[forked], s);
+    if (e == cudaSuccess) e = er;
+  }
+  if (e == cudaSuccess) e = lri::launch_sides_class(g, b->sides, 0, b->d_items, st);
+  for (int k = 1; k < forked; ++k) {
+    const cudaError_t ew = cudaStreamWaitEvent(st, b->side_ev[k], 0);
+    if (e == cudaSuccess) e = ew;
+  }
+  return e != cudaSuccess ? e : lri::launch_core(g, b->desc.count, st);
+}
+
 cudaError_t launch_one(const lri_batch* b, double t, double dt, const void* Ynext, cudaStream_t st) {
   const int count = b->desc.count;
+  if (b->sides.nclass) return launch_sides(b, make_args<lri::dfloat>(b, t, dt, Ynext), st);
   if (b->desc.dtype == LRI_F32)
     return lri::launch_step<float>(make_args<float>(b, t, dt, Ynext), count, st, b->ctas_per_sm);
   if (b->desc.dtype == LRI_DF) {
@@ -287,6 +317,14 @@ lri_status lri_batch_create(lri_batch** out, const lri_batch_desc* desc, const l
     if (desc->op == LRI_OP_DATA || alg->kind == LRI_ALG_GREEDY) b->totY += n * m;
   }
   // small FP64 BUG batches run on clusters (engine_wide.cu)
+  std::vector<int32_t> items;
+  if (desc->dtype == LRI_DF && alg->kind == LRI_ALG_BUG && desc->op == LRI_OP_SYLVESTER_TRIDIAG) {
+    int dev = 0, sms = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
+        !lri::sides_plan(&b->sides, count, b->n.data(), b->m.data(), b->r.data(), sms, &items))
+      b->sides.nclass = 0;
+  }
   if (desc->dtype == LRI_F64 && alg->kind == LRI_ALG_BUG &&
       (desc->op == LRI_OP_SYLVESTER_TRIDIAG || desc->op == LRI_OP_DATA)) {
     int dev = 0, sms = 0;
@@ -331,6 +369,16 @@ lri_status lri_batch_create(lri_batch** out, const lri_batch_desc* desc, const l
   if (e == cudaSuccess) e = cudaMemset(b->d_status, 0, sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(b->d_proj_valid, 0, sizeof(int32_t) * count);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking);
+  if (b->sides.nclass) {
+    alloc((void**)&b->d_items, sizeof(int32_t) * items.size());
+    if (e == cudaSuccess)
+      e = cudaMemcpy(b->d_items, items.data(), sizeof(int32_t) * items.size(), cudaMemcpyHostToDevice);
+    if (e == cudaSuccess && b->sides.nclass > 1) e = cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming);
+    for (int k = 1; k < b->sides.nclass && e == cudaSuccess; ++k) {
+      e = cudaStreamCreateWithFlags(&b->side_st[k], cudaStreamNonBlocking);
+      if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->side_ev[k], cudaEventDisableTiming);
+    }
+  }
   if (e != cudaSuccess) {
     lri_batch_destroy(b);
     return LRI_ERR_CUDA;
@@ -348,6 +396,12 @@ lri_status lri_batch_destroy(lri_batch* b) {
   if (!b) return LRI_ERR_ARG;
   free_graph(b);
   if (b->cap_stream) cudaStreamDestroy(b->cap_stream);
+  for (cudaStream_t s : b->side_st)
+    if (s) cudaStreamDestroy(s);
+  for (cudaEvent_t ev : b->side_ev)
+    if (ev) cudaEventDestroy(ev);
+  if (b->fork_ev) cudaEventDestroy(b->fork_ev);
+  cudaFree(b->d_items);
   cudaFree(b->d_inst);
   cudaFree(b->d_order);
   cudaFree(b->d_rank);
@@ -534,8 +588,9 @@ int32_t lri_batch_launches_per_step(const lri_batch* b) {
   if (!b) return 0;
   // one engine launch; double-float batches add the three write-back
   // conversions (and one snapshot conversion for data problems) per call
-  if (b->desc.dtype == LRI_DF) return 4 + (b->totY > 0 ? 1 : 0);
-  return b->wide.C ? 2 : 1;  // clusters: the sides, then the core
+  const int step = b->sides.nclass ? b->sides.nclass + 1 : (b->wide.C ? 2 : 1);  // the sides, then the core
+  if (b->desc.dtype == LRI_DF) return step + 3 + (b->totY > 0 ? 1 : 0);
+  return step;
 }
 
 }  // extern "C"

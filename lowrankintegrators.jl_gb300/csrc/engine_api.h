@@ -7,6 +7,7 @@
 
 #include <atomic>
 #include <type_traits>
+#include <vector>
 
 namespace lri_df {
 struct dfloat;  // double-float value (dfloat.cuh); the host only passes pointers to it
@@ -121,6 +122,26 @@ struct WidePlan {
 };
 WidePlan wide_plan(int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms);
 cudaError_t launch_wide_step(const StepArgs<double>& g, int count, const WidePlan& p, cudaStream_t st);
+
+// Double-float BUG steps of Sylvester batches (engine_sides.cu): the (instance,
+// side) pairs grouped into launches by cluster size and shared memory, then
+// one core launch (engine_impl.cuh).
+struct SidesPlan {
+  static constexpr int kMaxClass = 12;
+  struct Class {
+    int32_t C, first, count;
+    size_t smem;
+  };
+  int nclass = 0;  // 0: the batch takes the step kernel
+  Class cls[kMaxClass];
+};
+// fills the plan and the item list (2 * instance + side, class by class); false
+// when a side does not fit
+bool sides_plan(SidesPlan* p, int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms,
+                std::vector<int32_t>* items);
+cudaError_t launch_sides_class(const StepArgs<dfloat>& g, const SidesPlan& p, int k, const int32_t* items,
+                               cudaStream_t st);
+cudaError_t launch_core(const StepArgs<dfloat>& g, int count, cudaStream_t st);
 
 // double <-> double-float conversions of n elements (dfloat storage is a
 // pair of floats, 8 bytes per element)

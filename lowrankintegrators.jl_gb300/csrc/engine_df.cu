@@ -7,6 +7,49 @@ namespace lri {
 template cudaError_t launch_step_occ<dfloat, 3>(const StepArgs<dfloat>&, int, cudaStream_t);
 template size_t step_smem_bytes<dfloat>();
 
+// The S step of a BUG step whose sides ran as sides_kernel (engine_sides.cu), one
+// CTA per instance: basis swap of a first step, S~0 = M S0 N^T, the substep,
+// the new projections (blocks B_RK, B_RL) made current.
+static __global__ void __launch_bounds__(NT, 3) core_kernel(const __grid_constant__ StepArgs<dfloat> g) {
+  extern __shared__ __align__(16) unsigned char smem_raw[];
+  Smem<dfloat>& sm = *reinterpret_cast<Smem<dfloat>*>(smem_raw);
+  const int inst = g.order[blockIdx.x];
+  const InstDesc d = g.inst[inst];
+  const int r = g.rank[inst];
+  if (r < 1 || r > d.rcap) return;  // reported by the sides
+  Inst<dfloat> I;
+  I.n = d.n; I.m = d.m; I.rcap = d.rcap; I.W = d.wcap; I.inst = inst;
+  I.U = g.U + d.offU;
+  I.S = g.S + d.offS;
+  I.V = g.V + d.offV;
+  I.small = g.small + d.offSmall;
+  const int W = I.W;
+  dfloat* GU = I.blk(B_GU);
+  dfloat* GV = I.blk(B_GV);
+  if (g.proj_valid[inst] == 0) {
+    copy_mat<dfloat>(d.n, r, g.work + d.offWK, d.n, I.U, d.n);
+    copy_mat<dfloat>(d.m, r, g.work + d.offWL, d.m, I.V, d.m);
+    if (threadIdx.x == 0) g.proj_valid[inst] = 1;
+  }
+  copy_mat<dfloat>(r, r, I.blk(B_RK), W, GU + (int64_t)r * W, W);
+  copy_mat<dfloat>(r, r, I.blk(B_RL), W, GV + (int64_t)r * W, W);
+  dfloat* St = I.blk(B_ST);
+  dfloat* T1 = I.blk(B_T1);
+  small_gemm<dfloat>(r, r, r, dfloat(1), I.S, I.rcap, false, I.blk(B_N), W, true, dfloat(0), T1, W);
+  small_gemm<dfloat>(r, r, r, dfloat(1), I.blk(B_M), W, false, T1, W, false, dfloat(0), St, W);
+  substep_core<dfloat>(g, I, St, r, r, dfloat(1), GU, GV, I.U, I.V, g.sS, g.dt, sm);
+  copy_mat<dfloat>(r, r, St, W, I.S, I.rcap);
+  check_finite<dfloat>(g, I.S, r, I.rcap);
+}
+
+cudaError_t launch_core(const StepArgs<dfloat>& g, int count, cudaStream_t st) {
+  static std::atomic<uint64_t> done{0};
+  cudaError_t e = set_smem_limit(core_kernel, (int)sizeof(Smem<dfloat>), done);
+  if (e != cudaSuccess) return e;
+  core_kernel<<<count, NT, sizeof(Smem<dfloat>), st>>>(g);
+  return cudaGetLastError();
+}
+
 __global__ void f64_to_df_kernel(const double* __restrict__ in, dfloat* __restrict__ out, int64_t n) {
   for (int64_t i = blockIdx.x * (int64_t)blockDim.x + threadIdx.x; i < n; i += (int64_t)gridDim.x * blockDim.x)
     out[i] = dfloat(in[i]);

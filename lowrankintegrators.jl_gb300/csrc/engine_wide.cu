@@ -101,7 +101,7 @@ __host__ __device__ inline size_t misc_doubles(int R0, int r) {
 }
 __host__ __device__ inline size_t side_doubles(int N, int r, int C) {
   const int R0 = (N + C - 1) / C, ld = (R0 + 2) | 1;
-  return 3 * (size_t)r * ld + misc_doubles(R0, r) + QrSmem::doubles(C, r);
+  return 3 * (size_t)r * ld + misc_doubles(R0, r) + QrSmem<double>::elems(C, r);
 }
 
 __global__ void __launch_bounds__(WT, 1) wide_sides(const __grid_constant__ StepArgs<double> g, int C) {
@@ -127,7 +127,7 @@ __global__ void __launch_bounds__(WT, 1) wide_sides(const __grid_constant__ Step
   double* p1 = sp; sp += r * ldr;
   double* p2 = sp; sp += r * ldr;
   double* misc = sp; sp += misc_doubles(R0, r);
-  const QrSmem qs = QrSmem::carve(sp, C, r);
+  const QrSmem<double> qs = QrSmem<double>::carve(sp, C, r);
   double* Go = I.blk(kside ? WB_GV : WB_GU);  // projections of the other basis
   tm.cl.sync();  // every CTA runs before any distributed access
   if (fresh) {
@@ -277,7 +277,7 @@ __global__ void __launch_bounds__(WT, 1) wide_sides(const __grid_constant__ Step
       __syncthreads();
     }
   }
-  wide::qr(tm, N, lo, rows, r, win + 1, ldr, wout + 1, nullptr, 0, qs);
+  wide::qr<double>(tm, N, lo, rows, r, win + 1, ldr, wout + 1, nullptr, 0, qs);
   // basis change X1^T X0 and, for the flow, the new basis's projections
   double* Q = wout;
   double* part = misc;

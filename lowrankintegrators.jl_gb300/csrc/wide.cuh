@@ -1,7 +1,8 @@
-// wide.cuh - FP64 building blocks for one instance spread over thread-block
-// clusters (engine_wide.cu, adjoint.cu): the rows of a tall panel are split
-// over the CTAs of a cluster, reductions and small matrices go through
-// distributed shared memory.
+// wide.cuh - building blocks for one side of an instance on a thread-block
+// cluster (engine_wide.cu, engine_sides.cu, adjoint.cu): the rows of a tall
+// panel are split over the CTAs of a cluster (one CTA for small panels) and
+// stay in shared memory; reductions and small matrices go through distributed
+// shared memory.
 //
 // GB300 runs FP64 at 1/64 of the FP32 rate (about 1.9 multiply-adds per clock
 // and SM), so a warp's FP64 instruction occupies its unit for 16 clocks of
@@ -18,6 +19,7 @@
 #include <atomic>
 #include <cstdint>
 
+#include "engine.cuh"
 #include "engine_api.h"
 
 namespace lri {
@@ -65,21 +67,53 @@ struct Team {
   __device__ int lo(int N) const { return min(N, q * rows_per(N)); }
   __device__ int hi(int N) const { return min(N, (q + 1) * rows_per(N)); }
   template <typename P>
-  __device__ P* at(P* p, int rank) const { return cl.map_shared_rank(p, rank); }
+  __device__ P* at(P* p, int rank) const { return C > 1 ? cl.map_shared_rank(p, rank) : p; }
+  __device__ void barrier() const {
+    if (C > 1) cl.sync();
+    else __syncthreads();
+  }
   // all threads of the cluster; orders shared, distributed and global accesses
   __device__ void sync() const {
-    __threadfence();
-    cl.sync();
+    if (C > 1) __threadfence();
+    barrier();
   }
 };
 
+// Quotient and remainder by a fixed divisor for 0 <= e < 2^21 (the rounding of
+// (e + 1/2) / d stays below 1 / (2 d)): a few instructions where the integer
+// division takes tens.
+struct FastDiv {
+  int d;
+  float inv;
+  __device__ explicit FastDiv(int d_) : d(d_), inv(1.0f / (float)max(d_, 1)) {}
+  __device__ int div(int e) const { return (int)(((float)e + 0.5f) * inv); }
+};
+
+// Lanes per output for nout outputs on WT threads: the largest power of two <=
+// 32 that still fits, else (more outputs than threads) the one of 1 .. 8 that
+// leaves the fewest threads idle in the last round.
+__device__ __forceinline__ int lanes_for(int nout) {
+  int L = 1;
+  if (nout <= WT) {
+    while (L < 32 && nout * L * 2 <= WT) L *= 2;
+    return L;
+  }
+  int best = (nout + WT - 1) / WT * 8;
+  for (int t = 2; t <= 8; t *= 2) {
+    const int cost = (nout * t + WT - 1) / WT * (8 / t);
+    if (cost < best) {
+      best = cost;
+      L = t;
+    }
+  }
+  return L;
+}
+
 // out(o) for o in [0, nout): f(o, l, L) returns lane l's share (of L) of the
-// sum, summed over the lanes; done(o, v) runs on one lane.  L is the largest
-// power of two <= 32 with nout * L <= WT, so few outputs still fill the CTA.
+// sum, summed over the lanes; done(o, v) runs on one lane.
 template <class F, class D>
 __device__ __forceinline__ void outputs(int nout, const F& f, const D& done) {
-  int L = 1;
-  while (L < 32 && nout * L * 2 <= WT) L *= 2;
+  const int L = lanes_for(nout);
   const int l = threadIdx.x & (L - 1);
   const int per = WT / L;
   for (int o0 = 0; o0 < nout; o0 += per) {  // uniform trip count: every lane reaches the shuffles
@@ -94,22 +128,27 @@ __device__ __forceinline__ void outputs(int nout, const F& f, const D& done) {
 // CTA): done(e, sum) runs for each e on one CTA.  The terms are added in
 // rank order.  Cluster-synchronises before (the parts are complete) and
 // after (done's global writes are visible, part may be reused).
-template <class D>
-__device__ void reduce_parts(const Team& tm, double* part, int len, const D& done) {
+template <typename A, class D>
+__device__ void reduce_parts(const Team& tm, A* part, int len, const D& done) {
   tm.sync();
   const int per = (len + tm.C - 1) / tm.C, e0 = tm.q * per, e1 = min(len, e0 + per);
   for (int e = e0 + threadIdx.x; e < e1; e += WT) {
-    double s = 0.0;
-    for (int k = 0; k < tm.C; ++k) s += tm.at(part, k)[e];
+    A s = part[e];
+    if (tm.C > 1) {
+      s = tm.at(part, 0)[e];
+      for (int k = 1; k < tm.C; ++k) s += tm.at(part, k)[e];
+    }
     done(e, s);
   }
   tm.sync();
 }
 
 // rows [lo, lo + rows) of a global panel (ld N) into a smem panel
-static __device__ void load_rows(const double* X, int N, int lo, int rows, int r, double* p, int ld) {
+template <typename T>
+__device__ void load_rows(const T* X, int N, int lo, int rows, int r, T* p, int ld) {
+  const FastDiv by_rows(rows);
   for (int e = threadIdx.x; e < rows * r; e += WT) {
-    const int i = e % rows, k = e / rows;
+    const int k = by_rows.div(e), i = e - k * rows;
     p[k * ld + 1 + i] = X[lo + i + (int64_t)k * N];
   }
 }
@@ -117,7 +156,8 @@ static __device__ void load_rows(const double* X, int N, int lo, int rows, int r
 // pushes this CTA's first and last rows into the neighbours' halo rows
 // (panel at the same shared address in every CTA); the cluster must
 // synchronise before they are read
-static __device__ void push_halos(const Team& tm, int N, int rows, int r, double* p, int ld) {
+template <typename T>
+__device__ void push_halos(const Team& tm, int N, int rows, int r, T* p, int ld) {
   if (rows == 0) return;
   const int R0 = tm.rows_per(N);
   const bool up = tm.q > 0, dn = tm.q + 1 < tm.C && tm.lo(N) + rows < N;
@@ -129,10 +169,11 @@ static __device__ void push_halos(const Team& tm, int N, int rows, int r, double
 }
 
 // the same with the halo rows from memory (zero outside [0, N))
-static __device__ void load_rows_halo(const double* X, int N, int lo, int rows, int r, double* p, int ld) {
+template <typename T>
+__device__ void load_rows_halo(const T* X, int N, int lo, int rows, int r, T* p, int ld) {
   for (int e = threadIdx.x; e < (rows + 2) * r; e += WT) {
     const int i = e % (rows + 2), k = e / (rows + 2), g = lo - 1 + i;
-    p[k * ld + i] = (g >= 0 && g < N) ? X[g + (int64_t)k * N] : 0.0;
+    p[k * ld + i] = (g >= 0 && g < N) ? X[g + (int64_t)k * N] : T(0);
   }
 }
 
@@ -155,18 +196,20 @@ struct Tri {
 };
 
 // Shared scratch of the distributed QR, carved from dynamic memory.
+template <typename T>
 struct QrSmem {
-  double* slot;  // 2 x C x r: partial dots of every CTA, alternating by column
-  double* row;   // 2 x r: the pivot row
-  double* part;  // (WT / 32) x r
-  double* dots;  // r
-  double* v1;    // r x (r + 1): pivot rows of V, v1[k LT + j], j < k
-  double* tri;   // r x (r + 1): T of the compact WY form, T(i, k) at i LT + k
-  double* coef;  // beta, tau, scal
-  __host__ __device__ static constexpr size_t doubles(int C, int r) {
-    return (size_t)r * (2 * C + 2 + WT / 32 + 1) + 2 * (size_t)r * (r + 1) + 4;
+  T* slot;  // 2 x C x r: partial dots of every CTA, alternating by column
+  T* row;   // 2 x r: the pivot row
+  T* part;  // (WT / 32) x r
+  T* dots;  // r
+  T* v1;    // r x (r + 1): pivot rows of V, v1[k LT + j], j < k
+  T* tri;   // r x (r + 1): T of the compact WY form, T(i, k) at i LT + k
+  T* coef;  // beta, tau, scal
+  T* sgn;   // r: column scales, then signs (fast forms)
+  __host__ __device__ static constexpr size_t elems(int C, int r) {
+    return (size_t)r * (2 * C + 2 + WT / 32 + 1) + 2 * (size_t)r * (r + 1) + 4 + r;
   }
-  __device__ static QrSmem carve(double* p, int C, int r) {
+  __device__ static QrSmem carve(T* p, int C, int r) {
     QrSmem s;
     s.slot = p;
     s.row = s.slot + 2 * C * r;
@@ -175,98 +218,173 @@ struct QrSmem {
     s.v1 = s.dots + r;
     s.tri = s.v1 + r * (r + 1);
     s.coef = s.tri + r * (r + 1);
+    s.sgn = s.coef + 4;
     return s;
   }
 };
 
-// Householder QR (LAPACK signs) of an N x r panel whose rows [lo, lo + rows)
-// are this CTA's a[k ld + i]; the explicit Q goes to qout (same layout) and,
-// when R is given, the factor to R (global, ld ldr, zeros below).  One
+__device__ __forceinline__ float two_to(float, int e) { return ldexpf(1.0f, e); }
+__device__ __forceinline__ dfloat two_to(dfloat, int e) { return dfloat(ldexpf(1.0f, e), 0.0f); }
+__device__ __forceinline__ float lead(float x) { return x; }
+__device__ __forceinline__ float lead(dfloat x) { return x.hi; }
+
+// Householder QR (LAPACK signs; POS: a positive diagonal of R) of an N x r
+// panel whose rows [lo, lo + rows) are this CTA's a[k ld + i]; the explicit Q
+// goes to qout (same layout) and, when R is given, the factor to R (global, ld
+// ldr, zeros below; not with the scaled columns of the FP32-based types).  One
 // cluster barrier per column: a single pass forms x^T A for every column (the
 // trailing ones, and the earlier reflectors for the compact WY form), its
 // partials and the pivot row are pushed to every CTA, and every CTA derives
 // the reflector from the same sums.  Q = [I; 0] - V (T V1^T), T from those
 // products, replaces the backward accumulation: N r^2 / 2 multiply-adds and
 // no further barrier.  a is overwritten.
-static __device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, double* a, int ld,
-                                       double* qout, double* R, int ldr, const QrSmem& s) {
+// float and dfloat columns are first scaled by powers of two to a largest
+// entry in [1, 2) (Q does not change), so that the squares of graded columns
+// stay inside the FP32 exponent range; their dots are summed in runs of eight
+// rows.
+template <typename T, bool POS = false>
+__device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, T* a, int ld, T* qout, T* R, int ldr,
+                                const QrSmem<T>& s) {
+  constexpr bool F64 = std::is_same<T, double>::value;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int LT = r + 1;
   const int R0 = tm.rows_per(N);
-  for (int e = tid; e < r * LT; e += WT) s.tri[e] = s.v1[e] = 0.0;
-  __syncthreads();
+  const int jw = r <= 8 ? 8 : (r <= 16 ? 16 : 32), ncls = WT / jw, cls = tid / jw;
+  const FastDiv by_rows(rows);
+  for (int e = tid; e < r * LT; e += WT) s.tri[e] = s.v1[e] = T(0);
+  if constexpr (!F64) {
+    // column maxima: warps take columns, every CTA learns all (slot 0 of both buffers)
+    for (int j = warp; j < r; j += WT / 32) {
+      float m = 0.0f;
+      for (int i = lane; i < rows; i += 32) m = fmaxf(m, fabsf(lead(a[j * ld + i])));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      for (int c = lane; c < tm.C; c += 32) tm.at(s.slot, c)[tm.q * r + j] = T(m);
+    }
+    tm.barrier();
+    if (tid < r) {
+      float m = 0.0f;
+      for (int c = 0; c < tm.C; ++c) m = fmaxf(m, lead(s.slot[c * r + tid]));
+      int e = 0;
+      if (m > 0.0f && m < 3.0e38f) frexpf(m, &e);
+      s.sgn[tid] = two_to(T(0), max(-120, min(120, 1 - e)));
+    }
+    __syncthreads();
+    for (int e = tid; e < rows * r; e += WT) {
+      const int k = by_rows.div(e), i = e - k * rows;
+      a[k * ld + i] = a[k * ld + i] * s.sgn[k];
+    }
+    tm.barrier();  // the slots are reused
+  } else {
+    __syncthreads();
+  }
   for (int k = 0; k < r; ++k) {
-    double* slot = s.slot + (k & 1) * tm.C * r;
-    double* row = s.row + (k & 1) * r;
-    double* x = a + k * ld;
+    T* slot = s.slot + (k & 1) * tm.C * r;
+    T* row = s.row + (k & 1) * r;
+    T* x = a + k * ld;
     const int i0 = max(0, k + 1 - lo);  // rows below the pivot
-    // partial dots: lane = column, warp = row class
-    for (int j = lane; j < r; j += 32) {
-      double p = 0.0;
-      for (int i = i0 + warp; i < rows; i += WT / 32) p = fma(x[i], a[j * ld + i], p);
-      s.part[warp * r + j] = p;
+    // partial dots: lanes along the columns (jw per row class), a warp's row
+    // classes combined by shuffles
+    for (int jb = 0; jb < r; jb += jw) {
+      const int j = jb + (lane & (jw - 1));
+      const T* aj = a + min(j, r - 1) * ld;
+      T p = T(0);
+      if constexpr (F64) {
+        for (int i = i0 + cls; i < rows; i += ncls) p = fma(x[i], aj[i], p);
+      } else {
+        for (int ib = i0 + cls; ib < rows; ib += 8 * ncls) {
+          T q = T(0);
+#pragma unroll
+          for (int u = 0; u < 8; ++u) {
+            const int i = ib + u * ncls;
+            if (i < rows) q = fma_acc(x[i], aj[i], q);
+          }
+          p += renorm(q);
+        }
+      }
+      for (int o = jw; o < 32; o <<= 1) p += shfl_xor(p, o);
+      if (lane < jw && j < r) s.part[warp * r + j] = p;
     }
     if (tm.q == k / R0)
       for (int e = tid; e < r * tm.C; e += WT) tm.at(row, e / r)[e % r] = a[(e % r) * ld + (k - lo)];
     __syncthreads();
     if (tid < r) {
-      double p = 0.0;
+      T p = T(0);
 #pragma unroll
       for (int w = 0; w < WT / 32; ++w) p += s.part[w * r + tid];
-      for (int c = 0; c < tm.C; ++c) tm.at(slot, c)[tm.q * r + tid] = p;
+      if (tm.C == 1) s.dots[tid] = p;
+      else
+        for (int c = 0; c < tm.C; ++c) tm.at(slot, c)[tm.q * r + tid] = p;
     }
-    tm.cl.sync();
-    // totals: four lanes per column
-    for (int j0 = 0; j0 < r; j0 += WT / 4) {
-      const int j = j0 + (tid >> 2);
-      double p = 0.0;
-      if (j < r)
-        for (int c = tid & 3; c < tm.C; c += 4) p += slot[c * r + j];
-      p += __shfl_xor_sync(0xffffffffu, p, 1);
-      p += __shfl_xor_sync(0xffffffffu, p, 2);
-      if (j < r && (tid & 3) == 0) s.dots[j] = p;
+    tm.barrier();
+    if (tm.C > 1) {
+      // totals: four lanes per column
+      for (int j0 = 0; j0 < r; j0 += WT / 4) {
+        const int j = j0 + (tid >> 2);
+        T p = T(0);
+        if (j < r)
+          for (int c = tid & 3; c < tm.C; c += 4) p += slot[c * r + j];
+        p += shfl_xor(p, 1);
+        p += shfl_xor(p, 2);
+        if (j < r && (tid & 3) == 0) s.dots[j] = p;
+      }
+      __syncthreads();
     }
-    __syncthreads();
     if (warp == 0) {
-      const double xn2 = s.dots[k], alpha = row[k];
-      double beta = alpha, tau = 0.0, scal = 0.0;
-      if (xn2 > 0.0) {
+      const T xn2 = s.dots[k], alpha = row[k];
+      T beta = alpha, tau = T(0), scal = T(0);
+      if (xn2 > T(0)) {
         beta = -copysign(sqrt(fma(alpha, alpha, xn2)), alpha);
         tau = (beta - alpha) / beta;
-        scal = 1.0 / (alpha - beta);
+        scal = T(1) / (alpha - beta);
       }
       if (lane == 0) {
         s.coef[0] = beta;
         s.coef[1] = tau;
         s.coef[2] = scal;
+        if constexpr (!F64) s.sgn[k] = (POS && lead(beta) < 0.0f) ? T(-1.0f) : T(1.0f);
       }
     }
     __syncthreads();
-    const double beta = s.coef[0], tau = s.coef[1], scal = s.coef[2];
+    const T beta = s.coef[0], tau = s.coef[1], scal = s.coef[2];
     // w_j (trailing columns) and z_j = -tau V_j^T v_k (earlier reflectors)
     if (tid < r) {
       const int j = tid;
-      const double rk = row[j];
-      const double t = (j != k) ? tau * fma(scal, s.dots[j], rk) : 0.0;
+      const T rk = row[j];
+      const T t = (j != k) ? tau * fma(scal, s.dots[j], rk) : T(0);
       if (j < k) {
         s.v1[k * LT + j] = rk;
         s.tri[j * LT + k] = -t;
       }
       if (j == k) s.tri[k * LT + k] = tau;
-      if (R && tm.q == 0) R[k + (int64_t)j * ldr] = (j > k) ? rk - t : ((j == k) ? beta : 0.0);
+      if (F64 && R && tm.q == 0) R[k + (int64_t)j * ldr] = (j > k) ? rk - t : ((j == k) ? beta : T(0));
       s.dots[j] = t;
     }
     __syncthreads();
     // trailing update, the reflector stored in column k
     const int ib = max(0, k - lo), nr = rows - ib, nj = r - k - 1;
-    if (tau != 0.0 && nr > 0) {
-      for (int e = tid; e < nr * nj; e += WT) {
-        const int i = ib + e % nr, j = k + 1 + e / nr;
-        const double vi = (lo + i == k) ? 1.0 : x[i] * scal;
-        a[j * ld + i] = fma(-vi, s.dots[j], a[j * ld + i]);
+    if (tau != T(0) && nr > 0) {
+      if (nr >= WT / 2) {
+        // a row per thread
+        for (int i = ib + tid; i < rows; i += WT) {
+          T vi = T(1);
+          if (lo + i > k) {
+            vi = x[i] * scal;
+            x[i] = vi;
+          }
+#pragma unroll 4
+          for (int j = k + 1; j < r; ++j) a[j * ld + i] = fma(-vi, s.dots[j], a[j * ld + i]);
+        }
+      } else {
+        const FastDiv by_nr(nr);
+        for (int e = tid; e < nr * nj; e += WT) {
+          const int q = by_nr.div(e), i = ib + e - q * nr, j = k + 1 + q;
+          const T vi = (lo + i == k) ? T(1) : x[i] * scal;
+          a[j * ld + i] = fma(-vi, s.dots[j], a[j * ld + i]);
+        }
+        __syncthreads();
+        for (int i = i0 + tid; i < rows; i += WT) x[i] = x[i] * scal;
       }
-      __syncthreads();
-      for (int i = i0 + tid; i < rows; i += WT) x[i] *= scal;
     }
     __syncthreads();
   }
@@ -274,16 +392,18 @@ static __device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, 
   // lanes per row
   constexpr int TU = WR_MAX * 8 / WT;
   for (int k = 1; k < r; ++k) {
-    double v[TU];
+    T v[TU];
 #pragma unroll
     for (int u = 0; u < TU; ++u) {
       const int i = (tid + u * WT) >> 3;
-      double p = 0.0;
-      if (i < k)
-        for (int l = i + (tid & 7); l < k; l += 8) p = fma(s.tri[i * LT + l], s.tri[l * LT + k], p);
-      p += __shfl_xor_sync(0xffffffffu, p, 1);
-      p += __shfl_xor_sync(0xffffffffu, p, 2);
-      p += __shfl_xor_sync(0xffffffffu, p, 4);
+      T p = T(0);
+      if (u * (WT / 8) < r) {  // uniform
+        if (i < k)
+          for (int l = i + (tid & 7); l < k; l += 8) p = fma(s.tri[i * LT + l], s.tri[l * LT + k], p);
+        p += shfl_xor(p, 1);
+        p += shfl_xor(p, 2);
+        p += shfl_xor(p, 4);
+      }
       v[u] = p;
     }
     __syncthreads();
@@ -294,37 +414,54 @@ static __device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, 
     }
     __syncthreads();
   }
-  // X = T V1^T (V1 unit lower triangular), X(i, j) at j LT + i for i <= j, over
-  // the rows of v1 that it is formed from
-  constexpr int XU = WR_MAX * WR_MAX / WT;
-  double xv[XU];
-#pragma unroll
-  for (int u = 0; u < XU; ++u) {
-    const int e = tid + u * WT, i = e % r, j = e / r;
-    double p = 0.0;
-    if (j < r && i <= j) {
-      p = s.tri[i * LT + j];
-      for (int l = i; l < j; ++l) p = fma(s.tri[i * LT + l], s.v1[j * LT + l], p);
-    }
-    xv[u] = p;
+  // X = T V1^T (V1 unit lower triangular), X(i, j) at j LT + i for i <= j: the
+  // result takes the places of T's transpose
+  for (int e = tid; e < r * r; e += WT) {
+    const int i = e % r, j = e / r;
+    if (i > j) continue;
+    T p = s.tri[i * LT + j];
+    for (int l = i; l < j; ++l) p = fma(s.tri[i * LT + l], s.v1[j * LT + l], p);
+    if (i < j) s.tri[j * LT + i] = p;  // strictly lower entries: T has none there
+    else s.tri[j * LT + r] = p;        // the diagonal: the spare column
   }
   // explicit V: zeros above the unit diagonal
-  for (int e = tid; e < rows * r; e += WT) {
-    const int i = e % rows, k = e / rows;
-    if (lo + i <= k) a[k * ld + i] = (lo + i == k) ? 1.0 : 0.0;
+  for (int e = tid; e < min(rows, max(0, r - lo)) * r; e += WT) {
+    const int i = e / r, k = e - i * r;
+    if (lo + i <= k) a[k * ld + i] = (lo + i == k) ? T(1) : T(0);
   }
   __syncthreads();
+  if constexpr (F64) {
+    for (int e = tid; e < rows * r; e += WT) {
+      const int j = by_rows.div(e), i = e - j * rows;
+      T p = (lo + i == j) ? T(1) : T(0);
+      for (int k = 0; k < j; ++k) p = fma(-a[k * ld + i], s.tri[j * LT + k], p);
+      qout[j * ld + i] = fma(-a[j * ld + i], s.tri[j * LT + r], p);
+    }
+  } else {
+    // four columns per thread share the loads of V
+    const int ng = (r + 3) >> 2;
+    for (int e = tid; e < rows * ng; e += WT) {
+      const int g = by_rows.div(e), i = e - g * rows, j0 = 4 * g, kn = min(r, j0 + 4);
+      T p[4] = {T(0), T(0), T(0), T(0)};
+      for (int k = 0; k < j0; ++k) {
+        const T v = a[k * ld + i];
 #pragma unroll
-  for (int u = 0; u < XU; ++u) {
-    const int e = tid + u * WT, i = e % r, j = e / r;
-    if (j < r && i <= j) s.v1[j * LT + i] = xv[u];
-  }
-  __syncthreads();
-  for (int e = tid; e < rows * r; e += WT) {
-    const int i = e % rows, j = e / rows;
-    double p = (lo + i == j) ? 1.0 : 0.0;
-    for (int k = 0; k <= j; ++k) p = fma(-a[k * ld + i], s.v1[j * LT + k], p);
-    qout[j * ld + i] = p;
+        for (int u = 0; u < 4; ++u) p[u] = fma_acc(v, s.tri[min(j0 + u, r - 1) * LT + k], p[u]);
+      }
+      for (int k = j0; k < kn; ++k) {
+        const T v = a[k * ld + i];
+#pragma unroll
+        for (int u = 0; u < 4; ++u)
+          if (k <= j0 + u && j0 + u < r) p[u] = fma_acc(v, s.tri[(j0 + u) * LT + ((k == j0 + u) ? r : k)], p[u]);
+      }
+#pragma unroll
+      for (int u = 0; u < 4; ++u)
+        if (j0 + u < r) {
+          T q = ((lo + i == j0 + u) ? T(1) : T(0)) - renorm(p[u]);
+          if constexpr (POS) q = q * s.sgn[j0 + u];
+          qout[(j0 + u) * ld + i] = q;
+        }
+    }
   }
   __syncthreads();
 }
