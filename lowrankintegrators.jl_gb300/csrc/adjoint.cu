@@ -1197,34 +1197,38 @@ size_t adjoint_work_elems(int64_t n, int64_t m, int64_t r, int ns_k, int ns_l) {
 
 int adjoint_max_stages() { return kAdjMaxStages; }
 
-WidePlan adjoint_plan(const WidePlan& step, int count, const int64_t* n, const int64_t* m, const int64_t* r) {
-  WidePlan p;
-  p.C = step.C;
-  for (int i = 0; i < count && p.C; ++i)
+AdjointPlan adjoint_plan(int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms) {
+  AdjointPlan p;
+  int64_t tall = 0;
+  for (int i = 0; i < count; ++i) tall = std::max(tall, std::max(n[i], m[i]));
+  p.C = wide_cluster(count, tall, sms);
+  if (p.C < 2) return AdjointPlan{};
+  for (int i = 0; i < count; ++i)
     for (int64_t N : {n[i], m[i]}) {
       const int ri = (int)r[i];
-      p.side_smem = std::max(p.side_smem, sizeof(double) * adj_fwd_doubles((int)N, ri, p.C));
-      p.core_smem = std::max(p.core_smem, sizeof(double) * adj_rev_doubles((int)N, ri, p.C));
+      if (ri > wide::WR_MAX) return AdjointPlan{};
+      p.fwd_smem = std::max(p.fwd_smem, sizeof(double) * adj_fwd_doubles((int)N, ri, p.C));
+      p.rev_smem = std::max(p.rev_smem, sizeof(double) * adj_rev_doubles((int)N, ri, p.C));
     }
-  if (p.side_smem > kWideSmemMax || p.core_smem > kWideSmemMax) return WidePlan{};
-  p.side_smem = std::max(p.side_smem, (size_t)120 * 1024);  // a CTA per SM
-  p.core_smem = std::max(p.core_smem, (size_t)120 * 1024);
+  if (p.fwd_smem > kWideSmemMax || p.rev_smem > kWideSmemMax) return AdjointPlan{};
+  p.fwd_smem = std::max(p.fwd_smem, (size_t)120 * 1024);  // a CTA per SM
+  p.rev_smem = std::max(p.rev_smem, (size_t)120 * 1024);
   return p;
 }
 
 cudaError_t launch_adjoint_step(const InstDesc* inst, const int64_t* adj_off, const int64_t* th_off, int count,
                                 const double* U0, const double* S0, const double* V0, double* Ub, double* Sb,
                                 double* Vb, double* thb, const double* opA, const double* opB, double* work,
-                                const Scheme& sK, const Scheme& sL, const Scheme& sS, double dt, const WidePlan& plan,
+                                const Scheme& sK, const Scheme& sL, const Scheme& sS, double dt, const AdjointPlan& plan,
                                 cudaStream_t st) {
   AdjArgs g{inst, adj_off, th_off, U0, S0, V0, Ub, Sb, Vb, thb, opA, opB, work, sK, sL, sS, dt, 0};
   if (plan.C) {
     static std::atomic<uint64_t> d0{0}, d1{0}, d2{0}, d3{0};
     const int C = plan.C;
-    cudaError_t e = adj_launch(adj_fwd, g, 2 * C * count, C, plan.side_smem, d0, st);
+    cudaError_t e = adj_launch(adj_fwd, g, 2 * C * count, C, plan.fwd_smem, d0, st);
     if (e == cudaSuccess) e = adj_launch(adj_core, g, C * count, C, 0, d1, st);
-    if (e == cudaSuccess) e = adj_launch(adj_rev, g, 2 * C * count, C, plan.core_smem, d2, st);
-    if (e == cudaSuccess) e = adj_launch(adj_out, g, 2 * C * count, C, plan.core_smem, d3, st);
+    if (e == cudaSuccess) e = adj_launch(adj_rev, g, 2 * C * count, C, plan.rev_smem, d2, st);
+    if (e == cudaSuccess) e = adj_launch(adj_out, g, 2 * C * count, C, plan.rev_smem, d3, st);
     return e != cudaSuccess ? e : cudaGetLastError();
   }
   const size_t smem = sizeof(Smem<double>);

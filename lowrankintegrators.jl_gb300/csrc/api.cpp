@@ -53,15 +53,16 @@ struct lri_batch {
   const void* opB = nullptr;
   bool bound = false;
   bool data_ready = false;
-  // double-float BUG steps by sides (nclass = 0: the step kernel), the
-  // work list, and streams of their own for the classes after the first
-  lri::SidesPlan sides;
+  // BUG steps by sides (nclass = 0: the step kernel): the FP64 plan, or the
+  // double-float one in its place; the work list, and streams of their own for
+  // the classes after the first
+  lri::WidePlan wide;
+  const lri::SidesPlan& sides() const { return wide.sides; }
   int32_t* d_items = nullptr;
   cudaStream_t side_st[lri::SidesPlan::kMaxClass] = {};
   cudaEvent_t side_ev[lri::SidesPlan::kMaxClass] = {};
   cudaEvent_t fork_ev = nullptr;
-  lri::WidePlan adj_wide;   // the same for the adjoint step
-  lri::WidePlan wide;       // clusters of small FP64 BUG batches (C = 0: the step kernel)
+  lri::AdjointPlan adj_plan;  // clusters of the adjoint step
   int32_t ctas_per_sm = 3;  // register budget of the step kernel (lri_batch_set_occupancy)
   // discrete adjoint (allocated by lri_batch_adjoint_prepare)
   double* d_adj_work = nullptr;
@@ -139,40 +140,52 @@ StepArgs<T> make_args(const lri_batch* b, double t, double dt, const void* Ynext
   return g;
 }
 
-// One BUG step by sides: the classes beside each other (forked from and joined
-// to st by events, also while st is captured: the joins happen on errors too),
-// then the cores.
-cudaError_t launch_sides(const lri_batch* b, const StepArgs<lri::dfloat>& g, cudaStream_t st) {
-  const int nc = b->sides.nclass;
+// The sides of a BUG step, class by class beside each other (forked from and
+// joined to st by events, also while st is captured: the joins happen on
+// errors too); launch(k, stream) launches class k.
+template <class F>
+cudaError_t launch_classes(const lri_batch* b, const lri::SidesPlan& p, cudaStream_t st, const F& launch) {
+  const int nc = p.nclass;
   cudaError_t e = nc > 1 ? cudaEventRecord(b->fork_ev, st) : cudaSuccess;
   int forked = 1;
   for (; forked < nc && e == cudaSuccess; ++forked) {
     cudaStream_t s = b->side_st[forked];
     if ((e = cudaStreamWaitEvent(s, b->fork_ev, 0)) != cudaSuccess) break;
-    e = lri::launch_sides_class(g, b->sides, forked, b->d_items, s);
+    e = launch(forked, s);
     const cudaError_t er = cudaEventRecord(b->side_ev[forked], s);
     if (e == cudaSuccess) e = er;
   }
-  if (e == cudaSuccess) e = lri::launch_sides_class(g, b->sides, 0, b->d_items, st);
+  if (e == cudaSuccess) e = launch(0, st);
   for (int k = 1; k < forked; ++k) {
     const cudaError_t ew = cudaStreamWaitEvent(st, b->side_ev[k], 0);
     if (e == cudaSuccess) e = ew;
   }
-  return e != cudaSuccess ? e : lri::launch_core(g, b->desc.count, st);
+  return e;
 }
 
 cudaError_t launch_one(const lri_batch* b, double t, double dt, const void* Ynext, cudaStream_t st) {
   const int count = b->desc.count;
-  if (b->sides.nclass) return launch_sides(b, make_args<lri::dfloat>(b, t, dt, Ynext), st);
   if (b->desc.dtype == LRI_F32)
     return lri::launch_step<float>(make_args<float>(b, t, dt, Ynext), count, st, b->ctas_per_sm);
+  const lri::SidesPlan& sides = b->sides();
+  if (sides.nclass && b->desc.dtype == LRI_DF) {
+    const StepArgs<lri::dfloat> g = make_args<lri::dfloat>(b, t, dt, Ynext);
+    const cudaError_t e = launch_classes(
+        b, sides, st, [&](int k, cudaStream_t s) { return lri::launch_sides_class(g, sides, k, b->d_items, s); });
+    return e != cudaSuccess ? e : lri::launch_core(g, count, st);
+  }
+  if (sides.nclass) {
+    const StepArgs<double> g = make_args<double>(b, t, dt, Ynext);
+    const cudaError_t e = launch_classes(
+        b, sides, st, [&](int k, cudaStream_t s) { return lri::launch_wide_side(g, b->wide, k, b->d_items, s); });
+    return e != cudaSuccess ? e : lri::launch_wide_core(g, count, b->wide, st);
+  }
   if (b->desc.dtype == LRI_DF) {
     cudaError_t e = cudaSuccess;
     if (Ynext) e = lri::convert_f64_to_df(static_cast<const double*>(Ynext), b->iYn, b->totY, st);
     if (e != cudaSuccess) return e;
     return lri::launch_step<lri::dfloat>(make_args<lri::dfloat>(b, t, dt, Ynext), count, st, b->ctas_per_sm);
   }
-  if (b->wide.C) return lri::launch_wide_step(make_args<double>(b, t, dt, Ynext), count, b->wide, st);
   return lri::launch_step<double>(make_args<double>(b, t, dt, Ynext), count, st);
 }
 
@@ -316,22 +329,21 @@ lri_status lri_batch_create(lri_batch** out, const lri_batch_desc* desc, const l
     d.offY = b->totY;
     if (desc->op == LRI_OP_DATA || alg->kind == LRI_ALG_GREEDY) b->totY += n * m;
   }
-  // small FP64 BUG batches run on clusters (engine_wide.cu)
+  // BUG steps of FP64 and double-float batches run by sides where they fit
   std::vector<int32_t> items;
-  if (desc->dtype == LRI_DF && alg->kind == LRI_ALG_BUG && desc->op == LRI_OP_SYLVESTER_TRIDIAG) {
+  const bool sylv = desc->op == LRI_OP_SYLVESTER_TRIDIAG;
+  if (alg->kind == LRI_ALG_BUG && desc->dtype != LRI_F32 &&
+      (sylv || (desc->op == LRI_OP_DATA && desc->dtype == LRI_F64))) {
     int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) != cudaSuccess ||
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess ||
-        !lri::sides_plan(&b->sides, count, b->n.data(), b->m.data(), b->r.data(), sms, &items))
-      b->sides.nclass = 0;
-  }
-  if (desc->dtype == LRI_F64 && alg->kind == LRI_ALG_BUG &&
-      (desc->op == LRI_OP_SYLVESTER_TRIDIAG || desc->op == LRI_OP_DATA)) {
-    int dev = 0, sms = 0;
-    if (cudaGetDevice(&dev) == cudaSuccess &&
-        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess)
-      b->wide = lri::wide_plan(count, b->n.data(), b->m.data(), b->rcap.data(), sms);
-    b->adj_wide = lri::adjoint_plan(b->wide, count, b->n.data(), b->m.data(), b->rcap.data());
+    bool ok = cudaGetDevice(&dev) == cudaSuccess &&
+              cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) == cudaSuccess;
+    if (ok && desc->dtype == LRI_DF)
+      ok = lri::sides_plan(&b->wide.sides, count, b->n.data(), b->m.data(), b->r.data(), sms, &items);
+    else if (ok)
+      ok = lri::wide_plan(&b->wide, count, b->n.data(), b->m.data(), b->r.data(), sms, &items);
+    if (!ok) b->wide.sides.nclass = 0;
+    if (desc->dtype == LRI_F64 && sylv)
+      b->adj_plan = lri::adjoint_plan(count, b->n.data(), b->m.data(), b->rcap.data(), sms);
   }
   // longest-processing-time-first launch order: CTAs start in block order
   b->order.resize(count);
@@ -369,12 +381,12 @@ lri_status lri_batch_create(lri_batch** out, const lri_batch_desc* desc, const l
   if (e == cudaSuccess) e = cudaMemset(b->d_status, 0, sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMemset(b->d_proj_valid, 0, sizeof(int32_t) * count);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&b->cap_stream, cudaStreamNonBlocking);
-  if (b->sides.nclass) {
+  if (b->sides().nclass) {
     alloc((void**)&b->d_items, sizeof(int32_t) * items.size());
     if (e == cudaSuccess)
       e = cudaMemcpy(b->d_items, items.data(), sizeof(int32_t) * items.size(), cudaMemcpyHostToDevice);
-    if (e == cudaSuccess && b->sides.nclass > 1) e = cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming);
-    for (int k = 1; k < b->sides.nclass && e == cudaSuccess; ++k) {
+    if (e == cudaSuccess && b->sides().nclass > 1) e = cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming);
+    for (int k = 1; k < b->sides().nclass && e == cudaSuccess; ++k) {
       e = cudaStreamCreateWithFlags(&b->side_st[k], cudaStreamNonBlocking);
       if (e == cudaSuccess) e = cudaEventCreateWithFlags(&b->side_ev[k], cudaEventDisableTiming);
     }
@@ -588,7 +600,7 @@ int32_t lri_batch_launches_per_step(const lri_batch* b) {
   if (!b) return 0;
   // one engine launch; double-float batches add the three write-back
   // conversions (and one snapshot conversion for data problems) per call
-  const int step = b->sides.nclass ? b->sides.nclass + 1 : (b->wide.C ? 2 : 1);  // the sides, then the core
+  const int step = b->sides().nclass ? b->sides().nclass + 1 : 1;  // the sides' classes, then the core
   if (b->desc.dtype == LRI_DF) return step + 3 + (b->totY > 0 ? 1 : 0);
   return step;
 }
@@ -655,7 +667,7 @@ lri_status lri_batch_adjoint_step(lri_batch* b, double dt, const void* U0, const
       static_cast<const double*>(V0), static_cast<double*>(Ubar), static_cast<double*>(Sbar),
       static_cast<double*>(Vbar), static_cast<double*>(theta_bar), static_cast<const double*>(b->opA),
       static_cast<const double*>(b->opB), b->d_adj_work, to_scheme(b->alg.K_alg), to_scheme(b->alg.L_alg),
-      to_scheme(b->alg.S_alg), dt, b->adj_wide, (cudaStream_t)stream));
+      to_scheme(b->alg.S_alg), dt, b->adj_plan, (cudaStream_t)stream));
 }
 
 // ---------------------------------------------------------------------------

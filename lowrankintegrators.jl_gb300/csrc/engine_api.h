@@ -112,20 +112,10 @@ inline cudaError_t launch_step(const StepArgs<T>& g, int count, cudaStream_t str
   }
 }
 
-// FP64 BUG steps of small batches on clusters (engine_wide.cu): CTAs per
-// cluster (0: the batch takes the step kernel) and the shared memory of the
-// two launches.
-constexpr size_t kWideSmemMax = 226 * 1024;
-struct WidePlan {
-  int C = 0;
-  size_t side_smem = 0, core_smem = 0;
-};
-WidePlan wide_plan(int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms);
-cudaError_t launch_wide_step(const StepArgs<double>& g, int count, const WidePlan& p, cudaStream_t st);
-
-// Double-float BUG steps of Sylvester batches (engine_sides.cu): the (instance,
-// side) pairs grouped into launches by cluster size and shared memory, then
-// one core launch (engine_impl.cuh).
+// BUG steps by sides: the (instance, side) pairs grouped into launches by
+// cluster size and shared memory.
+constexpr size_t kWideSmemMax = 226 * 1024;  // dynamic shared memory of one CTA per SM
+constexpr size_t kHalfSmem = 112 * 1024;     // of two
 struct SidesPlan {
   static constexpr int kMaxClass = 12;
   struct Class {
@@ -135,13 +125,37 @@ struct SidesPlan {
   int nclass = 0;  // 0: the batch takes the step kernel
   Class cls[kMaxClass];
 };
-// fills the plan and the item list (2 * instance + side, class by class); false
-// when a side does not fit
+struct SideItem {
+  int32_t id;  // 2 * instance + side
+  int C;       // CTAs of its cluster
+  size_t smem;
+  double cost;
+};
+// sorts the items into classes; fills the plan and the work list (class by class)
+bool group_sides(std::vector<SideItem>& v, SidesPlan* p, std::vector<int32_t>* items);
+
+// Double-float Sylvester batches (engine_sides.cu), then one core launch per
+// step (engine_df.cu).  The plans are false when a side does not fit.
 bool sides_plan(SidesPlan* p, int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms,
                 std::vector<int32_t>* items);
 cudaError_t launch_sides_class(const StepArgs<dfloat>& g, const SidesPlan& p, int k, const int32_t* items,
                                cudaStream_t st);
 cudaError_t launch_core(const StepArgs<dfloat>& g, int count, cudaStream_t st);
+
+// FP64 batches (engine_wide.cu): sides, then the cores on clusters of C CTAs.
+struct WidePlan {
+  SidesPlan sides;
+  int C = 0;
+  size_t core_smem = 0;
+};
+bool wide_plan(WidePlan* w, int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms,
+               std::vector<int32_t>* items);
+cudaError_t launch_wide_side(const StepArgs<double>& g, const WidePlan& p, int k, const int32_t* items,
+                             cudaStream_t st);
+cudaError_t launch_wide_core(const StepArgs<double>& g, int count, const WidePlan& p, cudaStream_t st);
+// CTAs per side (a power of two, 1 to 16) for `count` instances of up to `tall`
+// rows: two clusters per instance on SMs of their own, at least four rows each
+int wide_cluster(int count, int64_t tall, int sms);
 
 // double <-> double-float conversions of n elements (dfloat storage is a
 // pair of floats, 8 bytes per element)
@@ -150,6 +164,14 @@ cudaError_t convert_df_to_f64(const void* in, double* out, int64_t n, cudaStream
 template <typename T>
 size_t step_smem_bytes();
 
+// Clusters of the adjoint step (C = 0: adjoint_step_kernel) and the shared
+// memory of its forward recomputation and of its reversal.
+struct AdjointPlan {
+  int C = 0;
+  size_t fwd_smem = 0, rev_smem = 0;
+};
+AdjointPlan adjoint_plan(int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms);
+
 // Discrete adjoint of the FP64 BUG step (adjoint.cu): workspace elements per
 // instance, the largest nstages * nsub it supports, and the launch.
 size_t adjoint_work_elems(int64_t n, int64_t m, int64_t r, int ns_k, int ns_l);
@@ -157,10 +179,7 @@ int adjoint_max_stages();
 cudaError_t launch_adjoint_step(const InstDesc* inst, const int64_t* adj_off, const int64_t* th_off, int count,
                                 const double* U0, const double* S0, const double* V0, double* Ub, double* Sb,
                                 double* Vb, double* thb, const double* opA, const double* opB, double* work,
-                                const Scheme& sK, const Scheme& sL, const Scheme& sS, double dt, const WidePlan& plan,
+                                const Scheme& sK, const Scheme& sL, const Scheme& sS, double dt, const AdjointPlan& plan,
                                 cudaStream_t st);
-// the adjoint's plan on clusters for a batch whose steps take `step` (side_smem:
-// the forward recomputation, core_smem: the reversal); C = 0 where it does not fit
-WidePlan adjoint_plan(const WidePlan& step, int count, const int64_t* n, const int64_t* m, const int64_t* r);
 
 }  // namespace lri

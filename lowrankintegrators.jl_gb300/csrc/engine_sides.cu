@@ -531,36 +531,11 @@ __global__ void __launch_bounds__(WT, 2)
 
 }  // namespace
 
-// Cluster sizes and classes.  Target: at most half of an SM's shared memory, so
-// that two CTAs hide each other's barriers, with the smallest cluster that
-// reaches it; where the batch leaves SMs idle, larger clusters down to 32 rows
-// per CTA.
-bool sides_plan(SidesPlan* p, int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms,
-                std::vector<int32_t>* items) {
-  constexpr size_t half = 112 * 1024;
-  constexpr int least = 32;
-  struct Item {
-    int32_t id;
-    int C;
-    size_t smem;
-    double cost;
-  };
-  std::vector<Item> v;
-  for (int i = 0; i < count; ++i) {
-    if (r[i] > wide::WR_MAX) return false;
-    for (int s = 0; s < 2; ++s) {
-      const int N = (int)(s ? m[i] : n[i]), ri = (int)r[i];
-      int C = 1;
-      while (C < wide::WC_MAX && side_bytes(N, ri, C) > half) C *= 2;
-      while (C < wide::WC_MAX && 4 * (int64_t)C * count <= sms && N >= 2 * C * least) C *= 2;
-      const size_t b = side_bytes(N, ri, C);
-      if (b > kWideSmemMax) return false;
-      v.push_back({(int32_t)(2 * i + s), C, b, (double)N * ri * (ri + 8.0) / C});
-    }
-  }
-  auto group = [&](const Item& x) { return 2 * x.C + (x.smem > half ? 1 : 0); };
-  // classes with the largest clusters first, longest work first inside a class
-  std::stable_sort(v.begin(), v.end(), [&](const Item& a, const Item& b) {
+// Classes by cluster size (the largest first) and by whether two CTAs fit an SM,
+// longest work first inside a class.
+bool group_sides(std::vector<SideItem>& v, SidesPlan* p, std::vector<int32_t>* items) {
+  auto group = [](const SideItem& x) { return 2 * x.C + (x.smem > kHalfSmem ? 1 : 0); };
+  std::stable_sort(v.begin(), v.end(), [&](const SideItem& a, const SideItem& b) {
     const int ga = group(a), gb = group(b);
     return ga != gb ? ga > gb : a.cost > b.cost;
   });
@@ -577,6 +552,26 @@ bool sides_plan(SidesPlan* p, int count, const int64_t* n, const int64_t* m, con
     items->push_back(v[i].id);
   }
   return true;
+}
+
+// Double-float sides: the smallest cluster whose panels leave room for two CTAs
+// on an SM (they hide each other's barriers); where the batch leaves SMs idle,
+// larger clusters down to 32 rows per CTA.
+bool sides_plan(SidesPlan* p, int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms,
+                std::vector<int32_t>* items) {
+  std::vector<SideItem> v;
+  for (int i = 0; i < count; ++i) {
+    if (r[i] > wide::WR_MAX) return false;
+    for (int s = 0; s < 2; ++s) {
+      const int N = (int)(s ? m[i] : n[i]), ri = (int)r[i];
+      int C = 1;
+      while (C < wide::WC_MAX && side_bytes(N, ri, C) > kHalfSmem) C *= 2;
+      while (C < wide::WC_MAX && 4 * (int64_t)C * count <= sms && N >= 64 * C) C *= 2;
+      if (side_bytes(N, ri, C) > kWideSmemMax) return false;
+      v.push_back({(int32_t)(2 * i + s), C, side_bytes(N, ri, C), (double)N * ri * (ri + 8.0) / C});
+    }
+  }
+  return group_sides(v, p, items);
 }
 
 cudaError_t launch_sides_class(const StepArgs<dfloat>& g, const SidesPlan& p, int k, const int32_t* items,

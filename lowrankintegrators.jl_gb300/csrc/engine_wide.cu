@@ -1,5 +1,6 @@
-// engine_wide.cu - FP64 BUG steps of small batches, each instance spread over
-// thread-block clusters (Sylvester flow and data streams).
+// engine_wide.cu - FP64 BUG steps (Sylvester flow and data streams) with the
+// panels of a side in shared memory, each side on one CTA or spread over a
+// thread-block cluster.
 //
 // An FP64 step of one instance is bound by the FP64 units of the SMs it runs
 // on (about 1.9 multiply-adds per clock each); on one 2-CTA pair a batch of
@@ -53,8 +54,7 @@ struct WInst {
   __device__ double* blk(int i) const { return small + (int64_t)i * (((int64_t)W * W + 3) & ~int64_t(3)); }
 };
 
-__device__ __forceinline__ bool wide_inst(const StepArgs<double>& g, int slot, WInst& I) {
-  const int inst = g.order[slot];
+__device__ __forceinline__ bool wide_inst(const StepArgs<double>& g, int inst, WInst& I) {
   const InstDesc d = g.inst[inst];
   I.n = d.n; I.m = d.m; I.W = d.wcap; I.rcap = d.rcap; I.inst = inst;
   I.U = g.U + d.offU;
@@ -104,13 +104,14 @@ __host__ __device__ inline size_t side_doubles(int N, int r, int C) {
   return 3 * (size_t)r * ld + misc_doubles(R0, r) + QrSmem<double>::elems(C, r);
 }
 
-__global__ void __launch_bounds__(WT, 1) wide_sides(const __grid_constant__ StepArgs<double> g, int C) {
+__global__ void __launch_bounds__(WT, 2)
+    wide_sides(const __grid_constant__ StepArgs<double> g, const int32_t* __restrict__ items, int C) {
   extern __shared__ __align__(16) double dsm[];
   Team tm{wide::cg::this_cluster(), (int)wide::cg::this_cluster().block_rank(), C};
-  const int ci = blockIdx.x / C, tid = threadIdx.x;
+  const int item = items[blockIdx.x / C], tid = threadIdx.x;
   WInst I;
-  if (!wide_inst(g, ci >> 1, I)) return;  // the same in every CTA of the cluster
-  const bool kside = (ci & 1) == 0;
+  if (!wide_inst(g, item >> 1, I)) return;  // the same in every CTA of the cluster
+  const bool kside = (item & 1) == 0;
   const int r = I.r, W = I.W, N = kside ? I.n : I.m, No = kside ? I.m : I.n;
   double* X = kside ? I.U : I.V;
   const double* Xo = kside ? I.V : I.U;
@@ -326,7 +327,7 @@ __global__ void __launch_bounds__(WT, 1) wide_core(const __grid_constant__ StepA
   Team tm{wide::cg::this_cluster(), (int)wide::cg::this_cluster().block_rank(), C};
   const int tid = threadIdx.x;
   WInst I;
-  if (!wide_inst(g, blockIdx.x / C, I)) return;
+  if (!wide_inst(g, g.order[blockIdx.x / C], I)) return;
   const bool sylv = g.op == OP_SYLVESTER;
   const int r = I.r, W = I.W, rr = r * r;
   const int cpc = (r + C - 1) / C, c0 = min(r, tm.q * cpc), nc = min(r, c0 + cpc) - c0;  // own columns
@@ -486,45 +487,69 @@ __global__ void __launch_bounds__(WT, 1) wide_core(const __grid_constant__ StepA
   if (tm.q == 0 && tid == 0) g.proj_valid[I.inst] = 1;
 }
 
-cudaError_t cluster_launch(void (*kern)(const StepArgs<double>, int), const StepArgs<double>& g, int blocks, int C,
-                           size_t smem, std::atomic<uint64_t>& done, cudaStream_t st) {
-  cudaError_t e = wide::cluster_attributes(kern, done);
+}  // namespace
+
+int wide_cluster(int count, int64_t tall, int sms) {
+  int C = wide::WC_MAX;
+  while (C > 1 && (2 * (int64_t)C * count > sms || tall < 4 * C)) C /= 2;
+  return C;
+}
+
+// Sides: the smallest cluster whose panels leave room for two CTAs on an SM;
+// where the batch leaves SMs idle, larger clusters, down to four rows per CTA
+// (below that the barriers outweigh the split).  Cores: a cluster only where
+// SMs are idle.
+bool wide_plan(WidePlan* w, int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms,
+               std::vector<int32_t>* items) {
+  std::vector<SideItem> v;
+  w->core_smem = 0;
+  w->C = wide::WC_MAX;
+  while (w->C > 1 && (int64_t)w->C * count > sms) w->C /= 2;
+  int64_t ctas = 0, tall = 0;
+  for (int i = 0; i < count; ++i) {
+    const int ri = (int)r[i];
+    if (ri > wide::WR_MAX) return false;
+    for (int s = 0; s < 2; ++s) {
+      const int N = (int)(s ? m[i] : n[i]);
+      auto bytes = [&](int C) { return sizeof(double) * side_doubles(N, ri, C); };
+      int C = wide_cluster(count, N, sms);
+      while (C < wide::WC_MAX && bytes(C) > kHalfSmem) C *= 2;
+      if (bytes(C) > kWideSmemMax) return false;
+      v.push_back({(int32_t)(2 * i + s), C, bytes(C), (double)N * ri * (ri + 8.0) / C});
+      ctas += C;
+      tall = std::max<int64_t>(tall, N);
+    }
+  }
+  while (w->C > 1 && tall < 4 * w->C) w->C /= 2;
+  for (int i = 0; i < count; ++i)
+    w->core_smem = std::max(w->core_smem, sizeof(double) * core_doubles((int)r[i], w->C));
+  if (w->core_smem > kWideSmemMax) return false;
+  // a few CTAs take an SM each, with all its FP64 units
+  if (ctas <= sms)
+    for (SideItem& x : v) x.smem = std::max(x.smem, (size_t)120 * 1024);
+  return group_sides(v, &w->sides, items);
+}
+
+cudaError_t launch_wide_side(const StepArgs<double>& g, const WidePlan& p, int k, const int32_t* items,
+                             cudaStream_t st) {
+  static std::atomic<uint64_t> done{0};
+  const SidesPlan::Class& c = p.sides.cls[k];
+  cudaError_t e = wide::cluster_attributes(wide_sides, done);
   if (e != cudaSuccess) return e;
   cudaLaunchConfig_t cfg = {};
   cudaLaunchAttribute attr[1];
-  wide::cluster_config(cfg, attr, blocks, C, smem, st);
-  return cudaLaunchKernelEx(&cfg, kern, g, C);
+  wide::cluster_config(cfg, attr, c.C * c.count, c.C, c.smem, st);
+  return cudaLaunchKernelEx(&cfg, wide_sides, g, items + c.first, (int)c.C);
 }
 
-}  // namespace
-
-WidePlan wide_plan(int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms) {
-  WidePlan p;
-  int64_t tall = 0;
-  for (int i = 0; i < count; ++i) tall = std::max(tall, std::max(n[i], m[i]));
-  // Two clusters per instance on SMs of their own, and at least four rows to a
-  // CTA: below that the barriers outweigh the split.
-  int C = wide::WC_MAX;
-  while (C > 1 && (2 * (int64_t)C * count > sms || tall < 4 * C)) C /= 2;
-  if (C < 2) return p;
-  for (int i = 0; i < count; ++i) {
-    const int ri = (int)r[i];
-    if (ri > wide::WR_MAX) return WidePlan{};
-    for (int64_t N : {n[i], m[i]}) p.side_smem = std::max(p.side_smem, sizeof(double) * side_doubles((int)N, ri, C));
-    p.core_smem = std::max(p.core_smem, sizeof(double) * core_doubles(ri, C));
-  }
-  if (p.side_smem > kWideSmemMax || p.core_smem > kWideSmemMax) return WidePlan{};
-  // a CTA per SM, so that each has the SM's FP64 units
-  p.side_smem = std::max(p.side_smem, (size_t)120 * 1024);
-  p.C = C;
-  return p;
-}
-
-cudaError_t launch_wide_step(const StepArgs<double>& g, int count, const WidePlan& p, cudaStream_t st) {
-  static std::atomic<uint64_t> ds{0}, dc{0};
-  cudaError_t e = cluster_launch(wide_sides, g, 2 * p.C * count, p.C, p.side_smem, ds, st);
-  if (e == cudaSuccess) e = cluster_launch(wide_core, g, p.C * count, p.C, p.core_smem, dc, st);
-  return e != cudaSuccess ? e : cudaGetLastError();
+cudaError_t launch_wide_core(const StepArgs<double>& g, int count, const WidePlan& p, cudaStream_t st) {
+  static std::atomic<uint64_t> done{0};
+  cudaError_t e = wide::cluster_attributes(wide_core, done);
+  if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg = {};
+  cudaLaunchAttribute attr[1];
+  wide::cluster_config(cfg, attr, p.C * count, p.C, p.core_smem, st);
+  return cudaLaunchKernelEx(&cfg, wide_core, g, p.C);
 }
 
 }  // namespace lri
