@@ -730,7 +730,7 @@ __global__ void __launch_bounds__(WT, 1) adj_fwd(const __grid_constant__ AdjArgs
       win = wout;
       wout = t;
     }
-  wide::qr<double>(tm, N, lo, rows, r, win + 1, ld, wout + 1, blkp(s.small, W, s.kside ? A_RK : A_RL), W, qs);
+  wide::qr<double>(tm, N, lo, rows, r, win + 1, ld, wout + 1, ld, blkp(s.small, W, s.kside ? A_RK : A_RL), W, qs);
   // M = Q^T X0 and the projections of Q
   double* Q = wout;
   double* part = misc;

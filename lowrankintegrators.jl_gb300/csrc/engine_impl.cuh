@@ -18,6 +18,7 @@
 
 #include "engine.cuh"
 #include "engine_api.h"
+#include "wide.cuh"
 
 namespace lri {
 
@@ -76,8 +77,33 @@ __device__ __noinline__ void projections(const Inst<T>& I, const T* X, int N, in
 // (ld N) and, when R is given, the triangular factor to R (ld ldr).  The
 // panel is factored in shared memory when it fits in the staging area
 // (which the QR does not otherwise use), else in place in global memory.
+// FP64 panels, and panels whose column signs do not matter (any_signs: the
+// rank-adaptive step's augmented bases, rotated by the core's SVD), take the
+// one-reduction-per-column form (wide::qr) where its scratch fits; FP32 bases
+// handed to the caller keep hh_factor's rounding, which decides the sign of a
+// column whose pivot is at rounding level.
 template <typename T>
-__device__ __noinline__ void qr_panel(T* Kp, int N, int W, T* Qdst, T* R, int ldr, Smem<T>& sm) {
+__device__ __noinline__ void qr_panel(T* Kp, int N, int W, T* Qdst, T* R, int ldr, Smem<T>& sm,
+                                      bool any_signs = false) {
+  if (std::is_same<T, double>::value || (any_signs && !R)) {
+    const int scr = ((int)wide::QrSmem<T>::elems(1, W) + 3) & ~3;
+    if (scr <= Stage<T>::ELEMS) {
+      const wide::Team one{cooperative_groups::this_cluster(), 0, 1};
+      const wide::QrSmem<T> qs = wide::QrSmem<T>::carve(sm.stage, 1, W);
+      const int ld = N | 1;  // odd: threads along the columns hit distinct banks
+      T* a = Kp;
+      int lda = N;
+      if ((int64_t)ld * W <= Stage<T>::ELEMS - scr) {
+        a = sm.stage + scr;
+        lda = ld;
+        for (int j = 0; j < W; ++j)
+          for (int i = threadIdx.x; i < N; i += NT) a[i + j * ld] = Kp[i + (int64_t)j * N];
+        __syncthreads();
+      }
+      wide::qr<T>(one, N, 0, N, W, a, lda, Qdst, N, R, ldr, qs);
+      return;
+    }
+  }
   const int off = NW * WMAX;  // hh_* keep their reduction scratch below this offset
   if ((int64_t)N * W <= (int64_t)(Stage<T>::ELEMS - off)) {
     T* A = sm.stage + off;
@@ -728,12 +754,12 @@ __device__ __noinline__ void ra_bug_step(const StepArgs<T>& g, Inst<T>& I, int r
   // K step: Uhat = orth([K1 | U0]) (rank_adaptive_unconventional.jl:197-206)
   k_step<T>(g, I, I.k, 0, I.U, I.S, I.rcap, false, I.k.PY, r, GV, I.V, g.sK, g.dt, sm);
   copy_mat<T>(n, r, I.U, n, I.k.PY + (int64_t)r * n, n);
-  qr_panel<T>(I.k.PY, n, w2, I.k.PQ, nullptr, 0, sm);
+  qr_panel<T>(I.k.PY, n, w2, I.k.PQ, nullptr, 0, sm, true);
   tile_gram<T>(n, w2, r, sm.stage, RowLoadPanel<T>{I.k.PQ, n, w2}, RowLoadPanel<T>{I.U, n, r}, Mm, W, T(1), T(0));
   // L step (:208-217)
   k_step<T>(g, I, I.l, 1, I.V, I.S, I.rcap, true, I.l.PY, r, GU, I.U, g.sL, g.dt, sm);
   copy_mat<T>(m, r, I.V, m, I.l.PY + (int64_t)r * m, m);
-  qr_panel<T>(I.l.PY, m, w2, I.l.PQ, nullptr, 0, sm);
+  qr_panel<T>(I.l.PY, m, w2, I.l.PQ, nullptr, 0, sm, true);
   tile_gram<T>(m, w2, r, sm.stage, RowLoadPanel<T>{I.l.PQ, m, w2}, RowLoadPanel<T>{I.V, m, r}, Nm, W, T(1), T(0));
   // S step on the augmented bases (:219-220)
   if (sylv) {

@@ -488,7 +488,7 @@ __global__ void __launch_bounds__(WT, 2)
     const QrSmem<T> qs = QrSmem<T>::carve(reinterpret_cast<T*>(fac), C, r);
     if (!cholqr(tm, N, lo, rows, r, win + 1, ld, cs)) {  // uniform over the cluster
       tm.barrier();
-      wide::qr<T, true>(tm, N, lo, rows, r, win + 1, ld, wout + 1, static_cast<T*>(nullptr), 0, qs);
+      wide::qr<T, true>(tm, N, lo, rows, r, win + 1, ld, wout + 1, ld, static_cast<T*>(nullptr), 0, qs);
       T* t = win;
       win = wout;
       wout = t;

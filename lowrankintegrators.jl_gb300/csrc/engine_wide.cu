@@ -278,7 +278,7 @@ __global__ void __launch_bounds__(WT, 2)
       __syncthreads();
     }
   }
-  wide::qr<double>(tm, N, lo, rows, r, win + 1, ldr, wout + 1, nullptr, 0, qs);
+  wide::qr<double>(tm, N, lo, rows, r, win + 1, ldr, wout + 1, ldr, nullptr, 0, qs);
   // basis change X1^T X0 and, for the flow, the new basis's projections
   double* Q = wout;
   double* part = misc;

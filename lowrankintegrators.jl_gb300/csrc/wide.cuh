@@ -230,7 +230,7 @@ __device__ __forceinline__ float lead(dfloat x) { return x.hi; }
 
 // Householder QR (LAPACK signs; POS: a positive diagonal of R) of an N x r
 // panel whose rows [lo, lo + rows) are this CTA's a[k ld + i]; the explicit Q
-// goes to qout (same layout) and, when R is given, the factor to R (global, ld
+// goes to qout (ld ldq) and, when R is given, the factor to R (global, ld
 // ldr, zeros below; not with the scaled columns of the FP32-based types).  One
 // cluster barrier per column: a single pass forms x^T A for every column (the
 // trailing ones, and the earlier reflectors for the compact WY form), its
@@ -243,8 +243,8 @@ __device__ __forceinline__ float lead(dfloat x) { return x.hi; }
 // stay inside the FP32 exponent range; their dots are summed in runs of eight
 // rows.
 template <typename T, bool POS = false>
-__device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, T* a, int ld, T* qout, T* R, int ldr,
-                                const QrSmem<T>& s) {
+__device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, T* a, int ld, T* qout, int ldq, T* R,
+                                int ldr, const QrSmem<T>& s) {
   constexpr bool F64 = std::is_same<T, double>::value;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int LT = r + 1;
@@ -435,7 +435,7 @@ __device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, 
       const int j = by_rows.div(e), i = e - j * rows;
       T p = (lo + i == j) ? T(1) : T(0);
       for (int k = 0; k < j; ++k) p = fma(-a[k * ld + i], s.tri[j * LT + k], p);
-      qout[j * ld + i] = fma(-a[j * ld + i], s.tri[j * LT + r], p);
+      qout[(int64_t)j * ldq + i] = fma(-a[j * ld + i], s.tri[j * LT + r], p);
     }
   } else {
     // four columns per thread share the loads of V
@@ -459,7 +459,7 @@ __device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, 
         if (j0 + u < r) {
           T q = ((lo + i == j0 + u) ? T(1) : T(0)) - renorm(p[u]);
           if constexpr (POS) q = q * s.sgn[j0 + u];
-          qout[(j0 + u) * ld + i] = q;
+          qout[(int64_t)(j0 + u) * ldq + i] = q;
         }
     }
   }
