@@ -676,6 +676,9 @@ __device__ bool fused_substep(int N, int r, const T* X, int ldx, const T* C, int
   // area; TR = TH - 2H output rows per tile (multiple of 4, <= 256)
   int TH = ((Stage<T>::ELEMS - 2 * r * ldw) / (3 * r)) & ~3;
   if (TH > 256 + 2 * H + 3) TH = (256 + 2 * H + 3) & ~3;
+  // a tile a little larger than one micro-tile per thread would take two
+  // rounds, the second nearly empty (ranks 13-15, 17, 18, 21)
+  if (TH / 4 * c4 > NT && TH / 4 * c4 <= NT + NT / 4) TH = NT / c4 * 4;
   const int TR = (TH - 2 * H) & ~3;
   if (TR < 16) return false;
   T* bufA = stage;
@@ -1389,7 +1392,7 @@ __device__ __noinline__ void tile_gram_acc(int N, int a, int c, float* stage, co
   const int MT = a4 * c4;  // <= NT
   const int lxs = a4 * 4 + 4, lys = c4 * 4 + 4;
   float* xs = stage;
-  float* ys = stage + TRG * lxs;
+  float* ys;
   const int splits = NT / MT;
   const int mt = tid % MT, split = tid / MT;
   const bool active = split < splits;
@@ -1397,23 +1400,34 @@ __device__ __noinline__ void tile_gram_acc(int N, int a, int c, float* stage, co
   dfloat acc[16];
 #pragma unroll
   for (int e = 0; e < 16; ++e) acc[e] = dfloat(0.0f, 0.0f);
-  for (int i0 = 0; i0 < N; i0 += TRG) {
-    const int rows = min(TRG, N - i0);
-    lx(xs, i0, rows, lxs);
-    ly(ys, i0, rows, lys);
+  // as many chunks of TRG rows per stage as the staging area holds (two
+  // barriers per stage); sums renormalised after every chunk
+  const int ch = max(1, Stage<float>::ELEMS / (TRG * (lxs + lys)));
+  ys = stage + ch * TRG * lxs;
+  for (int s0 = 0; s0 < N; s0 += ch * TRG) {
+    for (int c = 0; c < ch && s0 + c * TRG < N; ++c) {
+      const int i0 = s0 + c * TRG, rows = min(TRG, N - i0);
+      lx(xs + c * TRG * lxs, i0, rows, lxs);
+      ly(ys + c * TRG * lys, i0, rows, lys);
+    }
     __syncthreads();
     if (active) {
-      for (int ii = split; ii < rows; ii += splits) {
-        float xv[4], yv[4];
-        ld4(xs + ii * lxs + 4 * ma, xv);
-        ld4(ys + ii * lys + 4 * mc, yv);
+      for (int c = 0; c < ch && s0 + c * TRG < N; ++c) {
+        const int rows = min(TRG, N - s0 - c * TRG);
+        const float* xc = xs + c * TRG * lxs;
+        const float* yc = ys + c * TRG * lys;
+        for (int ii = split; ii < rows; ii += splits) {
+          float xv[4], yv[4];
+          ld4(xc + ii * lxs + 4 * ma, xv);
+          ld4(yc + ii * lys + 4 * mc, yv);
 #pragma unroll
-        for (int p = 0; p < 4; ++p)
+          for (int p = 0; p < 4; ++p)
 #pragma unroll
-          for (int q = 0; q < 4; ++q) acc[p * 4 + q] = acc_mul_acc(acc[p * 4 + q], xv[p], yv[q]);
+            for (int q = 0; q < 4; ++q) acc[p * 4 + q] = acc_mul_acc(acc[p * 4 + q], xv[p], yv[q]);
+        }
+#pragma unroll
+        for (int e = 0; e < 16; ++e) acc[e] = renorm(acc[e]);
       }
-#pragma unroll
-      for (int e = 0; e < 16; ++e) acc[e] = renorm(acc[e]);
     }
     __syncthreads();
   }
