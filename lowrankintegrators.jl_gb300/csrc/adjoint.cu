@@ -615,6 +615,7 @@ __global__ void __launch_bounds__(WT, 1) adj_fwd(const __grid_constant__ AdjArgs
   const int R0 = tm.rows_per(N), lo = tm.lo(N), rows = tm.hi(N) - lo, ld = (int)adj_ld(N, C);
   const int64_t len = (int64_t)N * r;
   const Tri T{s.tri, N, lo};
+  const wide::FastDiv by_rows(rows);
   double* p0 = dsm;
   double* p1 = p0 + (size_t)r * ld;
   double* y = p1 + (size_t)r * ld;
@@ -669,7 +670,7 @@ __global__ void __launch_bounds__(WT, 1) adj_fwd(const __grid_constant__ AdjArgs
   load_rows(s.X0, N, lo, rows, r, p1, ld);
   __syncthreads();
   for (int e = tid; e < rows * r; e += WT) {
-    const int i = e % rows, c = e / rows;
+    const int c = by_rows.div(e), i = e - c * rows;
     double v = 0.0;
     for (int k = 0; k < r; ++k) v = fma(p1[k * ld + 1 + i], Ps[k * r + c], v);
     p0[c * ld + 1 + i] = y[c * ld + 1 + i] = v;
@@ -692,11 +693,11 @@ __global__ void __launch_bounds__(WT, 1) adj_fwd(const __grid_constant__ AdjArgs
       int big = full;
       if (!full) {
         for (int e = tid; e < rows * r; e += WT) {
-          const int i = e % rows, k = e / rows;
+          const int k = by_rows.div(e), i = e - k * rows;
           const double tw = T.mul(win, ld, i, k);
           wout[k * ld + 1 + i] = tw;
           tf[e] = (float)tw;
-          big |= !(fabs(tw) < 0x1p100);
+          big |= !wide::below_2_100(tw);
         }
         big = __syncthreads_or(big);
       }
@@ -704,7 +705,7 @@ __global__ void __launch_bounds__(WT, 1) adj_fwd(const __grid_constant__ AdjArgs
       const double bs = sc.b[st], ha = last ? 0.0 : h * sc.a[st + 1];
       double* Zn = s.Z + (int64_t)(sub * sc.nstages + st + 1) * len;
       for (int e = tid; e < rows * r; e += WT) {
-        const int i = e % rows, c = e / rows, o = c * ld + 1 + i;
+        const int c = by_rows.div(e), i = e - c * rows, o = c * ld + 1 + i;
         double v;
         if (!big) {
           float ef = 0.0f;
@@ -738,12 +739,12 @@ __global__ void __launch_bounds__(WT, 1) adj_fwd(const __grid_constant__ AdjArgs
   push_halos(tm, N, rows, r, Q, ld);
   tm.cl.sync();
   for (int e = tid; e < rows * r; e += WT) {
-    const int i = e % rows, k = e / rows;
+    const int k = by_rows.div(e), i = e - k * rows;
     y[k * ld + 1 + i] = T.mul(Q, ld, i, k);
     s.Q[lo + i + (int64_t)k * N] = Q[k * ld + 1 + i];
   }
   __syncthreads();
-  outputs(3 * rr, [&](int o, int l, int L) {
+  outputs(3 * rr, rows, [&](int o, int l, int L) {
     const int a = o % r, c = (o / r) % r, w = o / rr;
     if (w == 1 && a > c) return 0.0;
     const double* x = (w == 0) ? win : (w == 1 ? Q : y);
@@ -768,13 +769,14 @@ template <class F>
 __device__ __forceinline__ void dgemm(const Team& tm, int r, int W, const double* A, bool ta, const double* B, bool tb,
                                       const F& fin) {
   const int per = (r * r + tm.C - 1) / tm.C, e0 = tm.q * per, e1 = min(r * r, e0 + per);
-  outputs(max(0, e1 - e0), [&](int o, int l, int L) {
+  outputs(max(0, e1 - e0), r, [&](int o, int l, int L) {
     const int i = (e0 + o) % r, j = (e0 + o) / r;
     double v = 0.0;
     for (int k = l; k < r; k += L)
       v = fma(ta ? A[k + (int64_t)i * W] : A[i + (int64_t)k * W], tb ? B[j + (int64_t)k * W] : B[k + (int64_t)j * W], v);
     return v;
-  }, [&](int o, double v) { fin((e0 + o) % r + (int64_t)((e0 + o) / r) * W, v); });
+  }, [&](int o, double v) { fin((e0 + o) % r + (int64_t)((e0 + o) / r) * W, v); },
+          wide::lanes_for(max(1, e1 - e0)));  // (operands from L2: latency, not FP64 issue)
 }
 
 // Phase 2: the S step forward and reversed; entries split over one cluster,
@@ -887,14 +889,15 @@ __device__ __forceinline__ double proj_adj(const double* X, const double* TX, co
 // theta_bar[lo + i] += sum_c X(i, c) sum_k X(i, k) C1(c, k)
 __device__ void theta_proj(const Team& tm, int rows, int lo, int r, const double* X, int ld, const double* C1s,
                            double* scr, double* thb) {
+  const wide::FastDiv by_rows(rows);
   for (int e = threadIdx.x; e < rows * r; e += WT) {
-    const int i = e % rows, c = e / rows;
+    const int c = by_rows.div(e), i = e - c * rows;
     double v = 0.0;
     for (int k = 0; k < r; ++k) v = fma(X[k * ld + 1 + i], C1s[c * r + k], v);
     scr[c * ld + 1 + i] = v * X[c * ld + 1 + i];
   }
   __syncthreads();
-  outputs(rows, [&](int i, int l, int L) {
+  outputs(rows, r, [&](int i, int l, int L) {
     double v = 0.0;
     for (int c = l; c < r; c += L) v += scr[c * ld + 1 + i];
     return v;
@@ -920,6 +923,7 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
   const int lo = tm.lo(N), rows = tm.hi(N) - lo, ld = (int)adj_ld(N, C);
   const int64_t len = (int64_t)N * r;
   const Tri T{s.tri, N, lo};
+  const wide::FastDiv by_rows(rows);
   double* p0 = dsm;
   double* p1 = p0 + (size_t)r * ld;
   double* yb = p1 + (size_t)r * ld;
@@ -940,13 +944,13 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
   load_rows(s.X0, N, lo, rows, r, p1, ld);
   __syncthreads();
   for (int e = tid; e < rows * r; e += WT) {
-    const int i = e % rows, k = e / rows;
+    const int k = by_rows.div(e), i = e - k * rows;
     p3[k * ld + 1 + i] = T.mul(p0, ld, i, k);
     p4[k * ld + 1 + i] = T.mul_t(p0, ld, i, k);
   }
   __syncthreads();
   for (int e = tid; e < rows * r; e += WT) {
-    const int i = e % rows, c = e / rows;
+    const int c = by_rows.div(e), i = e - c * rows;
     double v = s.Xb[lo + i + (int64_t)c * N], x = 0.0;
     for (int k = 0; k < r; ++k) {
       v = fma(p1[k * ld + 1 + i], Mb[c * r + k], v);
@@ -961,7 +965,7 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
   {
     double* part = misc + 2 * rr;
     __syncthreads();
-    outputs(rr, [&](int o, int l, int L) {
+    outputs(rr, rows, [&](int o, int l, int L) {
       const int a = o % r, c = o / r;
       double v = 0.0;
       for (int i = 1 + l; i <= rows; i += L) v = fma(-yb[a * ld + i], p0[c * ld + i], v);
@@ -980,7 +984,7 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
     if (tid < r) inv[tid] = 1.0 / R[tid + (int64_t)tid * W];
     __syncthreads();
     for (int e = tid; e < rows * r; e += WT) {
-      const int i = e % rows, c = e / rows;
+      const int c = by_rows.div(e), i = e - c * rows;
       double v = yb[c * ld + 1 + i];
       for (int k = 0; k < r; ++k) v = fma(p0[k * ld + 1 + i], Cl[k * r + c], v);
       yb[c * ld + 1 + i] = v;
@@ -1025,13 +1029,13 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
   tm.cl.sync();
   for (int sub = sc.nsub - 1; sub >= 0; --sub) {
     for (int e = tid; e < rows * r; e += WT) {
-      const int o = (e / rows) * ld + 1 + e % rows;
+      const int q = by_rows.div(e), o = q * ld + 1 + e - q * rows;
       ybn[o] = yb[o];
     }
     for (int st = sc.nstages - 1; st >= 0; --st) {
       const double hb = h * sc.b[st], ha = (st + 1 < sc.nstages) ? h * sc.a[st + 1] : 0.0;
       for (int e = tid; e < rows * r; e += WT) {  // every thread its own entries
-        const int o = (e / rows) * ld + 1 + e % rows;
+        const int q = by_rows.div(e), o = q * ld + 1 + e - q * rows;
         kb[o] = (st + 1 < sc.nstages) ? fma(ha, p3[o], hb * ybn[o]) : hb * ybn[o];
       }
       load_rows_halo(s.Z + (int64_t)(sub * sc.nstages + st) * len, N, lo, rows, r, z, ld);
@@ -1039,12 +1043,12 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
       push_halos(tm, N, rows, r, kb, ld);
       int zbig = full;
       for (int e = tid; e < rows * r; e += WT) {
-        const int o = (e / rows) * ld + 1 + e % rows;
+        const int q = by_rows.div(e), o = q * ld + 1 + e - q * rows;
         p3[o] = T.mul(z, ld, e % rows, e / rows);
-        zbig |= !(fabs(z[o]) < 0x1p100);
+        zbig |= !wide::below_2_100(z[o]);
       }
       tm.cl.sync();
-      outputs(2 * rr, [&](int o, int l, int L) {
+      outputs(2 * rr, rows, [&](int o, int l, int L) {
         const int a = o % r, c = (o / r) % r;
         const double* x = (o < rr) ? p3 : kb;
         const double* y = (o < rr) ? kb : z;
@@ -1055,7 +1059,7 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
       zbig = __syncthreads_or(zbig);  // T z is consumed
       if (s.kside) {
         for (int e = tid; e < rows * r; e += WT) {
-          const int i = e % rows, c = e / rows;
+          const int c = by_rows.div(e), i = e - c * rows;
           double v;
           if (!zbig) {
             float ef = 0.0f;  // Es holds the transpose of G - I
@@ -1068,7 +1072,7 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
           p3[c * ld + 1 + i] = v * kb[c * ld + 1 + i];
         }
         __syncthreads();
-        outputs(rows, [&](int i, int l, int L) {
+        outputs(rows, r, [&](int i, int l, int L) {
           double v = 0.0;
           for (int c = l; c < r; c += L) v += p3[c * ld + 1 + i];
           return v;
@@ -1078,16 +1082,16 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
       int big = full;
       if (!full) {
         for (int e = tid; e < rows * r; e += WT) {
-          const int i = e % rows, k = e / rows;
+          const int k = by_rows.div(e), i = e - k * rows;
           const double tk = T.mul_t(kb, ld, i, k);
           p3[k * ld + 1 + i] = tk;
           tf[e] = (float)tk;
-          big |= !(fabs(tk) < 0x1p100);
+          big |= !wide::below_2_100(tk);
         }
         big = __syncthreads_or(big);
       }
       for (int e = tid; e < rows * r; e += WT) {
-        const int i = e % rows, c = e / rows, o = c * ld + 1 + i;
+        const int c = by_rows.div(e), i = e - c * rows, o = c * ld + 1 + i;
         double v;
         if (!big) {
           float ef = 0.0f;
@@ -1112,12 +1116,12 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
   load_rows(s.X0, N, lo, rows, r, p4, ld);
   __syncthreads();
   for (int e = tid; e < rows * r; e += WT) {
-    const int i = e % rows, c = e / rows;
+    const int c = by_rows.div(e), i = e - c * rows;
     double v = s.xb[lo + i + (int64_t)c * N];
     for (int k = 0; k < r; ++k) v = fma(yb[k * ld + 1 + i], Ps[k * r + c], v);
     s.xb[lo + i + (int64_t)c * N] = v;
   }
-  outputs(rr, [&](int o, int l, int L) {
+  outputs(rr, rows, [&](int o, int l, int L) {
     const int a = o % r, c = o / r;
     const double* x = s.kside ? p4 : yb;
     const double* y = s.kside ? yb : p4;
@@ -1145,6 +1149,7 @@ __global__ void __launch_bounds__(WT, 1) adj_out(const __grid_constant__ AdjArgs
   const int r = s.r, W = s.W, N = s.N, rr = r * r;
   const int lo = tm.lo(N), rows = tm.hi(N) - lo, ld = (int)adj_ld(N, C);
   const Tri T{s.tri, N, lo};
+  const wide::FastDiv by_rows(rows);
   double* p0 = dsm;
   double* p3 = p0 + (size_t)r * ld;
   double* p4 = p3 + (size_t)r * ld;
@@ -1156,13 +1161,13 @@ __global__ void __launch_bounds__(WT, 1) adj_out(const __grid_constant__ AdjArgs
   load_rows_halo(s.X0, N, lo, rows, r, p0, ld);
   __syncthreads();
   for (int e = tid; e < rows * r; e += WT) {
-    const int i = e % rows, k = e / rows;
+    const int k = by_rows.div(e), i = e - k * rows;
     p3[k * ld + 1 + i] = T.mul(p0, ld, i, k);
     p4[k * ld + 1 + i] = T.mul_t(p0, ld, i, k);
   }
   __syncthreads();
   for (int e = tid; e < rows * r; e += WT) {
-    const int i = e % rows, c = e / rows;
+    const int c = by_rows.div(e), i = e - c * rows;
     const int64_t o = lo + i + (int64_t)c * N;
     s.Xb[o] = proj_adj(p0, p3, p4, ld, r, i, c, C1s, C2s, s.xb[o]);
   }

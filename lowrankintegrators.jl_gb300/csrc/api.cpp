@@ -101,6 +101,7 @@ Scheme to_scheme(const lri_scheme& s) {
     o.b[i] = s.b[i];
     o.c[i] = s.c[i];
   }
+  o.set_stability();
   return o;
 }
 
@@ -340,7 +341,7 @@ lri_status lri_batch_create(lri_batch** out, const lri_batch_desc* desc, const l
     if (ok && desc->dtype == LRI_DF)
       ok = lri::sides_plan(&b->wide.sides, count, b->n.data(), b->m.data(), b->r.data(), sms, &items);
     else if (ok)
-      ok = lri::wide_plan(&b->wide, count, b->n.data(), b->m.data(), b->r.data(), sms, &items);
+      ok = lri::wide_plan(&b->wide, count, b->n.data(), b->m.data(), b->r.data(), !sylv, sms, &items);
     if (!ok) b->wide.sides.nclass = 0;
     if (desc->dtype == LRI_F64 && sylv)
       b->adj_plan = lri::adjoint_plan(count, b->n.data(), b->m.data(), b->rcap.data(), sms);

@@ -38,6 +38,20 @@ enum StatusBits : uint32_t {
 struct Scheme {
   int32_t nstages, nsub;
   double a[4], b[4], c[4];
+  // stability polynomial R(z) = sum_j gam[j] z^j, gam[0] = 1, gam[j+1] =
+  // sum_{s>=j} b_s a_s a_{s-1} ... a_{s-j+1} (set_stability; the kernels by
+  // sides take it from here: on the device it is a chain of FP64 operations
+  // in every thread)
+  double gam[5];
+  void set_stability() {
+    for (int j = 0; j < 5; ++j) gam[j] = (j == 0) ? 1.0 : 0.0;
+    for (int j = 0; j < nstages; ++j)
+      for (int s = j; s < nstages; ++s) {
+        double p = b[s];
+        for (int t = s - j + 1; t <= s; ++t) p *= a[t];
+        gam[j + 1] += p;
+      }
+  }
 };
 
 // Per-instance descriptor (device resident).
@@ -148,7 +162,7 @@ struct WidePlan {
   int C = 0;
   size_t core_smem = 0;
 };
-bool wide_plan(WidePlan* w, int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms,
+bool wide_plan(WidePlan* w, int count, const int64_t* n, const int64_t* m, const int64_t* r, bool data, int sms,
                std::vector<int32_t>* items);
 cudaError_t launch_wide_side(const StepArgs<double>& g, const WidePlan& p, int k, const int32_t* items,
                              cudaStream_t st);

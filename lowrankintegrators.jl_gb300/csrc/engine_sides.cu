@@ -440,13 +440,11 @@ __global__ void __launch_bounds__(WT, 2)
   tm.barrier();
   // Horner form of the substep flow: w <- g_j y + h (T w + w P^T)
   const Scheme& sc = kside ? g.sK : g.sL;
-  double gam[5];
-  horner_coeffs(sc, gam);
   const T h = T(g.dt / sc.nsub);
   for (int sub = 0; sub < sc.nsub; ++sub) {
-    T hw = h * T(gam[sc.nstages]);
+    T hw = h * T(sc.gam[sc.nstages]);
     for (int j = sc.nstages - 1; j >= 0; --j) {
-      const T gj = (j == 0) ? T(1) : T(gam[j]);
+      const T gj = (j == 0) ? T(1) : T(sc.gam[j]);
       const bool up = tm.q > 0, dn = tm.q + 1 < C && lo + rows < N;
       panel_mul(rows, r, win + 1, ld, mat, rp, [&](int i, int c0, const T (&acc)[4]) {
         const T cs = ts[i], cd = ts[R0 + i], cp = ts[2 * R0 + i];

@@ -75,21 +75,6 @@ __device__ __forceinline__ bool wide_inst(const StepArgs<double>& g, int inst, W
   return true;
 }
 
-// Coefficients of the stability polynomial R(z) = sum_j gam[j] z^j of an
-// explicit RK scheme with a sub-diagonal tableau (gam[0] = 1).
-__device__ void wide_horner(const Scheme& sc, double gam[5]) {
-  for (int j = 0; j < 5; ++j) gam[j] = (j == 0) ? 1.0 : 0.0;
-  for (int j = 0; j < sc.nstages; ++j) {
-    double sum = 0.0;
-    for (int st = j; st < sc.nstages; ++st) {
-      double prod = sc.b[st];
-      for (int t = st - j + 1; t <= st; ++t) prod *= sc.a[t];
-      sum += prod;
-    }
-    gam[j + 1] = sum;
-  }
-}
-
 // Shared memory of wide_sides: three panels of the cluster's rows, p[k ld + 1 +
 // i] with a halo row on each side (i = -1 and i = R0), the small matrices and
 // the FP32 copy of T w (later the Gram partials, or a data step's chunks), the
@@ -121,6 +106,7 @@ __global__ void __launch_bounds__(WT, 2)
   const bool fresh = sylv && g.proj_valid[I.inst] == 0;
   const int R0 = tm.rows_per(N), lo = tm.lo(N), rows = tm.hi(N) - lo;
   const Tri T{kside ? I.opA : I.opB, N, lo};
+  const wide::FastDiv by_rows(rows);
   const int ldr = (R0 + 2) | 1;
   // carve
   double* sp = dsm;
@@ -180,7 +166,7 @@ __global__ void __launch_bounds__(WT, 2)
   load_rows(X, N, lo, rows, r, p1, ldr);
   __syncthreads();
   for (int e = tid; e < rows * r; e += WT) {
-    const int i = e % rows, c = e / rows;
+    const int c = by_rows.div(e), i = e - c * rows;
     double s = 0.0;
     for (int k = 0; k < r; ++k) s = fma(p1[k * ldr + 1 + i], Cs[k * r + c], s);
     p0[c * ldr + 1 + i] = s;
@@ -211,27 +197,25 @@ __global__ void __launch_bounds__(WT, 2)
     push_halos(tm, N, rows, r, win, ldr);
     tm.cl.sync();
     const Scheme& sc = kside ? g.sK : g.sL;
-    double gam[5];
-    wide_horner(sc, gam);
     const double h = g.dt / sc.nsub;
     for (int sub = 0; sub < sc.nsub; ++sub) {
-      double hw = h * gam[sc.nstages];
+      double hw = h * sc.gam[sc.nstages];
       for (int j = sc.nstages - 1; j >= 0; --j) {
-        const double gj = (j == 0) ? 1.0 : gam[j];
+        const double gj = (j == 0) ? 1.0 : sc.gam[j];
         int big = full;
         if (!full) {
           // T w into this thread's own entries of wout, its FP32 copy for the row
           for (int e = tid; e < rows * r; e += WT) {
-            const int i = e % rows, k = e / rows;
+            const int k = by_rows.div(e), i = e - k * rows;
             const double tw = T.mul(win, ldr, i, k);
             wout[k * ldr + 1 + i] = tw;
             tf[e] = (float)tw;
-            big |= !(fabs(tw) < 0x1p100);
+            big |= !wide::below_2_100(tw);
           }
           big = __syncthreads_or(big);
         }
         for (int e = tid; e < rows * r; e += WT) {
-          const int i = e % rows, c = e / rows;
+          const int c = by_rows.div(e), i = e - c * rows;
           double s;
           if (!big) {
             float ef = 0.0f;
@@ -269,7 +253,7 @@ __global__ void __launch_bounds__(WT, 2)
       }
       for (int e = tid; e < nj * r; e += WT) xo[(e % nj) * r + e / nj] = Xo[j0 + e % nj + (int64_t)(e / nj) * No];
       __syncthreads();
-      outputs(rows * r, [&](int o, int l, int L) {
+      outputs(rows * r, nj, [&](int o, int l, int L) {
         const int i = o % rows, c = o / rows;
         double s = 0.0;
         for (int jj = l; jj < nj; jj += L) s = fma(dl[jj * R0 + i], xo[jj * r + c], s);
@@ -286,11 +270,14 @@ __global__ void __launch_bounds__(WT, 2)
   if (sylv) {
     push_halos(tm, N, rows, r, Q, ldr);
     tm.cl.sync();
-    for (int e = tid; e < rows * r; e += WT) p2[(e / rows) * ldr + 1 + e % rows] = T.mul(Q, ldr, e % rows, e / rows);
+    for (int e = tid; e < rows * r; e += WT) {
+      const int k = by_rows.div(e), i = e - k * rows;
+      p2[k * ldr + 1 + i] = T.mul(Q, ldr, i, k);
+    }
   }
   __syncthreads();
   const int nout = (sylv ? 3 : 1) * r * r;
-  outputs(nout, [&](int o, int l, int L) {
+  outputs(nout, rows, [&](int o, int l, int L) {
     const int a = o % r, c = (o / r) % r, w = o / (r * r);
     if (w == 1 && a > c) return 0.0;  // G is symmetric
     const double* y = (w == 0) ? win : (w == 1 ? Q : p2);
@@ -359,14 +346,14 @@ __global__ void __launch_bounds__(WT, 1) wide_core(const __grid_constant__ StepA
   for (int e = tid; e < r * nc; e += WT) gv[e] = Nn[c0 + e / r + (int64_t)(e % r) * W];  // N(c, k)
   __syncthreads();
   // S~0 = M (S0 N^T), own columns, to every CTA
-  outputs(r * nc, [&](int o, int l, int L) {
+  outputs(r * nc, r, [&](int o, int l, int L) {
     const int i = o % r, c = o / r;
     double s = 0.0;
     for (int k = l; k < r; k += L) s = fma(Z1[i + k * r], gv[k + c * r], s);
     return s;
   }, [&](int o, double v) { t1[o] = v; });
   __syncthreads();
-  outputs(r * nc, [&](int o, int l, int L) {
+  outputs(r * nc, r, [&](int o, int l, int L) {
     const int i = o % r, c = o / r;
     double s = 0.0;
     for (int k = l; k < r; k += L) s = fma(PU[i + k * r], t1[k + c * r], s);
@@ -392,7 +379,7 @@ __global__ void __launch_bounds__(WT, 1) wide_core(const __grid_constant__ StepA
           dy[(e / ni) * 32 + e % ni] = I.Yn[o] - I.Yp[o];
         }
         __syncthreads();
-        outputs(ni * r, [&](int o, int l, int L) {
+        outputs(ni * r, nj, [&](int o, int l, int L) {
           const int i = o % ni, c = o / ni;
           double s = 0.0;
           for (int jj = l; jj < nj; jj += L) s = fma(dy[jj * 32 + i], I.QV[j0 + jj + (int64_t)c * I.m], s);
@@ -400,7 +387,7 @@ __global__ void __launch_bounds__(WT, 1) wide_core(const __grid_constant__ StepA
         }, [&](int o, double v) { zc[(o / ni) * 32 + o % ni] += v; });
       }
       __syncthreads();
-      outputs(rr, [&](int o, int l, int L) {
+      outputs(rr, ni, [&](int o, int l, int L) {
         const int a = o % r, c = o / r;
         double s = 0.0;
         for (int i = l; i < ni; i += L) s = fma(I.QU[i0 + i + (int64_t)a * I.n], zc[c * 32 + i], s);
@@ -440,7 +427,7 @@ __global__ void __launch_bounds__(WT, 1) wide_core(const __grid_constant__ StepA
   for (int sub = 0; sub < sc.nsub; ++sub)
     for (int s = 0; s < sc.nstages; ++s) {
       // t1 = Z G_V, t2 = Z P_V^T (own columns)
-      outputs(2 * r * nc, [&](int o, int l, int L) {
+      outputs(2 * r * nc, r, [&](int o, int l, int L) {
         const int e = (o < r * nc) ? o : o - r * nc, i = e % r, c = e / r;
         const double* b = (o < r * nc) ? gv : pv;
         double v = 0.0;
@@ -450,7 +437,7 @@ __global__ void __launch_bounds__(WT, 1) wide_core(const __grid_constant__ StepA
       __syncthreads();
       const bool last = s + 1 == sc.nstages;
       const double bs = sc.b[s], ha = last ? 0.0 : h * sc.a[s + 1];
-      outputs(r * nc, [&](int o, int l, int L) {
+      outputs(r * nc, 2 * r, [&](int o, int l, int L) {
         const int i = o % r, c = o / r;
         double v = 0.0;
         for (int k = l; k < r; k += L) v = fma(PU[i + k * r], t1[k + c * r], fma(GU[i + k * r], t2[k + c * r], v));
@@ -499,16 +486,17 @@ int wide_cluster(int count, int64_t tall, int sms) {
 // where the batch leaves SMs idle, larger clusters, down to four rows per CTA
 // (below that the barriers outweigh the split).  Cores: a cluster only where
 // SMs are idle.
-bool wide_plan(WidePlan* w, int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms,
+bool wide_plan(WidePlan* w, int count, const int64_t* n, const int64_t* m, const int64_t* r, bool data, int sms,
                std::vector<int32_t>* items) {
   std::vector<SideItem> v;
   w->core_smem = 0;
   w->C = wide::WC_MAX;
   while (w->C > 1 && (int64_t)w->C * count > sms) w->C /= 2;
-  int64_t ctas = 0, tall = 0;
+  int64_t ctas = 0, tall = 0, rmax = 0;
   for (int i = 0; i < count; ++i) {
     const int ri = (int)r[i];
     if (ri > wide::WR_MAX) return false;
+    rmax = std::max(rmax, r[i]);
     for (int s = 0; s < 2; ++s) {
       const int N = (int)(s ? m[i] : n[i]);
       auto bytes = [&](int C) { return sizeof(double) * side_doubles(N, ri, C); };
@@ -520,7 +508,8 @@ bool wide_plan(WidePlan* w, int count, const int64_t* n, const int64_t* m, const
       tall = std::max<int64_t>(tall, N);
     }
   }
-  while (w->C > 1 && tall < 4 * w->C) w->C /= 2;
+  // (a core's columns are what its CTAs share, in a data step also its rows)
+  while (w->C > 1 && (tall < 4 * w->C || (!data && rmax <= w->C / 2))) w->C /= 2;
   for (int i = 0; i < count; ++i)
     w->core_smem = std::max(w->core_smem, sizeof(double) * core_doubles((int)r[i], w->C));
   if (w->core_smem > kWideSmemMax) return false;

@@ -109,20 +109,42 @@ __device__ __forceinline__ int lanes_for(int nout) {
   return L;
 }
 
-// out(o) for o in [0, nout): f(o, l, L) returns lane l's share (of L) of the
-// sum, summed over the lanes; done(o, v) runs on one lane.
+// Lanes per output for nout FP64 sums of K terms: a warp's FP64 instruction
+// occupies its scheduler's unit for 64 clocks, so the cost is the instructions
+// per scheduler, ceil(warps / 4) (ceil(K / L) + log2 L); more lanes shorten the
+// sums but add shuffle-and-add steps that whole warps execute.
+__device__ __forceinline__ int lanes_f64(int nout, int K) {
+  int best = 1 << 30, L = 1;
+#pragma unroll
+  for (int g = 0; g <= 5; ++g) {
+    const int warps = ((nout << g) + 31) >> 5, cost = ((warps + 3) >> 2) * (((K + (1 << g) - 1) >> g) + g);
+    if (cost < best) {
+      best = cost;
+      L = 1 << g;
+    }
+  }
+  return L;
+}
+
+// out(o) for o in [0, nout): f(o, l, L) returns lane l's share (of L) of a sum
+// of K terms, summed over the lanes; done(o, v) runs on one lane.  (L given:
+// sums bound by something else than FP64 issue.)
 template <class F, class D>
-__device__ __forceinline__ void outputs(int nout, const F& f, const D& done) {
-  const int L = lanes_for(nout);
+__device__ __forceinline__ void outputs(int nout, int K, const F& f, const D& done, int L = 0) {
+  if (L == 0) L = lanes_f64(nout, K);
   const int l = threadIdx.x & (L - 1);
   const int per = WT / L;
-  for (int o0 = 0; o0 < nout; o0 += per) {  // uniform trip count: every lane reaches the shuffles
+  const int warp0 = (threadIdx.x & ~31) / L;  // the warp's first output of a round
+  for (int o0 = 0; o0 + warp0 < nout; o0 += per) {  // warp-uniform: every lane reaches the shuffles
     const int o = o0 + threadIdx.x / L;
     double v = (o < nout) ? f(o, l, L) : 0.0;
     for (int s = L >> 1; s > 0; s >>= 1) v += __shfl_xor_sync(0xffffffffu, v, s);
     if (o < nout && l == 0) done(o, v);
   }
 }
+
+// |x| < 2^100 without an FP64 instruction (false for NaN)
+__device__ __forceinline__ bool below_2_100(double x) { return (__double2hiint(x) & 0x7fffffff) < 0x46300000; }
 
 // Adds every CTA's part[0 .. len) (shared memory, the same address in every
 // CTA): done(e, sum) runs for each e on one CTA.  The terms are added in
@@ -227,6 +249,29 @@ __device__ __forceinline__ float two_to(float, int e) { return ldexpf(1.0f, e); 
 __device__ __forceinline__ dfloat two_to(dfloat, int e) { return dfloat(ldexpf(1.0f, e), 0.0f); }
 __device__ __forceinline__ float lead(float x) { return x; }
 __device__ __forceinline__ float lead(dfloat x) { return x.hi; }
+__device__ __forceinline__ float lead(double x) { return (float)x; }
+
+// Square root and reciprocal of the reflector's scalars.  FP64: Newton steps
+// from the FP32 estimates (about 12 and 5 FP64 instructions, where the library
+// calls take some 25 and 12; one warp's chain of them is on the critical path
+// of every column), within the FP32 exponent range, else the library's.
+__device__ __forceinline__ float root(float x) { return sqrtf(x); }
+__device__ __forceinline__ dfloat root(dfloat x) { return lri_df::sqrt(x); }
+__device__ __forceinline__ double root(double x) {
+  if (!(x > 1.0e-30 && x < 1.0e30)) return ::sqrt(x);
+  double y = (double)rsqrtf((float)x);
+  y = y * fma(-0.5 * (x * y), y, 1.5);
+  y = y * fma(-0.5 * (x * y), y, 1.5);
+  const double s = x * y;
+  return fma(fma(-s, s, x), 0.5 * y, s);
+}
+__device__ __forceinline__ float reciprocal(float x) { return 1.0f / x; }
+__device__ __forceinline__ dfloat reciprocal(dfloat x) { return dfloat(1.0f, 0.0f) / x; }
+__device__ __forceinline__ double reciprocal(double x) {  // 1e-30 < |x| < 1e30
+  double q = (double)(1.0f / (float)x);
+  q = fma(q, fma(-x, q, 1.0), q);
+  return fma(q, fma(-x, q, 1.0), q);
+}
 
 // Householder QR (LAPACK signs; POS: a positive diagonal of R) of an N x r
 // panel whose rows [lo, lo + rows) are this CTA's a[k ld + i]; the explicit Q
@@ -334,9 +379,17 @@ __device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, 
       const T xn2 = s.dots[k], alpha = row[k];
       T beta = alpha, tau = T(0), scal = T(0);
       if (xn2 > T(0)) {
-        beta = -copysign(sqrt(fma(alpha, alpha, xn2)), alpha);
-        tau = (beta - alpha) / beta;
-        scal = T(1) / (alpha - beta);
+        beta = -copysign(root(fma(alpha, alpha, xn2)), alpha);
+        const T d = alpha - beta, bd = beta * d;
+        if (F64 && lead(bd) < -1.0e-30f && lead(bd) > -1.0e30f) {
+          // one reciprocal for both, 1 / (beta (alpha - beta))
+          const T q = reciprocal(bd);
+          tau = -(d * d) * q;
+          scal = q * beta;
+        } else {
+          tau = (beta - alpha) / beta;
+          scal = T(1) / d;
+        }
       }
       if (lane == 0) {
         s.coef[0] = beta;
