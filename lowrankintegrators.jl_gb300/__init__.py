@@ -447,9 +447,16 @@ class Batch:
         self.totals = tot
         dev = torch.device("cuda", torch.cuda.current_device())
         self.device = dev
-        mk = lambda k: torch.zeros(max(int(k), 4), dtype=self.dtype, device=dev)
-        self.U, self.S, self.V = mk(tot[0]), mk(tot[1]), mk(tot[2])
-        self.opA, self.opB = mk(tot[3]), mk(tot[4])
+        # the factors and coefficients share one buffer (parts on 256-byte
+        # boundaries): one allocation and one upload
+        self._sizes = [max(int(k), 4) for k in tot]
+        al = 256 // np.dtype(self.np_dtype).itemsize
+        self._starts = [0]
+        for k in self._sizes:
+            self._starts.append(self._starts[-1] + -(-k // al) * al)
+        self._flat = torch.zeros(self._starts[-1], dtype=self.dtype, device=dev)
+        self.U, self.S, self.V, self.opA, self.opB = self._split(self._flat)
+        self._stage = None
         self.offY = None
         self.has_data = op_kind == _native.LRI_OP_DATA or isinstance(alg, GreedyIntegrator)
         if self.has_data:
@@ -458,12 +465,13 @@ class Batch:
             _native.check(self.lib.lri_batch_data_layout(self.handle, self.offY.ctypes.data_as(I64P),
                                                          totY.ctypes.data_as(I64P)), "lri_batch_data_layout")
             self.totY = int(totY[0])
-            self.Ynext = mk(self.totY)
+            self.Ynext = torch.zeros(max(self.totY, 4), dtype=self.dtype, device=dev)
         self.bound = False
 
     # -- helpers -----------------------------------------------------------
     def _stream(self):
-        return C.c_void_p(self.torch.cuda.current_stream().cuda_stream)
+        t = self.torch
+        return C.c_void_p(t._C._cuda_getCurrentRawStream(t.cuda.current_device()))
 
     def close(self):
         if getattr(self, "handle", None) is not None and self.handle.value:
@@ -476,44 +484,40 @@ class Batch:
         except Exception:
             pass
 
+    def _split(self, flat):
+        return [flat[a:a + k] for a, k in zip(self._starts, self._sizes)]
+
     def pack_factors(self, factors: Sequence[SVDLikeRepresentation]):
         """Host-side packing of per-instance factors into the flat layout."""
-        hU = np.zeros(int(self.U.numel()), self.np_dtype)
-        hS = np.zeros(int(self.S.numel()), self.np_dtype)
-        hV = np.zeros(int(self.V.numel()), self.np_dtype)
+        return self._pack_into(factors, [np.zeros(k, self.np_dtype) for k in self._sizes[:3]])
+
+    def _pack_into(self, factors, parts):
+        hU, hS, hV = parts
         for i, Y in enumerate(factors):
             n, m, rc = int(self.n[i]), int(self.m[i]), int(self.rcap[i])
             r = Y.S.shape[0]
             if Y.U.shape != (n, r) or Y.V.shape != (m, r) or r > rc:
                 raise ValueError(f"instance {i}: factor shapes do not match the batch")
-            u = np.zeros((n, rc), self.np_dtype)
-            u[:, :r] = Y.U
-            hU[self.offU[i]:self.offU[i] + n * rc] = u.ravel(order="F")
-            s = np.zeros((rc, rc), self.np_dtype)
-            s[:r, :r] = Y.S
-            hS[self.offS[i]:self.offS[i] + rc * rc] = s.ravel(order="F")
-            v = np.zeros((m, rc), self.np_dtype)
-            v[:, :r] = Y.V
-            hV[self.offV[i]:self.offV[i] + m * rc] = v.ravel(order="F")
+            for h, off, rows, X in ((hU, self.offU, n, Y.U), (hS, self.offS, rc, Y.S), (hV, self.offV, m, Y.V)):
+                h[off[i]:off[i] + rows * rc].reshape((rows, rc), order="F")[:X.shape[0], :r] = X
         return hU, hS, hV
 
     def upload(self, factors: Sequence[SVDLikeRepresentation], operators=None):
-        hU, hS, hV = self.pack_factors(factors)
         t = self.torch
-        self.U.copy_(t.from_numpy(hU))
-        self.S.copy_(t.from_numpy(hS))
-        self.V.copy_(t.from_numpy(hV))
+        flat = np.zeros(self._starts[-1], self.np_dtype)
+        parts = self._split(flat)
+        self._pack_into(factors, parts[:3])
+        end = self._starts[3]  # the coefficients stay unless there are new ones
         if operators is not None and self.op_kind == _native.LRI_OP_SYLVESTER_TRIDIAG:
-            hA = np.zeros(int(self.opA.numel()), self.np_dtype)
-            hB = np.zeros(int(self.opB.numel()), self.np_dtype)
+            hA, hB = parts[3:]
             for i, op in enumerate(operators):
                 a, b = op.packed()
                 if len(a) != 3 * self.n[i] or len(b) != 3 * self.m[i]:
                     raise ValueError(f"instance {i}: operator size does not match the batch")
                 hA[self.offA[i]:self.offA[i] + len(a)] = a
                 hB[self.offB[i]:self.offB[i] + len(b)] = b
-            self.opA.copy_(t.from_numpy(hA))
-            self.opB.copy_(t.from_numpy(hB))
+            end = self._starts[5]
+        self._flat[:end].copy_(t.from_numpy(flat[:end]))
         if operators is not None and self.op_kind in (_native.LRI_OP_BURGERS_PERIODIC, _native.LRI_OP_LOCAL_FLOW):
             hB = np.zeros(int(self.opB.numel()), self.np_dtype)
             for i, op in enumerate(operators):
@@ -529,17 +533,36 @@ class Batch:
         self.bound = True
 
     def pack_data(self, snapshots: Sequence[np.ndarray]) -> np.ndarray:
-        h = np.zeros(self.totY, self.np_dtype)
+        return self._pack_data_into(snapshots, np.zeros(self.totY, self.np_dtype))
+
+    def _pack_data_into(self, snapshots, h):
         for i, Y in enumerate(snapshots):
             n, m = int(self.n[i]), int(self.m[i])
             Y = np.asarray(Y)
             if Y.shape != (n, m):
                 raise ValueError(f"instance {i}: snapshot shape {Y.shape} != {(n, m)}")
-            h[self.offY[i]:self.offY[i] + n * m] = Y.ravel(order="F")
+            h[self.offY[i]:self.offY[i] + n * m].reshape((n, m), order="F")[...] = Y
         return h
 
+    def _send_data(self, fill):
+        """fill(host array) writes a snapshot into one of two page-locked
+        buffers in turn; its copy to Ynext is queued behind the steps, so the
+        host packs the next snapshot while they run."""
+        t = self.torch
+        if t.cuda.is_current_stream_capturing():
+            raise RuntimeError("snapshots cannot be sent from the host while the stream is being captured")
+        if self._stage is None:
+            self._stage = [(t.zeros(max(self.totY, 4), dtype=self.dtype, pin_memory=True), t.cuda.Event())
+                           for _ in range(2)]
+        self._stage.reverse()
+        buf, ev = self._stage[0]
+        ev.synchronize()  # this buffer's last copy has left it
+        fill(buf.numpy())
+        self.Ynext.copy_(buf, non_blocking=True)
+        ev.record()
+
     def data_init(self, snapshots: Sequence[np.ndarray]):
-        self.Ynext.copy_(self.torch.from_numpy(self.pack_data(snapshots)))
+        self._send_data(lambda h: self._pack_data_into(snapshots, h))
         _native.check(self.lib.lri_batch_data_init(self.handle, C.c_void_p(self.Ynext.data_ptr()),
                                                    self._stream()), "lri_batch_data_init")
 
@@ -550,9 +573,11 @@ class Batch:
             if next_snapshots is None:
                 raise ValueError("data problems need the next snapshot")
             if isinstance(next_snapshots, np.ndarray) and next_snapshots.ndim == 1:
-                self.Ynext.copy_(self.torch.from_numpy(next_snapshots.astype(self.np_dtype, copy=False)))
+                if next_snapshots.size not in (1, self.Ynext.numel()):
+                    raise RuntimeError(f"{next_snapshots.size} snapshot values, the batch takes {self.Ynext.numel()}")
+                self._send_data(lambda h: np.copyto(h, next_snapshots, casting="unsafe"))
             else:
-                self.Ynext.copy_(self.torch.from_numpy(self.pack_data(next_snapshots)))
+                self._send_data(lambda h: self._pack_data_into(next_snapshots, h))
             yptr = C.c_void_p(self.Ynext.data_ptr())
         _native.check(self.lib.lri_batch_step(self.handle, float(t), float(dt), int(nsteps), yptr,
                                               self._stream()), "lri_batch_step")
@@ -600,9 +625,7 @@ class Batch:
 
     def unpack(self, hU, hS, hV, ranks) -> List[SVDLikeRepresentation]:
         """Per-instance factors from host copies of the packed buffers."""
-        hU = np.asarray(hU).astype(np.float64)
-        hS = np.asarray(hS).astype(np.float64)
-        hV = np.asarray(hV).astype(np.float64)
+        hU, hS, hV = (np.asarray(h, dtype=np.float64) for h in (hU, hS, hV))
         out = []
         for i in range(self.count):
             n, m, rc, r = int(self.n[i]), int(self.m[i]), int(self.rcap[i]), int(ranks[i])
@@ -632,8 +655,12 @@ class History:
     def host_buffers(self):
         """Page-locked host buffers (U, S, V, ranks) sized for one record."""
         t, b = self.torch, self.b
-        pin = lambda k, dt: t.empty(max(int(k), 1), dtype=dt, pin_memory=True)
-        return pin(b.U.numel(), b.dtype), pin(b.S.numel(), b.dtype), pin(b.V.numel(), b.dtype), pin(b.count, t.int32)
+        # one allocation, laid out like the device's ring slot (one transfer)
+        es = b.U.element_size()
+        k = [x.numel() for x in (b.U, b.S, b.V)]
+        flat = t.empty(sum(k) * es + max(b.count, 1) * 4, dtype=t.uint8, pin_memory=True)
+        f = flat[:sum(k) * es].view(b.dtype)
+        return f[:k[0]], f[k[0]:k[0] + k[1]], f[k[0] + k[1]:], flat[sum(k) * es:].view(t.int32)
 
     def record(self, host=None) -> int:
         """Queues a copy of the batch's current factors; returns its number.

@@ -173,6 +173,14 @@ int wide_cluster(int count, int64_t tall, int sms);
 
 // double <-> double-float conversions of n elements (dfloat storage is a
 // pair of floats, 8 bytes per element)
+// Four device-to-device copies (whole 32-bit words) in one launch.
+struct CopyParts {
+  void* dst[4];
+  const void* src[4];
+  size_t bytes[4];
+};
+cudaError_t copy_parts(const CopyParts& c, cudaStream_t stream);
+
 cudaError_t convert_f64_to_df(const double* in, void* out, int64_t n, cudaStream_t stream);
 cudaError_t convert_df_to_f64(const void* in, double* out, int64_t n, cudaStream_t stream);
 template <typename T>

@@ -66,6 +66,34 @@ static int conv_grid(int64_t n) {
   return g < 1 ? 1 : (int)g;
 }
 
+// Bound by the launch for small factors (one launch for four copies with a gap
+// after each) and by memory for large ones: the widest words that a part's
+// ends and length allow.
+template <class W>
+__device__ void copy_words(const CopyParts& c, int p) {
+  const size_t nt = (size_t)gridDim.x * blockDim.x, nw = c.bytes[p] / sizeof(W);
+  for (size_t i = (size_t)blockIdx.x * blockDim.x + threadIdx.x; i < nw; i += nt)
+    static_cast<W*>(c.dst[p])[i] = static_cast<const W*>(c.src[p])[i];
+}
+
+__global__ void __launch_bounds__(256) copy_parts_kernel(CopyParts c) {
+#pragma unroll
+  for (int p = 0; p < 4; ++p) {
+    const uintptr_t low = (uintptr_t)c.dst[p] | (uintptr_t)c.src[p] | c.bytes[p];
+    if ((low & 15) == 0) copy_words<uint4>(c, p);
+    else if ((low & 7) == 0) copy_words<uint2>(c, p);
+    else copy_words<uint32_t>(c, p);
+  }
+}
+
+cudaError_t copy_parts(const CopyParts& c, cudaStream_t stream) {
+  size_t most = 0;
+  for (size_t b : c.bytes) most = b > most ? b : most;
+  const int64_t g = conv_grid((int64_t)(most / 16 + 1));
+  copy_parts_kernel<<<(int)g, 256, 0, stream>>>(c);
+  return cudaGetLastError();
+}
+
 cudaError_t convert_f64_to_df(const double* in, void* out, int64_t n, cudaStream_t stream) {
   if (n <= 0) return cudaSuccess;
   f64_to_df_kernel<<<conv_grid(n), 256, 0, stream>>>(in, static_cast<dfloat*>(out), n);
