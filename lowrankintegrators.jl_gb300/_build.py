@@ -24,7 +24,7 @@ LIB_PATH = os.path.join(BUILD_DIR, "liblri_gb300.so")
 HEADER = os.path.join(os.path.dirname(HERE), "include", "lri.h")
 
 SOURCES = ["engine_f32.cu", "engine_f64.cu", "engine_df.cu", "engine_f32_occ2.cu", "engine_df_occ2.cu", "api.cpp",
-           "noalloc.cu", "adjoint.cu", "stream.cu", "tc_pass.cu", "core_svd.cu", "tc_kr.cu", "burgers_flow.cu",
+           "noalloc.cu", "adjoint.cu", "stream.cu", "tc_pass.cu", "core_svd.cu", "burgers_panel.cu", "burgers_flow.cu",
            "burgers_core.cu", "engine_wide.cu", "engine_sides.cu"]
 ARCH_FLAGS = ["-gencode", "arch=compute_103a,code=sm_103a"]
 COMMON_FLAGS = ["-O3", "-std=c++17", "-lineinfo", "-Xcompiler", "-fPIC", "-Xcompiler", "-fvisibility=hidden"]

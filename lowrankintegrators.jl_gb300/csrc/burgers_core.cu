@@ -85,8 +85,7 @@ __global__ void __launch_bounds__(SC_NT, 1)
   const int ka = 2 * min(a.R, (int)*a.rank), c = blockIdx.x;
   if (c >= ka) return;  // the whole CTA, before any barrier or allocation
   const int kch = (ka + 31) / 32;
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                                         ~static_cast<uintptr_t>(1023));
+  unsigned char* base = align_1024(smem_raw);
   unsigned char* zt = base;                     // 4 chunks x (hi, lo)
   unsigned char* tt = base + 8 * SC_TILE;       // SC_RING x (hi, lo)
   unsigned char* ctrl = tt + 2 * SC_RING * SC_TILE;
@@ -133,7 +132,7 @@ __global__ void __launch_bounds__(SC_NT, 1)
   };
   int loaded = 0;
   bool mma1 = false, mma2 = false;
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     for (; loaded < kch && loaded < SC_RING; ++loaded) load(loaded);
     bool ok = true;
     for (int j = 0; j < kch && ok; ++j) {
@@ -205,7 +204,7 @@ __global__ void __launch_bounds__(SC_NT, 1)
   }
   tc_fence_before();
   mbar_arrive(aready);
-  if (tid == 0 && wait(aready) && ok1) {
+  if (warp == 0 && ok1 && elect_one() && wait(aready)) {
     tc_fence_after();
     for (int j = 0; j < kch; ++j)
 #pragma unroll
@@ -264,7 +263,7 @@ __global__ void __launch_bounds__(SC_NT, 1)
       }
     }
   }
-  if (tid == 0 && *abort_flag) {  // let copies and MMAs in flight finish
+  if (warp == 0 && elect_one() && *abort_flag) {  // let copies and MMAs in flight finish
     for (int j = 0; j < loaded; ++j) wait(full(j), SC_WAIT / 4);
     if (mma1) wait(done1, SC_WAIT / 4);
     if (mma2) wait(done2, SC_WAIT / 4);
@@ -287,8 +286,7 @@ __global__ void __launch_bounds__(SC_NT, 1) __cluster_dims__(SC_WG_CL, 1, 1)
   const int ka = 2 * min(R, (int)*rank), np = ka * (ka + 1) / 2, nch = (np + 31) / 32;
   const int k0 = (int)((int64_t)blockIdx.x * nch / SC_WG_CTAS), nk = (int)((int64_t)(blockIdx.x + 1) * nch / SC_WG_CTAS) - k0;
   // the same alignment in every CTA of the cluster: dynamic shared memory starts at one offset
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                                         ~static_cast<uintptr_t>(1023));
+  unsigned char* base = align_1024(smem_raw);
   unsigned char* ctrl = base + 4 * SC_WG_CHUNKS * SC_TILE;
   const uint32_t bar0 = smem_u32(ctrl);
   auto full = [&](int j) { return bar0 + 8u * j; };  // j < SC_WG_CHUNKS
@@ -315,7 +313,7 @@ __global__ void __launch_bounds__(SC_NT, 1) __cluster_dims__(SC_WG_CL, 1, 1)
   __syncthreads();
   tc_fence_after();
   const uint32_t tmem = *tmem_slot;
-  if (tid == 0) {
+  if (warp == 0 && elect_one()) {
     const uint32_t st = smem_u32(base);
     for (int j = 0; j < nk; ++j) {
       const uint32_t s = st + (uint32_t)(4 * j) * SC_TILE;

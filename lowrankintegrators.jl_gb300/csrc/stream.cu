@@ -37,9 +37,9 @@
 #include "../../include/lri.h"
 #include "burgers_core.h"
 #include "burgers_flow.h"
+#include "burgers_panel.h"
 #include "core_svd.h"
 #include "engine.cuh"
-#include "tc_kr.h"
 #include "tc_pass.h"
 
 namespace lri {
@@ -1641,10 +1641,8 @@ struct lri_stream {
   // flow kernels for the current rank (burgers_flow.cu): 0 none (rank > 32),
   // 1 the K and L flows (rank <= 32), 2 also the S flow (rank <= 16)
   int fused = 0;
-  // FP32 Burgers engines: the Khatri-Rao products of the unfused flows
-  // (active width above 32) on the tensor cores (tc_kr.cu)
-  bool kr_ok = false, use_kr = false;
-  lri::TcKr kr;
+  bool panel_ok = false;  // FP32 Burgers engines: K and L flows at ranks above FLOW_KMAX (burgers_panel.cu)
+  lri::PanelFlow panel;
   bool core_ok = false;  // the S flow on the core (burgers_core.cu) at ranks above FLOW_KMAX / 2
   lri::SCore score;
 };
@@ -1786,11 +1784,15 @@ struct StreamOps {
                                        Tout);
     return cudaGetLastError();
   }
-  // the tensor-core Khatri-Rao products (FP32 Burgers engines, X == Y)
-  bool kr_tc() const { return std::is_same<T, float>::value && s->use_kr; }
+  // the K and L flows of ranks above FLOW_KMAX in one or a few launches
+  bool panel_flows(bool nonlin) const {
+    return std::is_same<T, float>::value && s->fused == 0 && s->panel_ok && nonlin;
+  }
+  cudaError_t panel_tensor(int k, const void* Tp) const {
+    return panel_flow_tensor(s->panel, k, (int)s->R, s->d_rank, static_cast<const float*>(Tp), (int)pairs_max(), st);
+  }
   int kz(int N, int aug) const {
     const int R = (int)s->R, ka = aug ? 2 * R : R;
-    if (kr_tc()) return tc_kr_splits(N, R, aug, std::max(1, s->sms), kZmax);
     const int tiles = ((N + KrTile<T>::BM - 1) / KrTile<T>::BM) * ((ka + 63) / 64);
     return std::max(1, std::min(kZmax, (2 * 152 + tiles - 1) / tiles));
   }
@@ -1799,12 +1801,6 @@ struct StreamOps {
   cudaError_t apply(int N, int aug, const T* X, const T* Y, const T* Tp, T* part, double scale = 1.0,
                     int accum = 0) const {
     const int R = (int)s->R, ka = aug ? 2 * R : R;
-    if constexpr (std::is_same<T, float>::value) {
-      const int k = (Tp == tp(s->tv)) ? 0 : (Tp == tp(s->tl)) ? 1 : (Tp == tp(s->th)) ? 2 : -1;
-      if (kr_tc() && X == Y && k >= 0)
-        return tc_kr_apply(&s->kr, k, N, aug, s->d_rank, X, part, kz(N, aug), scale, accum, s->d_status, ST_TIMEOUT,
-                           st);
-    }
     constexpr int BM = KrTile<T>::BM;
     static std::atomic<uint64_t> attr_same{0}, attr_diff{0};
     const int mx = (int)(2 * (2 * 64) * BM * sizeof(T));
@@ -1915,20 +1911,19 @@ struct StreamOps {
   }
 
   // TF32 split of flow tensor k for the tensor-core products
-  cudaError_t kr_split(int k, const T* Tp, int aug) const {
-    if constexpr (std::is_same<T, float>::value) return tc_kr_split(&s->kr, k, Tp, s->d_rank, aug, st);
-    return cudaSuccess;
-  }
-
-  // the whole L substep flow (Lp holds L0 and its RK panels): one launch up
-  // to rank FLOW_KMAX, else per stage the product panel, the Khatri-Rao
-  // partials and the combine (with the side stream's own panel and partials
-  // for scratch set 1)
+  // the whole L substep flow (Lp holds L0 and its RK panels): one launch, or
+  // (FP64 above rank FLOW_KMAX, or no quadratic term) per stage the product
+  // panel, the Khatri-Rao partials and the combine (with the side stream's
+  // own panel and partials for scratch set 1)
   cudaError_t l_flow(T* Lp, const double* Axx, bool nonlin) const {
     if (s->fused >= 1)
       return burgers_l_flow<T>(flow_kmax(), (int)s->m, (int)s->R, s->d_rank, Lp, static_cast<const T*>(s->nu), Axx,
                                tp(s->tl), (int)pairs_max(), nonlin ? 1 : 0, s->sc, s->bh_dt / s->sc.nsub,
                                s->d_status, st);
+    if constexpr (std::is_same<T, float>::value)
+      if (panel_flows(nonlin))
+        return panel_l_flow(s->panel, (int)s->m, (int)s->R, s->d_rank, Lp, static_cast<const T*>(s->nu), Axx, s->sc,
+                            s->bh_dt / s->sc.nsub, s->d_status, st);
     const int m = (int)s->m, R = (int)s->R, w = 2 * R;
     const int64_t nm = std::max(s->n, s->m);
     T* P2 = sid ? tp(s->pw2) : tp(s->pw) + 2 * nm * w;
@@ -1958,7 +1953,7 @@ struct StreamOps {
     const T* nu = static_cast<const T*>(s->nu);
     const double bh = s->bh, ba = s->balpha, bb = s->bbeta;
     const double ih2 = 1.0 / (bh * bh), ihx = 0.5 / bh;
-    const bool nonlin = (ba != 0.0 || bb != 0.0);
+    const bool nonlin = (ba != 0.0 || bb != 0.0), panel = panel_flows(nonlin);
     T* P0 = tp(s->pw);
     T* P1 = P0 + nm * w;
     T* P2 = P1 + nm * w;
@@ -1974,7 +1969,7 @@ struct StreamOps {
     scale_rows<T><<<g, 256, 0, st>>>(m, R, V, nu, P0);
     if ((e = gram(m, R, R, V, m, P0, m, 1.0, 0.0, Nnu, R)) != cudaSuccess) return e;
     if (nonlin && (e = tensor(m, 0, V, V, V, 1.0, 0, tp(s->tv))) != cudaSuccess) return e;
-    if (nonlin && kr_tc() && (e = kr_split(0, tp(s->tv), 0)) != cudaSuccess) return e;
+    if (panel && (e = panel_tensor(0, s->tv)) != cudaSuccess) return e;
     // operators of the L substep (U0 fixed): A_xx = U0^T Dxx U0,
     // T_L = alpha sym(KR(Dx U0, U0))^T U0 - beta KR(U0, U0)^T Dx U0
     double* Axx = blk(14);
@@ -1982,16 +1977,17 @@ struct StreamOps {
     if ((e = gram(n, R, R, U, n, P0, n, 1.0, 0.0, Axx, R)) != cudaSuccess) return e;
     if (ba != 0.0 && (e = tensor(n, 0, P1, U, U, ba, 0, tp(s->tl))) != cudaSuccess) return e;
     if (bb != 0.0 && (e = tensor(n, 0, U, U, P1, -bb, ba != 0.0, tp(s->tl))) != cudaSuccess) return e;
-    if (nonlin && kr_tc() && (e = kr_split(1, tp(s->tl), 0)) != cudaSuccess) return e;
+    if (panel && (e = panel_tensor(1, s->tl)) != cudaSuccess) return e;
     // K step: K0 = U0 S0, K' = (Dxx K) N_nu + alpha KR(Dx K, K) T'_V + beta Dx(KR(K, K) T'_V);
     // L step: L0 = V0 S0^T, L' = diag(nu) L A_xx + KR(L, L) T'_L.  The two
-    // flows are independent (both start from the old factors): with the
-    // fused stages the L flow runs on the side stream beside the K flow.
+    // flows are independent (both start from the old factors): the L flow runs
+    // on the side stream beside the K flow (one after the other above rank
+    // FLOW_KMAX in FP32, where either fills the GPU).
     T* Kp = tp(s->Kp);
     T* Lp = tp(s->Lp);
     if ((e = mul(n, R, R, U, n, blk(16), R, T(0), Kp, n)) != cudaSuccess) return e;
     if ((e = mul(m, R, R, V, m, blk(17), R, T(0), Lp, m)) != cudaSuccess) return e;
-    const bool fork = s->side != nullptr && (s->fused >= 1 || s->pw2 != nullptr);
+    const bool fork = s->side != nullptr && !panel && (s->fused >= 1 || s->pw2 != nullptr);
     cudaError_t el = cudaSuccess;
     if (fork) {
       if ((e = cudaEventRecord(s->ev_fork, st)) != cudaSuccess) return e;
@@ -2001,7 +1997,11 @@ struct StreamOps {
       if (el == cudaSuccess) el = ej;
     }
     const int zk = kz(n, 0);
-    if (s->fused >= 1)
+    if (panel) {
+      if constexpr (std::is_same<T, float>::value)
+        e = panel_k_flow(s->panel, n, R, s->d_rank, Kp, Kp + (int64_t)n * R, Nnu, ih2, ihx, ba, bb, s->sc,
+                         s->bh_dt / s->sc.nsub, s->d_status, st);
+    } else if (s->fused >= 1)
       e = burgers_k_flow<T>(flow_kmax(), n, R, s->d_rank, Kp, Kp + (int64_t)n * R, Nnu, tp(s->tv), (int)pairs_max(),
                             ih2, ihx, ba, bb, s->sc, s->bh_dt / s->sc.nsub, s->sms, s->d_status, st);
     else e = rk_panel((int64_t)n * R, Kp, [&](const T* Z, const RkStage<T>& rk) {
@@ -2042,7 +2042,6 @@ struct StreamOps {
     scale_rows<T><<<g, 256, 0, st>>>(m, w, Vh, nu, P0);
     if ((e = gram(m, w, w, Vh, m, P0, m, 1.0, 0.0, Nnuh, w)) != cudaSuccess) return e;
     if (nonlin && (e = tensor(m, 1, Vh, Vh, Vh, 1.0, 0, tp(s->th))) != cudaSuccess) return e;
-    if (nonlin && !wten && kr_tc() && (e = kr_split(2, tp(s->th), 1)) != cudaSuccess) return e;
     // S step on the augmented bases from S~0 = Mh S0 Nh^T (FP64 w x w):
     // S' = A_xx S N_nu + Uhat^T [alpha KR(Dx A, A) T'_Vhat + beta Dx(KR(A, A) T'_Vhat)], A = Uhat S
     small_msn<<<1, 1024, 0, st>>>(w, R, blk(3), blk(16), blk(4), Stmp, blk(18));
@@ -2368,9 +2367,9 @@ lri_status lri_burgers_create(lri_stream** out, int32_t dtype, int64_t n, int64_
   }
   // the S flow's tensor of Uhat
   alloc(&s->tw, s->es * PP * (s->core_ok ? 2 * R : std::min<int64_t>(2 * R, lri::FLOW_KMAX)));
-  if (e == cudaSuccess && dtype == LRI_F32 && lri::tc_kr_supported((int)R)) {
-    e = lri::tc_kr_init(&s->kr, (int)R);
-    s->kr_ok = s->use_kr = (e == cudaSuccess);
+  if (e == cudaSuccess && dtype == LRI_F32 && R > lri::FLOW_KMAX && R <= lri::PANEL_RMAX) {
+    e = lri::panel_flow_init(&s->panel);
+    s->panel_ok = (e == cudaSuccess);
   }
   if (e != cudaSuccess) {
     lri_stream_destroy(s);
@@ -2443,7 +2442,7 @@ lri_status lri_stream_destroy(lri_stream* s) {
   cudaFree(s->Xk);
   cudaFree(s->Xl);
   cudaFree(s->Zp);
-  lri::tc_kr_free(&s->kr);
+  lri::panel_flow_free(&s->panel);
   lri::s_core_free(&s->score);
   cudaFree(s->part);
   cudaFree(s->part2);

@@ -96,8 +96,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
                    const __grid_constant__ CUtensorMap tmXh, const __grid_constant__ CUtensorMap tmXl,
                    const TcArgs a) {
   extern __shared__ unsigned char smem_raw[];
-  unsigned char* base = reinterpret_cast<unsigned char*>((reinterpret_cast<uintptr_t>(smem_raw) + 1023) &
-                                                         ~static_cast<uintptr_t>(1023));
+  unsigned char* base = align_1024(smem_raw);
   const int NS = a.stages;
   const uint32_t xbytes = TC_BK * 4 * a.NB;  // one split-factor tile: NB rows of 128 bytes
   const uint32_t stage_bytes = 2 * TC_TILE_BYTES + 2 * xbytes;
