@@ -13,7 +13,11 @@
 // wb disjoint pairs; the pairs inside a block in the sweep's first round),
 // then every block moves to the CTA that holds it in the next round, through
 // distributed shared memory.  The rounds place the blocks by the circle
-// method, so every two blocks meet once per sweep.  Products of the whole
+// method, so every two blocks meet once per sweep.  A group of lanes keeps its
+// column of the first block in registers through a round's sub-rounds, with
+// the rows unrolled to the width in use (wa = 128: an FP32 sweep 112 -> 90 us,
+// a double-float one 265 -> 240 us, the whole SVD of a rank-64 stream step
+// 1.55 -> 1.30 ms).  Products of the whole
 // matrices (Newton-Schulz, the basis changes) are split by output columns
 // over the cluster and go through L2.
 //
@@ -31,6 +35,7 @@
 #include <algorithm>
 #include <atomic>
 #include <cstdint>
+#include <type_traits>
 
 #include "core_svd.h"
 #include "engine.cuh"
@@ -142,37 +147,46 @@ __device__ __forceinline__ bool rot_params(dfloat al, dfloat be, dfloat ga, dflo
   return true;
 }
 
-// One Jacobi rotation of columns (ap, aq) with right vectors (vp, vq) by a
-// group of G lanes (gl = lane in the group; the group's rows i = gl + k G of
-// the columns and of the right vectors are loaded at once and stay in
-// registers until the rotation); every lane of the
-// warp takes part in the reductions.  Same test and rotation as the one-CTA
+// A column and its right vector in the registers of a group of G lanes: lane
+// gl holds the rows i = gl + k G (zero beyond wa, and all of an invalid pair).
+template <typename T, int G, int KR>
+struct ColumnRegs {
+  T a[KR], v[KR];
+  __device__ __forceinline__ void load(const T* ap, const T* vp, bool valid, int wa, int gl) {
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+      const int i = gl + k * G;
+      const bool in = valid && i < wa;
+      a[k] = in ? ap[i] : T(0);
+      v[k] = in ? vp[i] : T(0);
+    }
+  }
+  __device__ __forceinline__ void store(T* ap, T* vp, int wa, int gl) const {
+#pragma unroll
+    for (int k = 0; k < KR; ++k) {
+      const int i = gl + k * G;
+      if (i < wa) {
+        ap[i] = a[k];
+        vp[i] = v[k];
+      }
+    }
+  }
+};
+
+// One Jacobi rotation of two columns in registers; every lane of the warp
+// takes part in the reductions.  Same test and rotation as the one-CTA
 // sweeps, with the parameters above.  A rotation sets fl and raises dm (the
 // rotation measure) in the lane's registers; the sweep reduces them once at
-// its end.
-template <typename T, int G>
-__device__ __forceinline__ void rotate_pair(T* ap, T* aq, T* vp, T* vq, bool valid, int wa, int gl, T eps, T tiny,
-                                            T reach, bool skip_noise, unsigned& fl, float& dm) {
-  constexpr int KR = (CORE_SVD_MAX_WA + G - 1) / G;
-  T x[KR], y[KR], u[KR], w[KR];  // the group's rows of the columns and of the right vectors
+// its end.  Returns whether the pair was rotated.
+template <typename T, int G, int KR>
+__device__ __forceinline__ bool rotate_pair(ColumnRegs<T, G, KR>& p, ColumnRegs<T, G, KR>& q, bool valid, T eps,
+                                            T tiny, T reach, bool skip_noise, unsigned& fl, float& dm) {
   T al = T(0), be = T(0), ga = T(0);
 #pragma unroll
   for (int k = 0; k < KR; ++k) {
-    const int i = gl + k * G;
-    if (valid && i < wa) {
-      x[k] = ap[i];
-      y[k] = aq[i];
-      u[k] = vp[i];
-      w[k] = vq[i];
-    } else {
-      x[k] = T(0);
-      y[k] = T(0);
-      u[k] = T(0);
-      w[k] = T(0);
-    }
-    al = fma_acc(x[k], x[k], al);
-    be = fma_acc(y[k], y[k], be);
-    ga = fma_acc(x[k], y[k], ga);
+    al = fma_acc(p.a[k], p.a[k], al);
+    be = fma_acc(q.a[k], q.a[k], be);
+    ga = fma_acc(p.a[k], q.a[k], ga);
   }
   al = renorm(al);
   be = renorm(be);
@@ -187,34 +201,88 @@ __device__ __forceinline__ void rotate_pair(T* ap, T* aq, T* vp, T* vq, bool val
       valid && (skip_noise ? (al > tiny && be > tiny && (al > reach || be > reach)) : (al > tiny || be > tiny));
   T cs_, sn;
   float dl;
-  if (live && rot_params(al, be, ga, eps, cs_, sn, dl)) {
+  if (!(live && rot_params(al, be, ga, eps, cs_, sn, dl))) return false;
 #pragma unroll
-    for (int k = 0; k < KR; ++k) {
-      const int i = gl + k * G;
-      if (i < wa) {
-        ap[i] = cs_ * x[k] - sn * y[k];
-        aq[i] = sn * x[k] + cs_ * y[k];
-      }
-    }
-#pragma unroll
-    for (int k = 0; k < KR; ++k) {
-      const int i = gl + k * G;
-      if (i < wa) {
-        vp[i] = cs_ * u[k] - sn * w[k];
-        vq[i] = sn * u[k] + cs_ * w[k];
-      }
-    }
-    fl = 1u;
-    dm = fmaxf(dm, dl);
+  for (int k = 0; k < KR; ++k) {
+    const T x = p.a[k], y = q.a[k], u = p.v[k], w = q.v[k];
+    p.a[k] = cs_ * x - sn * y;
+    q.a[k] = sn * x + cs_ * y;
+    p.v[k] = cs_ * u - sn * w;
+    q.v[k] = sn * u + cs_ * w;
   }
+  fl = 1u;
+  dm = fmaxf(dm, dl);
+  return true;
+}
+
+// The pairs inside each of the two blocks (circle method over wbe players).
+template <typename T, int G, int KR>
+__device__ __forceinline__ void rotate_inside(T* B0, T* B1, int b0, int b1, int wa, int wb, T eps, T tiny, T reach,
+                                              bool skip_noise, unsigned& fl, float& dm) {
+  const int gid = threadIdx.x / G, gl = threadIdx.x % G;
+  const int wbe = wb + (wb & 1), half = max(wbe / 2, 1);  // an even number of players
+  const int slot = gid / half, k = gid % half, b = slot ? b1 : b0;
+  T* Bk = slot ? B1 : B0;
+  for (int u = 0; u < wbe - 1; ++u) {
+    int x = u % (wbe - 1), y = wbe - 1;
+    if (k > 0) {
+      x = (u + k) % (wbe - 1);
+      y = (u - k + wbe - 1) % (wbe - 1);
+    }
+    if (x > y) {
+      const int tmp = x;
+      x = y;
+      y = tmp;
+    }
+    const bool valid = gid < wbe && y < wb && b * wb + y < wa;
+    const int xs = valid ? x : 0, ys = valid ? y : 0;
+    ColumnRegs<T, G, KR> p, q;
+    p.load(Bk + (size_t)xs * wa, Bk + (size_t)(wb + xs) * wa, valid, wa, gl);
+    q.load(Bk + (size_t)ys * wa, Bk + (size_t)(wb + ys) * wa, valid, wa, gl);
+    if (rotate_pair(p, q, valid, eps, tiny, reach, skip_noise, fl, dm)) {
+      p.store(Bk + (size_t)xs * wa, Bk + (size_t)(wb + xs) * wa, wa, gl);
+      q.store(Bk + (size_t)ys * wa, Bk + (size_t)(wb + ys) * wa, wa, gl);
+    }
+    __syncthreads();
+  }
+}
+
+// The pairs across the two blocks: in sub-round s column x of slot 0 meets
+// column (x + s) mod wb of slot 1.  A group keeps its column of slot 0 in
+// registers through the sub-rounds; only the other one passes through shared
+// memory.
+template <typename T, int G, int KR>
+__device__ __forceinline__ void rotate_across(T* B0, T* B1, int b0, int b1, int wa, int wb, T eps, T tiny, T reach,
+                                              bool skip_noise, unsigned& fl, float& dm) {
+  const int gid = threadIdx.x / G, gl = threadIdx.x % G;
+  const bool mine = gid < wb && b0 * wb + gid < wa;
+  T* a0 = B0 + (size_t)(mine ? gid : 0) * wa;
+  ColumnRegs<T, G, KR> c0, c1;
+  c0.load(a0, a0 + (size_t)wb * wa, mine, wa, gl);
+  bool changed = false;
+  int y = mine ? gid : 0;
+  for (int s = 0; s < wb; ++s) {
+    const bool valid = mine && b1 * wb + y < wa;
+    T* a1 = B1 + (size_t)(valid ? y : 0) * wa;
+    c1.load(a1, a1 + (size_t)wb * wa, valid, wa, gl);
+    // the lower column index first
+    const bool rot = (b0 > b1) ? rotate_pair(c1, c0, valid, eps, tiny, reach, skip_noise, fl, dm)
+                               : rotate_pair(c0, c1, valid, eps, tiny, reach, skip_noise, fl, dm);
+    if (rot) c1.store(a1, a1 + (size_t)wb * wa, wa, gl);
+    changed |= rot;
+    if (++y == wb) y = 0;
+    __syncthreads();
+  }
+  if (changed) c0.store(a0, a0 + (size_t)wb * wa, wa, gl);
+  __syncthreads();
 }
 
 // Jacobi sweeps over the cluster.  On entry and on return the blocks sit in
 // buffer `cur` in their round-0 places.  Returns whether the sweeps
 // converged (no rotation, or the largest rotation measure of a sweep at most
 // conv_delta; sqrt(eps) when negative).  The same on every CTA.
-template <typename T>
-__device__ bool cluster_jacobi(cg::cluster_group& cl, ClusterState& cs, T* base, int& cur, int wa, int wb,
+template <typename T, int G, int KR>
+__device__ __forceinline__ bool cluster_jacobi(cg::cluster_group& cl, ClusterState& cs, T* base, int& cur, int wa, int wb,
                                int max_sweeps, bool skip_noise, double conv_delta, double tiny_abs) {
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int cr = (int)cl.block_rank();
@@ -252,15 +320,6 @@ __device__ bool cluster_jacobi(cg::cluster_group& cl, ClusterState& cs, T* base,
   const T tiny = T(Prec<T>::eps * Prec<T>::eps * fro2);
   const T reach = T(tiny_abs);
   const float delta_stop = (float)((conv_delta >= 0.0) ? conv_delta : sqrt(Prec<T>::eps));
-  const int wbe = wb + (wb & 1);  // even number of players inside a block
-  const int G = (wbe <= CS_NT / 32) ? 32 : 16;
-  const int gid = tid / G, gl = tid % G;
-  auto rotate = [&](T* ap, T* aq, T* vp, T* vq, bool valid, unsigned& fl, float& dm) {
-    if (G == 32)
-      rotate_pair<T, 32>(ap, aq, vp, vq, valid, wa, gl, eps, tiny, reach, skip_noise, fl, dm);
-    else
-      rotate_pair<T, 16>(ap, aq, vp, vq, valid, wa, gl, eps, tiny, reach, skip_noise, fl, dm);
-  };
   const size_t bsz16 = bstride * sizeof(T) / 16;
   bool converged = false;
   for (int sweep = 0; sweep < max_sweeps && !converged; ++sweep) {
@@ -275,53 +334,8 @@ __device__ bool cluster_jacobi(cg::cluster_group& cl, ClusterState& cs, T* base,
       const int b0 = blk_first(cr, t), b1 = blk_second(cr, t);
       T* B0 = block(cur, 0);
       T* B1 = block(cur, 1);
-      if (t == 0) {
-        // pairs inside each block (circle method over wbe players)
-        const int half = wbe / 2;
-        for (int u = 0; u < wbe - 1; ++u) {
-          const int slot = gid / max(half, 1), k = gid % max(half, 1);
-          int x, y;
-          if (k == 0) {
-            x = u % (wbe - 1);
-            y = wbe - 1;
-          } else {
-            x = (u + k) % (wbe - 1);
-            y = (u - k + wbe - 1) % (wbe - 1);
-          }
-          if (x > y) {
-            const int tmp = x;
-            x = y;
-            y = tmp;
-          }
-          const int b = slot ? b1 : b0;
-          const bool valid = gid < wbe && y < wb && b * wb + y < wa;
-          T* Bk = slot ? B1 : B0;
-          const int xs = valid ? x : 0, ys = valid ? y : 0;
-          rotate(Bk + (size_t)xs * wa, Bk + (size_t)ys * wa, Bk + (size_t)(wb + xs) * wa, Bk + (size_t)(wb + ys) * wa,
-                 valid, fl, dm);
-          __syncthreads();
-        }
-      }
-      // pairs across the two blocks: column x of slot 0 with (x + s) mod wb of slot 1
-      for (int s = 0; s < wb; ++s) {
-        const int x = gid, y = (gid + s) % wb;
-        const bool valid = gid < wb && b0 * wb + x < wa && b1 * wb + y < wa;
-        const int xs = valid ? x : 0, ys = valid ? y : 0;
-        T* ap = B0 + (size_t)xs * wa;
-        T* vp = B0 + (size_t)(wb + xs) * wa;
-        T* aq = B1 + (size_t)ys * wa;
-        T* vq = B1 + (size_t)(wb + ys) * wa;
-        if (b0 * wb + x > b1 * wb + y) {  // the lower column index first
-          T* t1 = ap;
-          ap = aq;
-          aq = t1;
-          t1 = vp;
-          vp = vq;
-          vq = t1;
-        }
-        rotate(ap, aq, vp, vq, valid, fl, dm);
-        __syncthreads();
-      }
+      if (t == 0) rotate_inside<T, G, KR>(B0, B1, b0, b1, wa, wb, eps, tiny, reach, skip_noise, fl, dm);
+      rotate_across<T, G, KR>(B0, B1, b0, b1, wa, wb, eps, tiny, reach, skip_noise, fl, dm);
       // every block to its place in the next round (buffer cur ^ 1)
       const int tn = (t + 1) % (CS_NBLK - 1);
       for (int slot = 0; slot < 2; ++slot) {
@@ -361,6 +375,24 @@ __device__ bool cluster_jacobi(cg::cluster_group& cl, ClusterState& cs, T* base,
   return converged;
 }
 
+// 32 lanes per pair while a block has at most 8 columns, then 16; a lane's rows
+// (of 192 at most) unrolled to the next multiple of 32 or 16 that is in use.
+template <typename T>
+__device__ __noinline__ bool jacobi(cg::cluster_group& cl, ClusterState& cs, int& cur, int wa, int wb, int max_sweeps,
+                                    bool skip_noise, double conv_delta, double tiny_abs) {
+  extern __shared__ __align__(128) unsigned char smem[];
+  T* base = reinterpret_cast<T*>(smem);
+  auto run = [&](auto g, auto kr) {
+    return cluster_jacobi<T, decltype(g)::value, decltype(kr)::value>(cl, cs, base, cur, wa, wb, max_sweeps,
+                                                                      skip_noise, conv_delta, tiny_abs);
+  };
+  using std::integral_constant;
+  if (wb + (wb & 1) > CS_NT / 32)
+    return run(integral_constant<int, 16>{}, integral_constant<int, (CORE_SVD_MAX_WA + 15) / 16>{});
+  if (wa <= 64) return run(integral_constant<int, 32>{}, integral_constant<int, 2>{});
+  return run(integral_constant<int, 32>{}, integral_constant<int, CS_NBLK * (CS_NT / 32) / 32>{});
+}
+
 // out[:, j] (j0 <= j < j1) = op(A) B[:, j] for wa x wa double-float matrices
 // (ld wa) in global memory; A from AD (double-float) or A64 (FP64).
 // ns: out = 1.5 [i == j] - 0.5 (A^T B) (a Newton-Schulz factor).  Tiles of
@@ -371,6 +403,7 @@ __device__ void prod_cols(int wa, const dfloat* AD, const double* A64, bool tran
   const int tid = threadIdx.x;
   const int nJ = j1 - j0;
   if (nJ <= 0) return;
+  constexpr int PC = 2;
   dfloat* Bs = reinterpret_cast<dfloat*>(smem);  // nJ x wa
   dfloat* As = Bs + (size_t)nJ * wa;             // [k][33]: rows i0..i0+31 of op(A)
   __syncthreads();
@@ -393,16 +426,30 @@ __device__ void prod_cols(int wa, const dfloat* AD, const double* A64, bool tran
       As[k * 33 + ii] = (i < wa) ? (transA ? A_at(k, i) : A_at(i, k)) : dfloat(0.0f, 0.0f);
     }
     __syncthreads();
-    for (int o = tid; o < 32 * nJ; o += CS_NT) {
-      const int ii = o & 31, jj = o >> 5, i = i0 + ii;
-      dfloat acc(0.0f, 0.0f);
-      const dfloat* bj = Bs + (size_t)jj * wa;
-      for (int k = 0; k < wa; ++k) acc = fma_acc(As[k * 33 + ii], bj[k], acc);
-      acc = renorm(acc);
-      if (i < wa) {
-        const int j = j0 + jj;
-        if (ns) acc = ((i == j) ? dfloat(1.5f, 0.0f) : dfloat(0.0f, 0.0f)) - dfloat(0.5f, 0.0f) * acc;
-        out[i + (size_t)j * wa] = acc;
+    // up to PC columns of a row per thread: one chain of additions each
+    const int ii = tid & 31, i = i0 + ii;
+    for (int jb = tid >> 5; jb < nJ; jb += PC * CS_NT / 32) {
+      dfloat acc[PC];
+      const dfloat* bj[PC];
+#pragma unroll
+      for (int c = 0; c < PC; ++c) {
+        acc[c] = dfloat(0.0f, 0.0f);
+        bj[c] = Bs + (size_t)min(jb + c * CS_NT / 32, nJ - 1) * wa;
+      }
+#pragma unroll 4
+      for (int k = 0; k < wa; ++k) {
+        const dfloat x = As[k * 33 + ii];
+#pragma unroll
+        for (int c = 0; c < PC; ++c) acc[c] = fma_acc(x, bj[c][k], acc[c]);
+      }
+#pragma unroll
+      for (int c = 0; c < PC; ++c) {
+        const int jj = jb + c * CS_NT / 32, j = j0 + jj;
+        dfloat v = renorm(acc[c]);
+        if (i < wa && jj < nJ) {
+          if (ns) v = ((i == j) ? dfloat(1.5f, 0.0f) : dfloat(0.0f, 0.0f)) - dfloat(0.5f, 0.0f) * v;
+          out[i + (size_t)j * wa] = v;
+        }
       }
     }
   }
@@ -498,7 +545,7 @@ __global__ void __cluster_dims__(CS_C, 1, 1) __launch_bounds__(CS_NT, 1) core_sv
     __syncthreads();
     // a preconditioner: near FP32's resolution limit the sweeps need not
     // converge, so at most 12
-    cluster_jacobi<float>(cl, cs, base, cur, wa, wb, 12, false, -1.0, 0.0);
+    jacobi<float>(cl, cs, cur, wa, wb, 12, false, -1.0, 0.0);
     for (int slot = 0; slot < 2; ++slot) {
       const int b = slot ? blk_second(cr, 0) : blk_first(cr, 0);
       const float* V = base + (size_t)(cur * 2 + slot) * bstride + (size_t)wb * wa;
@@ -541,7 +588,7 @@ __global__ void __cluster_dims__(CS_C, 1, 1) __launch_bounds__(CS_NT, 1) core_sv
     }
   }
   __syncthreads();
-  bool ok = cluster_jacobi<dfloat>(cl, cs, base, cur, wa, wb, 40, true, 1e-4, tiny_abs);
+  bool ok = jacobi<dfloat>(cl, cs, cur, wa, wb, 40, true, 1e-4, tiny_abs);
   broadcast_sigma(cl, base, cur, wa, wb, sig);
   sort_sigma(wa, sig, perm);
   if (tid == 0) {
@@ -553,7 +600,7 @@ __global__ void __cluster_dims__(CS_C, 1, 1) __launch_bounds__(CS_NT, 1) core_sv
   double tiny_left = tiny_abs;
   if (redo) {
     // continue the sweeps without the truncation-level skip
-    ok = cluster_jacobi<dfloat>(cl, cs, base, cur, wa, wb, 40, true, 1e-4, 0.0);
+    ok = jacobi<dfloat>(cl, cs, cur, wa, wb, 40, true, 1e-4, 0.0);
     broadcast_sigma(cl, base, cur, wa, wb, sig);
     sort_sigma(wa, sig, perm);
     if (tid == 0) r_new = decide_rank(wa, R, a.rmin, a.tol, sig, perm);
