@@ -19,9 +19,11 @@
 //                  distributed shared memory;
 //   s_core_update  sums the 16 cluster partials, applies the RK stage to the
 //                  FP64 core and writes the split of the next stage input.
-// At rank 64 the three take 12.3 + 14.4 + 4.6 us per stage against 205 us of
-// the panel form (Khatri-Rao product 131, Uhat^T P2 23, five small products
-// and combines 51); a step at n = 4096, m = 16384 went from 88.8 to 44.6 ms.
+// At rank 64 the three took 12.0 + 14.1 + 4.6 us per stage (the panel form
+// 205 us: Khatri-Rao product 131, Uhat^T P2 23, five small products and
+// combines 51); with each kernel's prologue and constant operands loaded while
+// the one before it drains (programmatic dependent launch) a stage takes 25
+// us.
 // What bounds them now: operand staging (256 KB per CTA through L2) and the
 // serial chain of two 128^3 products; the MMAs themselves take about 3.5 us.
 // Every mbarrier wait is bounded (ST_TIMEOUT); a CTA that gives up waits for
@@ -84,6 +86,7 @@ __global__ void __launch_bounds__(SC_NT, 1)
   extern __shared__ unsigned char smem_raw[];
   const int ka = 2 * min(a.R, (int)*a.rank), c = blockIdx.x;
   if (c >= ka) return;  // the whole CTA, before any barrier or allocation
+  pdl_launch();
   const int kch = (ka + 31) / 32;
   unsigned char* base = align_1024(smem_raw);
   unsigned char* zt = base;                     // 4 chunks x (hi, lo)
@@ -123,17 +126,21 @@ __global__ void __launch_bounds__(SC_NT, 1)
   const uint32_t idesc = idesc_tf32(SC_W, 32 * kch);
   auto zaddr = [&](int j, int lo) { return smem_u32(zt) + (uint32_t)(2 * j + lo) * SC_TILE; };
   auto taddr = [&](int j, int lo) { return smem_u32(tt) + (uint32_t)(2 * (j % SC_RING) + lo) * SC_TILE; };
-  auto load = [&](int j) {
+  auto load_t = [&](int j) {
     mbar_expect_tx(full(j), 4 * SC_TILE);
-    tma_load_2d(zaddr(j, 0), &tmZh, 32 * j, 0, full(j));
     tma_load_2d(taddr(j, 0), &tmTh, 32 * j, c * SC_W, full(j));
-    tma_load_2d(zaddr(j, 1), &tmZl, 32 * j, 0, full(j));
     tma_load_2d(taddr(j, 1), &tmTl, 32 * j, c * SC_W, full(j));
+  };
+  auto load_z = [&](int j) {
+    tma_load_2d(zaddr(j, 0), &tmZh, 32 * j, 0, full(j));
+    tma_load_2d(zaddr(j, 1), &tmZl, 32 * j, 0, full(j));
   };
   int loaded = 0;
   bool mma1 = false, mma2 = false;
   if (warp == 0 && elect_one()) {
-    for (; loaded < kch && loaded < SC_RING; ++loaded) load(loaded);
+    for (; loaded < kch && loaded < SC_RING; ++loaded) load_t(loaded);
+    pdl_wait();  // Z is the previous kernel's; nothing is written before it has been read
+    for (int j = 0; j < loaded; ++j) load_z(j);
     bool ok = true;
     for (int j = 0; j < kch && ok; ++j) {
       if (!(ok = wait(full(j)))) break;
@@ -150,7 +157,8 @@ __global__ void __launch_bounds__(SC_NT, 1)
       if (j == 0 && kch > SC_RING) umma_commit(empty0);
       if (j == 1 && kch > SC_RING) {  // the fourth chunk takes the first one's ring slot
         if (!(ok = wait(empty0))) break;
-        load(loaded++);
+        load_t(loaded);
+        load_z(loaded++);
       }
     }
     umma_commit(done1);
@@ -283,6 +291,7 @@ __global__ void __launch_bounds__(SC_NT, 1) __cluster_dims__(SC_WG_CL, 1, 1)
               const int32_t* __restrict__ rank, float* __restrict__ part, uint32_t* status) {
   extern __shared__ unsigned char smem_raw[];
   cg::cluster_group cl = cg::this_cluster();
+  pdl_launch();
   const int ka = 2 * min(R, (int)*rank), np = ka * (ka + 1) / 2, nch = (np + 31) / 32;
   const int k0 = (int)((int64_t)blockIdx.x * nch / SC_WG_CTAS), nk = (int)((int64_t)(blockIdx.x + 1) * nch / SC_WG_CTAS) - k0;
   // the same alignment in every CTA of the cluster: dynamic shared memory starts at one offset
@@ -320,6 +329,10 @@ __global__ void __launch_bounds__(SC_NT, 1) __cluster_dims__(SC_WG_CL, 1, 1)
       mbar_expect_tx(full(j), 4 * SC_TILE);
       tma_load_2d(s, &tmWh, 32 * (k0 + j), 0, full(j));
       tma_load_2d(s + SC_TILE, &tmWl, 32 * (k0 + j), 0, full(j));
+    }
+    pdl_wait();  // G is the previous kernel's
+    for (int j = 0; j < nk; ++j) {
+      const uint32_t s = st + (uint32_t)(4 * j) * SC_TILE;
       tma_load_2d(s + 2 * SC_TILE, &tmGh, 32 * (k0 + j), 0, full(j));
       tma_load_2d(s + 3 * SC_TILE, &tmGl, 32 * (k0 + j), 0, full(j));
     }
@@ -392,6 +405,8 @@ __global__ void __launch_bounds__(256) s_core_update(int R, const int32_t* __res
                                                      double* __restrict__ y, double* __restrict__ acc, double b,
                                                      double ha, double h, int first, int last,
                                                      float* __restrict__ zh, float* __restrict__ zl) {
+  pdl_launch();
+  pdl_wait();
   const int r = min(R, (int)*rank), ka = 2 * r, w = 2 * R;
   const int e = blockIdx.x * 256 + threadIdx.x, d = e & (SC_W - 1), c = e / SC_W;
   if (d >= ka || c >= ka) return;
@@ -497,13 +512,37 @@ cudaError_t s_core_flow(const SCore& s, const int32_t* rank, double* Z, double* 
   a.gh = s.gh;
   a.gl = s.gl;
   a.status = status;
+  // From the second kernel on each starts its prologue and its loads of the
+  // step's constants while the one before it drains (the first one's
+  // constants are the setup's).
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  auto config = [&](int grid, size_t smem, bool dependent) {
+    cudaLaunchConfig_t c{};
+    c.gridDim = dim3((unsigned)grid);
+    c.blockDim = dim3(256);
+    c.dynamicSmemBytes = smem;
+    c.stream = st;
+    c.attrs = &attr;
+    c.numAttrs = dependent ? 1 : 0;
+    return c;
+  };
+  static_assert(SC_NT == 256, "block size");
+  bool first = true;
   for (int sub = 0; sub < sc.nsub; ++sub)
     for (int k = 0; k < sc.nstages; ++k) {
       const bool last = k + 1 == sc.nstages;
-      s_core_g<<<2 * s.R, SC_NT, SC_G_SMEM, st>>>(tm(0), tm(1), tm(2), tm(3), a);
-      s_core_wg<<<SC_WG_CTAS, SC_NT, SC_WG_SMEM, st>>>(tm(4), tm(5), tm(6), tm(7), s.R, rank, s.part, status);
-      s_core_update<<<SC_W * SC_W / 256, 256, 0, st>>>(s.R, rank, s.lin, s.part, Z, acc, sc.b[k],
-                                                       last ? 0.0 : h * sc.a[k + 1], h, k == 0, last, s.zh, s.zl);
+      cudaLaunchConfig_t c = config(2 * s.R, SC_G_SMEM, !first);
+      if ((e = cudaLaunchKernelEx(&c, s_core_g, tm(0), tm(1), tm(2), tm(3), a)) != cudaSuccess) return e;
+      c = config(SC_WG_CTAS, SC_WG_SMEM, true);
+      e = cudaLaunchKernelEx(&c, s_core_wg, tm(4), tm(5), tm(6), tm(7), s.R, rank, s.part, status);
+      if (e != cudaSuccess) return e;
+      c = config(SC_W * SC_W / 256, 0, true);
+      e = cudaLaunchKernelEx(&c, s_core_update, s.R, rank, (const float*)s.lin, (const float*)s.part, Z, acc, sc.b[k],
+                             last ? 0.0 : h * sc.a[k + 1], h, (int)(k == 0), (int)last, s.zh, s.zl);
+      if (e != cudaSuccess) return e;
+      first = false;
     }
   return cudaGetLastError();
 }

@@ -15,6 +15,13 @@ namespace {
 
 __device__ __forceinline__ uint32_t smem_u32(const void* p) { return (uint32_t)__cvta_generic_to_shared(p); }
 
+// Programmatic dependent launch: `pdl_wait` returns when the grids before this
+// one in the stream have finished and their writes are visible (at once
+// without the launch attribute); `pdl_launch` lets the next one start its
+// own prologue.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_launch() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
 // Start of the 1024-byte aligned part of dynamic shared memory (by an offset:
 // a pointer rounded as an integer is no longer known to be shared memory, and
 // every access through it becomes a generic one).
