@@ -121,8 +121,8 @@ __device__ __forceinline__ float rot_tan(float d, float ga) {
 
 __device__ __forceinline__ bool rot_params(float al, float be, float ga, float eps, float& cs, float& sn, float& dl) {
   dl = fabsf(ga) * rsqrtf(al) * rsqrtf(be);
+  const float t = rot_tan(be - al, ga);  // beside the measure's roots (unused without a rotation)
   if (!(dl > eps) || ga == 0.0f) return false;
-  const float t = rot_tan(be - al, ga);
   cs = rsqrtf(fmaf(t, t, 1.0f));
   sn = cs * t;
   return true;
@@ -140,8 +140,8 @@ __device__ __forceinline__ dfloat rsqrt_1pt2(float t) {
 __device__ __forceinline__ bool rot_params(dfloat al, dfloat be, dfloat ga, dfloat eps, dfloat& cs, dfloat& sn,
                                            float& dl) {
   dl = fabsf(ga.hi) * rsqrtf(al.hi) * rsqrtf(be.hi);
-  if (!(dl > eps.hi) || ga.hi == 0.0f) return false;
   const float t = rot_tan((be - al).hi, ga.hi);  // be - al in double-float: no cancellation
+  if (!(dl > eps.hi) || ga.hi == 0.0f) return false;
   cs = rsqrt_1pt2(t);
   sn = cs * dfloat(t);
   return true;
@@ -544,8 +544,9 @@ __global__ void __cluster_dims__(CS_C, 1, 1) __launch_bounds__(CS_NT, 1) core_sv
     }
     __syncthreads();
     // a preconditioner: near FP32's resolution limit the sweeps need not
-    // converge, so at most 12
-    jacobi<float>(cl, cs, cur, wa, wb, 12, false, -1.0, 0.0);
+    // converge, so at most 12, and after one whose largest rotation measure
+    // is small the next would only confirm it
+    jacobi<float>(cl, cs, cur, wa, wb, 12, false, 0.02, 0.0);
     for (int slot = 0; slot < 2; ++slot) {
       const int b = slot ? blk_second(cr, 0) : blk_first(cr, 0);
       const float* V = base + (size_t)(cur * 2 + slot) * bstride + (size_t)wb * wa;
