@@ -153,7 +153,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
 
   if (warp == 4) {
     // ---------------- TMA producer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       int last_par[TC_MAX_STAGES];
       for (int s = 0; s < TC_MAX_STAGES; ++s) last_par[s] = -1;
       bool ok = true;
@@ -183,7 +183,7 @@ __global__ void __launch_bounds__(TC_THREADS, 1)
     }
   } else if (warp == 5) {
     // ---------------- MMA issuer ----------------
-    if (lane == 0) {
+    if (elect_one()) {
       const uint32_t idesc = idesc_tf32(TC_BM, N);
       for (int it = 0; it < nk; ++it) {
         const int s = it % NS;
