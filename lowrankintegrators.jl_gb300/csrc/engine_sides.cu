@@ -555,20 +555,37 @@ bool group_sides(std::vector<SideItem>& v, SidesPlan* p, std::vector<int32_t>* i
 // Double-float sides: the smallest cluster whose panels leave room for two CTAs
 // on an SM (they hide each other's barriers); where the batch leaves SMs idle,
 // larger clusters down to 32 rows per CTA.
+//
+// The step kernel (one CTA per instance, three per SM, panels through L2) is
+// the better one for batches that fill the GPU with tall panels of high rank:
+// a side that needs a cluster pays for its barriers and for the QR's r x r work
+// on every CTA.  Costs in units of the work N r (r + 8) at the step kernel's
+// full rate, at which one CTA alone runs 1/230: the step kernel takes its
+// total, but at least its longest instance; sides take 0.75 of a panel on one
+// CTA or two and 1.35 on more.  Members of n, m to 1024, step kernel
+// against sides per step: r 23 to 32, 350: 4.5, 3.8 ms; 700: 6.3, 7.4 ms; 1400:
+// 10.8, 14.4 ms; r 4 to 32, 1000: 5.1, 5.4 ms; n, m to 512, r 4 to 24, 1000: 2.3,
+// 1.8 ms; n = m = 256, r 23 to 32, 366: 2.6, 1.9 ms.
 bool sides_plan(SidesPlan* p, int count, const int64_t* n, const int64_t* m, const int64_t* r, int sms,
                 std::vector<int32_t>* items) {
   std::vector<SideItem> v;
+  double total = 0.0, longest = 0.0, by_sides = 0.0;
   for (int i = 0; i < count; ++i) {
     if (r[i] > wide::WR_MAX) return false;
+    const double rr = (double)r[i] * ((double)r[i] + 8.0);
     for (int s = 0; s < 2; ++s) {
       const int N = (int)(s ? m[i] : n[i]), ri = (int)r[i];
       int C = 1;
       while (C < wide::WC_MAX && side_bytes(N, ri, C) > kHalfSmem) C *= 2;
+      by_sides += N * rr * (C <= 2 ? 0.75 : 1.35);
       while (C < wide::WC_MAX && 4 * (int64_t)C * count <= sms && N >= 64 * C) C *= 2;
       if (side_bytes(N, ri, C) > kWideSmemMax) return false;
-      v.push_back({(int32_t)(2 * i + s), C, side_bytes(N, ri, C), (double)N * ri * (ri + 8.0) / C});
+      v.push_back({(int32_t)(2 * i + s), C, side_bytes(N, ri, C), N * rr / C});
     }
+    total += (double)(n[i] + m[i]) * rr;
+    longest = std::max(longest, (double)(n[i] + m[i]) * rr);
   }
+  if (by_sides > std::max(total, 230.0 * longest)) return false;
   return group_sides(v, p, items);
 }
 

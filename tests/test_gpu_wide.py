@@ -138,3 +138,28 @@ def test_df_sides_match_oracle(lri, oracle, shapes, grade):
         assert oracle.rel_fro_err(y.full(), yo.full()) <= 1e-11
         for X in (y.U, y.V):
             assert np.abs(X.T @ X - np.eye(X.shape[1])).max() <= 1e-11
+
+
+# the step kernel keeps batches that fill the GPU with tall panels of high rank;
+# both routes take the same factors (one step of the first instances agrees)
+@pytest.mark.parametrize("count,n,r,sides", [(3, 768, 28, True), (480, 768, 28, False), (480, 128, 12, True)])
+def test_df_route_by_cost(lri, count, n, r, sides):
+    g = np.random.default_rng(3)
+    U, V = (np.linalg.qr(g.standard_normal((n, r)))[0] for _ in range(2))
+    Y = lri.SVDLikeRepresentation(U, np.diag(2.0 ** -np.arange(1, r + 1)), V)
+    T = (g.uniform(0.5, 1, n), -2 - g.uniform(0, 1, n), g.uniform(0.5, 1, n))
+    op = lri.SylvesterTridiagOperator(T, T)
+    alg = lri.UnconventionalAlgorithm(lri.RK4(1))
+    kind = lri._native.LRI_OP_SYLVESTER_TRIDIAG
+    one = lri.Batch([n], [n], [r], alg, kind, "df")
+    b = lri.Batch([n] * count, [n] * count, [r] * count, alg, kind, "df")
+    assert (b.launches_per_step() > 4) == sides and one.launches_per_step() > 4
+    for x, k in ((one, 1), (b, count)):
+        x.upload([Y] * k, [op] * k)
+        x.step(0.0, 1e-2)
+        x.check_status()
+    ref, got = one.download()[0].full(), b.download()[count - 1].full()
+    one.close()
+    b.close()
+    # double-float: 48 bits through some hundred dependent operations per entry
+    assert np.linalg.norm(got - ref) <= 1e-11 * np.linalg.norm(ref)
