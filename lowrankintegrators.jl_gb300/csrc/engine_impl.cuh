@@ -79,15 +79,16 @@ __device__ __noinline__ void projections(const Inst<T>& I, const T* X, int N, in
 // (which the QR does not otherwise use), else in place in global memory.
 // FP64 panels, and panels whose column signs do not matter (any_signs: the
 // rank-adaptive step's augmented bases, rotated by the core's SVD), take the
-// one-reduction-per-column form (wide::qr) where its scratch fits; FP32 bases
-// handed to the caller keep hh_factor's rounding, which decides the sign of a
-// column whose pivot is at rounding level.
+// one-reduction-per-column form (wide::qr) where its scratch fits and its
+// 32-bit offsets reach; FP32 bases handed to the caller keep hh_factor's
+// rounding, which decides the sign of a column whose pivot is at rounding
+// level.
 template <typename T>
 __device__ __noinline__ void qr_panel(T* Kp, int N, int W, T* Qdst, T* R, int ldr, Smem<T>& sm,
                                       bool any_signs = false) {
   if (std::is_same<T, double>::value || (any_signs && !R)) {
     const int scr = ((int)wide::QrSmem<T>::elems(1, W) + 3) & ~3;
-    if (scr <= Stage<T>::ELEMS) {
+    if (scr <= Stage<T>::ELEMS && (int64_t)N * W <= (int64_t)1 << 30) {
       const wide::Team one{cooperative_groups::this_cluster(), 0, 1};
       const wide::QrSmem<T> qs = wide::QrSmem<T>::carve(sm.stage, 1, W);
       const int ld = N | 1;  // odd: threads along the columns hit distinct banks

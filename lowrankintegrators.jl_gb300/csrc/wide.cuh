@@ -21,6 +21,7 @@
 
 #include "engine.cuh"
 #include "engine_api.h"
+#include "fast_div.h"
 
 namespace lri {
 namespace wide {
@@ -77,16 +78,6 @@ struct Team {
     if (C > 1) __threadfence();
     barrier();
   }
-};
-
-// Quotient and remainder by a fixed divisor for 0 <= e < 2^21 (the rounding of
-// (e + 1/2) / d stays below 1 / (2 d)): a few instructions where the integer
-// division takes tens.
-struct FastDiv {
-  int d;
-  float inv;
-  __device__ explicit FastDiv(int d_) : d(d_), inv(1.0f / (float)max(d_, 1)) {}
-  __device__ int div(int e) const { return (int)(((float)e + 0.5f) * inv); }
 };
 
 // Lanes per output for nout outputs on WT threads: the largest power of two <=
