@@ -217,7 +217,7 @@ struct QrSmem {
   T* dots;  // r
   T* v1;    // r x (r + 1): pivot rows of V, v1[k LT + j], j < k
   T* tri;   // r x (r + 1): T of the compact WY form, T(i, k) at i LT + k
-  T* coef;  // beta, tau, scal
+  T* coef;  // beta, tau, scal, flag
   T* sgn;   // r: column scales, then signs (fast forms)
   __host__ __device__ static constexpr size_t elems(int C, int r) {
     return (size_t)r * (2 * C + 2 + WT / 32 + 1) + 2 * (size_t)r * (r + 1) + 4 + r;
@@ -238,6 +238,7 @@ struct QrSmem {
 
 __device__ __forceinline__ float two_to(float, int e) { return ldexpf(1.0f, e); }
 __device__ __forceinline__ dfloat two_to(dfloat, int e) { return dfloat(ldexpf(1.0f, e), 0.0f); }
+__device__ __forceinline__ double two_to(double, int e) { return __hiloint2double((e + 1023) << 20, 0); }
 __device__ __forceinline__ float lead(float x) { return x; }
 __device__ __forceinline__ float lead(dfloat x) { return x.hi; }
 __device__ __forceinline__ float lead(double x) { return (float)x; }
@@ -264,57 +265,96 @@ __device__ __forceinline__ double reciprocal(double x) {  // 1e-30 < |x| < 1e30
   return fma(q, fma(-x, q, 1.0), q);
 }
 
-// Householder QR (LAPACK signs; POS: a positive diagonal of R) of an N x r
-// panel whose rows [lo, lo + rows) are this CTA's a[k ld + i]; the explicit Q
-// goes to qout (ld ldq) and, when R is given, the factor to R (global, ld
-// ldr, zeros below; not with the scaled columns of the FP32-based types).  One
-// cluster barrier per column: a single pass forms x^T A for every column (the
-// trailing ones, and the earlier reflectors for the compact WY form), its
-// partials and the pivot row are pushed to every CTA, and every CTA derives
-// the reflector from the same sums.  Q = [I; 0] - V (T V1^T), T from those
-// products, replaces the backward accumulation: N r^2 / 2 multiply-adds and
-// no further barrier.  a is overwritten.
-// float and dfloat columns are first scaled by powers of two to a largest
-// entry in [1, 2) (Q does not change), so that the squares of graded columns
-// stay inside the FP32 exponent range; their dots are summed in runs of eight
-// rows.
-template <typename T, bool POS = false>
-__device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, T* a, int ld, T* qout, int ldq, T* R,
-                                int ldr, const QrSmem<T>& s) {
+// A reflector's column x below the pivot alpha: whether alpha^2 + x^T x (xn2 =
+// x^T x) is so small that squares have lost bits at the end of the type's
+// exponent range.  (Integer tests: an FP64 comparison in every thread would
+// show in every column.)
+__device__ __forceinline__ bool squares_lost(float alpha, float xn2) {
+  return fabsf(alpha) < 0x1p-50f && xn2 < 0x1p-100f;
+}
+__device__ __forceinline__ bool squares_lost(dfloat alpha, dfloat xn2) {
+  return fabsf(alpha.hi) < 0x1p-45f && xn2.hi < 0x1p-90f;
+}
+__device__ __forceinline__ bool squares_lost(double alpha, double xn2) {  // 2^-450, 2^-900
+  return (__double2hiint(alpha) & 0x7fffffff) < (1023 - 450) << 20 &&
+         (__double2hiint(xn2) & 0x7fffffff) < (1023 - 900) << 20;
+}
+// magnitude as an integer that grows with it, and the power of two that brings
+// it near 1 (0 for zero and for values that are not finite)
+__device__ __forceinline__ int size_key(float x) { return __float_as_int(x) & 0x7fffffff; }
+__device__ __forceinline__ int size_key(dfloat x) { return size_key(x.hi); }
+__device__ __forceinline__ int size_key(double x) { return __double2hiint(x) & 0x7fffffff; }
+template <typename T>
+__device__ __forceinline__ int scale_exponent(int key) {
+  constexpr bool F64 = std::is_same<T, double>::value;
+  constexpr int mant = F64 ? 20 : 23, bias = F64 ? 1023 : 127, most = F64 ? 1000 : 120;
+  if (key == 0 || key >= (2 * bias + 1) << mant) return 0;
+  return max(-most, min(most, bias - (key >> mant)));
+}
+
+// The dots of column k again (s.dots) with the column scaled by a power of two
+// from the largest entry over the cluster, pivot included; returns the
+// exponent (0: a zero column, nothing changed).  `slot` holds this column's
+// partial dots, `other` the next one's (free).  The same on every thread; ends
+// with a barrier.
+template <typename T>
+__device__ __noinline__ int rescaled_dots(const Team& tm, int rows, int r, T* a, int ld, int k, int i0, T alpha,
+                                          T* slot, T* other, const QrSmem<T>& s) {
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  T* x = a + k * ld;
+  int* wmax = reinterpret_cast<int*>(s.part);
+  int* all = reinterpret_cast<int*>(other);
+  int key = size_key(alpha);
+  for (int i = i0 + tid; i < rows; i += WT) key = max(key, size_key(x[i]));
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) key = max(key, __shfl_xor_sync(0xffffffffu, key, o));
+  if (lane == 0) wmax[warp] = key;
+  __syncthreads();
+  if (tid < tm.C) {
+#pragma unroll
+    for (int w = 0; w < WT / 32; ++w) key = max(key, wmax[w]);
+    tm.at(all, tid)[tm.q] = key;
+  }
+  tm.barrier();
+  key = all[0];
+  for (int c = 1; c < tm.C; ++c) key = max(key, all[c]);
+  const int up = scale_exponent<T>(key);
+  if (up != 0) {
+    const T f = two_to(T(0), up);
+    for (int i = i0 + tid; i < rows; i += WT) x[i] = x[i] * f;
+    __syncthreads();
+    for (int j = warp; j < r; j += WT / 32) {
+      T p = T(0);
+      for (int i = i0 + lane; i < rows; i += 32) p = fma(x[i], a[j * ld + i], p);
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) p += shfl_xor(p, o);
+      for (int c = lane; c < tm.C; c += 32) tm.at(slot, c)[tm.q * r + j] = p;
+    }
+  }
+  tm.barrier();
+  if (up != 0) {
+    if (tid < r) {
+      T p = slot[tid];
+      for (int c = 1; c < tm.C; ++c) p += slot[c * r + tid];
+      s.dots[tid] = p;
+    }
+    __syncthreads();
+  }
+  return up;
+}
+
+// The reflectors of the columns from k0 on.  A column whose squares leave the
+// exponent range (seen by the warp that forms the scalars, so that the others
+// read a flag beside them) ends the plain form, which returns it with nothing of
+// it changed; the safe form scales such columns.  Returns r at the end.
+template <typename T, bool POS, bool SAFE>
+__device__ __forceinline__ int qr_columns(const Team& tm, int lo, int rows, int r, T* a, int ld, T* R, int ldr,
+                                          const QrSmem<T>& s, int R0, int k0) {
   constexpr bool F64 = std::is_same<T, double>::value;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int LT = r + 1;
-  const int R0 = tm.rows_per(N);
   const int jw = r <= 8 ? 8 : (r <= 16 ? 16 : 32), ncls = WT / jw, cls = tid / jw;
-  const FastDiv by_rows(rows);
-  for (int e = tid; e < r * LT; e += WT) s.tri[e] = s.v1[e] = T(0);
-  if constexpr (!F64) {
-    // column maxima: warps take columns, every CTA learns all (slot 0 of both buffers)
-    for (int j = warp; j < r; j += WT / 32) {
-      float m = 0.0f;
-      for (int i = lane; i < rows; i += 32) m = fmaxf(m, fabsf(lead(a[j * ld + i])));
-#pragma unroll
-      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
-      for (int c = lane; c < tm.C; c += 32) tm.at(s.slot, c)[tm.q * r + j] = T(m);
-    }
-    tm.barrier();
-    if (tid < r) {
-      float m = 0.0f;
-      for (int c = 0; c < tm.C; ++c) m = fmaxf(m, lead(s.slot[c * r + tid]));
-      int e = 0;
-      if (m > 0.0f && m < 3.0e38f) frexpf(m, &e);
-      s.sgn[tid] = two_to(T(0), max(-120, min(120, 1 - e)));
-    }
-    __syncthreads();
-    for (int e = tid; e < rows * r; e += WT) {
-      const int k = by_rows.div(e), i = e - k * rows;
-      a[k * ld + i] = a[k * ld + i] * s.sgn[k];
-    }
-    tm.barrier();  // the slots are reused
-  } else {
-    __syncthreads();
-  }
-  for (int k = 0; k < r; ++k) {
+  for (int k = k0; k < r; ++k) {
     T* slot = s.slot + (k & 1) * tm.C * r;
     T* row = s.row + (k & 1) * r;
     T* x = a + k * ld;
@@ -366,8 +406,13 @@ __device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, 
       }
       __syncthreads();
     }
+    int up = 0;
+    if constexpr (SAFE) {
+      if (squares_lost(row[k], s.dots[k]))
+        up = rescaled_dots(tm, rows, r, a, ld, k, i0, row[k], slot, s.slot + ((k + 1) & 1) * tm.C * r, s);
+    }
     if (warp == 0) {
-      const T xn2 = s.dots[k], alpha = row[k];
+      const T xn2 = s.dots[k], alpha = SAFE && up ? row[k] * two_to(T(0), up) : row[k];
       T beta = alpha, tau = T(0), scal = T(0);
       if (xn2 > T(0)) {
         beta = -copysign(root(fma(alpha, alpha, xn2)), alpha);
@@ -383,13 +428,15 @@ __device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, 
         }
       }
       if (lane == 0) {
-        s.coef[0] = beta;
+        s.coef[0] = SAFE && up ? beta * two_to(T(0), -up) : beta;
         s.coef[1] = tau;
         s.coef[2] = scal;
+        if constexpr (!SAFE) s.coef[3] = squares_lost(alpha, xn2) ? T(1) : T(0);
         if constexpr (!F64) s.sgn[k] = (POS && lead(beta) < 0.0f) ? T(-1.0f) : T(1.0f);
       }
     }
     __syncthreads();
+    if (!SAFE && size_key(s.coef[3]) != 0) return k;
     const T beta = s.coef[0], tau = s.coef[1], scal = s.coef[2];
     // w_j (trailing columns) and z_j = -tau V_j^T v_k (earlier reflectors)
     if (tid < r) {
@@ -432,6 +479,67 @@ __device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, 
     }
     __syncthreads();
   }
+  return r;
+}
+
+// Householder QR (LAPACK signs; POS: a positive diagonal of R) of an N x r
+// panel whose rows [lo, lo + rows) are this CTA's a[k ld + i]; the explicit Q
+// goes to qout (ld ldq) and, when R is given, the factor to R (global, ld
+// ldr, zeros below; not with the scaled columns of the FP32-based types).  One
+// cluster barrier per column: a single pass forms x^T A for every column (the
+// trailing ones, and the earlier reflectors for the compact WY form), its
+// partials and the pivot row are pushed to every CTA, and every CTA derives
+// the reflector from the same sums.  Q = [I; 0] - V (T V1^T), T from those
+// products, replaces the backward accumulation: N r^2 / 2 multiply-adds and
+// no further barrier.  a is overwritten.
+// float and dfloat columns are first scaled by powers of two to a largest
+// entry in [1, 2) (Q does not change), so that the squares of graded columns
+// stay inside the FP32 exponent range; their dots are summed in runs of eight
+// rows.
+// The plain form is left at a column that it cannot take (see qr_columns), and
+// the safe one goes on from there.  Two functions without calls of their own:
+// with the scaling's call inside the plain one an FP64 ensemble's step took 5 %
+// longer (18.3 against 17.5 ms), like this 0.2 %.
+template <typename T, bool POS, bool SAFE>
+__device__ __forceinline__ int qr_form(const Team& tm, int N, int lo, int rows, int r, T* a, int ld, T* qout, int ldq,
+                                       T* R, int ldr, const QrSmem<T>& s, int k0) {
+  constexpr bool F64 = std::is_same<T, double>::value;
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int LT = r + 1;
+  const int R0 = tm.rows_per(N);
+  const FastDiv by_rows(rows);
+  if constexpr (!SAFE)
+    for (int e = tid; e < r * LT; e += WT) s.tri[e] = s.v1[e] = T(0);
+  if constexpr (SAFE) {
+    tm.barrier();  // every CTA is past its reads of column k0's partial dots
+  } else if constexpr (!F64) {
+    // column maxima: warps take columns, every CTA learns all (slot 0 of both buffers)
+    for (int j = warp; j < r; j += WT / 32) {
+      float m = 0.0f;
+      for (int i = lane; i < rows; i += 32) m = fmaxf(m, fabsf(lead(a[j * ld + i])));
+#pragma unroll
+      for (int o = 16; o > 0; o >>= 1) m = fmaxf(m, __shfl_xor_sync(0xffffffffu, m, o));
+      for (int c = lane; c < tm.C; c += 32) tm.at(s.slot, c)[tm.q * r + j] = T(m);
+    }
+    tm.barrier();
+    if (tid < r) {
+      float m = 0.0f;
+      for (int c = 0; c < tm.C; ++c) m = fmaxf(m, lead(s.slot[c * r + tid]));
+      int e = 0;
+      if (m > 0.0f && m < 3.0e38f) frexpf(m, &e);
+      s.sgn[tid] = two_to(T(0), max(-120, min(120, 1 - e)));
+    }
+    __syncthreads();
+    for (int e = tid; e < rows * r; e += WT) {
+      const int k = by_rows.div(e), i = e - k * rows;
+      a[k * ld + i] = a[k * ld + i] * s.sgn[k];
+    }
+    tm.barrier();  // the slots are reused
+  } else {
+    __syncthreads();
+  }
+  const int done = qr_columns<T, POS, SAFE>(tm, lo, rows, r, a, ld, R, ldr, s, R0, k0);
+  if (!SAFE && done < r) return done;
   // T: column k is T[:, 0:k] z_k (z_k sits in column k), diagonal tau; eight
   // lanes per row
   constexpr int TU = WR_MAX * 8 / WT;
@@ -508,6 +616,25 @@ __device__ __noinline__ void qr(const Team& tm, int N, int lo, int rows, int r, 
     }
   }
   __syncthreads();
+  return r;
+}
+
+template <typename T, bool POS>
+__device__ __noinline__ int qr_plain(const Team& tm, int N, int lo, int rows, int r, T* a, int ld, T* qout, int ldq,
+                                     T* R, int ldr, const QrSmem<T>& s) {
+  return qr_form<T, POS, false>(tm, N, lo, rows, r, a, ld, qout, ldq, R, ldr, s, 0);
+}
+template <typename T, bool POS>
+__device__ __noinline__ void qr_safe(const Team& tm, int N, int lo, int rows, int r, T* a, int ld, T* qout, int ldq,
+                                     T* R, int ldr, const QrSmem<T>& s, int k0) {
+  qr_form<T, POS, true>(tm, N, lo, rows, r, a, ld, qout, ldq, R, ldr, s, k0);
+}
+
+template <typename T, bool POS = false>
+__device__ __forceinline__ void qr(const Team& tm, int N, int lo, int rows, int r, T* a, int ld, T* qout, int ldq,
+                                   T* R, int ldr, const QrSmem<T>& s) {
+  const int done = qr_plain<T, POS>(tm, N, lo, rows, r, a, ld, qout, ldq, R, ldr, s);
+  if (done < r) qr_safe<T, POS>(tm, N, lo, rows, r, a, ld, qout, ldq, R, ldr, s, done);
 }
 
 }  // namespace wide
