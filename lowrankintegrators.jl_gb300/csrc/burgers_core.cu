@@ -19,11 +19,19 @@
 //                  distributed shared memory;
 //   s_core_update  sums the 16 cluster partials, applies the RK stage to the
 //                  FP64 core and writes the split of the next stage input.
+// An accumulator cuts what lies below its last bit at every addition, always
+// towards zero, so that a chain of K / 8 additions shortens its sum: the lo
+// parts go first (their cut is 2^-11 of the others'), and M1 has an
+// accumulator per chunk, G one for every other chunk and W' G one per chunk,
+// at most 4, 8 and 4 additions at the sum's size.  With one chain each (16, 16
+// and 12) the quadratic increment was short by 1e-6 of itself at rank 64 and
+// its error up to 16 % larger than that of FP64 sums (2.3e-6 against 2.0e-6
+// of it); now 4e-7 and 2.1e-6, for 0.25 ms of a 21.3 ms step.
 // At rank 64 the three took 12.0 + 14.1 + 4.6 us per stage (the panel form
 // 205 us: Khatri-Rao product 131, Uhat^T P2 23, five small products and
 // combines 51); with each kernel's prologue and constant operands loaded while
-// the one before it drains (programmatic dependent launch) a stage takes 25
-// us.
+// the one before it drains (programmatic dependent launch) a stage took 25
+// us, with the accumulators above 26.
 // What bounds them now: operand staging (256 KB per CTA through L2) and the
 // serial chain of two 128^3 products; the MMAs themselves take about 3.5 us.
 // Every mbarrier wait is bounded (ST_TIMEOUT); a CTA that gives up waits for
@@ -67,6 +75,31 @@ __device__ __forceinline__ void umma_tf32_ss(uint32_t d_tmem, uint64_t adesc, ui
       "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n}" ::"r"(d_tmem),
       "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
       : "memory");
+}
+
+// v = the sum of the accumulators at taddr, taddr + 128, ... (count of them, the
+// same in every thread of the warp)
+__device__ __forceinline__ void sum_blocks(uint32_t taddr, int count, float (&v)[16]) {
+  float w[16];
+#pragma unroll
+  for (int q = 0; q < 16; ++q) v[q] = 0.0f;
+  int j = 0;
+  if (count >= 2) {
+    tmem_ld16x2(taddr, taddr + 128u, v, w);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] += w[q];
+    j = 2;
+  }
+  if (j + 2 <= count) {
+    float u[16];
+    tmem_ld16x2(taddr + 256u, taddr + 384u, u, w);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] += u[q] + w[q];
+  } else if (j < count) {
+    tmem_ld16(taddr + 128u * j, w);
+#pragma unroll
+    for (int q = 0; q < 16; ++q) v[q] += w[q];
+  }
 }
 
 struct SGArgs {
@@ -122,7 +155,9 @@ __global__ void __launch_bounds__(SC_NT, 1)
   tc_fence_before();
   __syncthreads();
   tc_fence_after();
-  const uint32_t tmem = *tmem_slot;  // D main [0, 128), D correction [128, 256), A hi [256, 384), A lo [384, 512)
+  // M1: an accumulator per chunk, [128 j, 128 (j + 1)); then A hi [256, 384), A lo
+  // [384, 512) and two accumulators of G, [0, 128) and [128, 256)
+  const uint32_t tmem = *tmem_slot;
   const uint32_t idesc = idesc_tf32(SC_W, 32 * kch);
   auto zaddr = [&](int j, int lo) { return smem_u32(zt) + (uint32_t)(2 * j + lo) * SC_TILE; };
   auto taddr = [&](int j, int lo) { return smem_u32(tt) + (uint32_t)(2 * (j % SC_RING) + lo) * SC_TILE; };
@@ -145,15 +180,17 @@ __global__ void __launch_bounds__(SC_NT, 1)
     for (int j = 0; j < kch && ok; ++j) {
       if (!(ok = wait(full(j)))) break;
       tc_fence_after();
+      const uint32_t d = tmem + 128u * j;
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
         const uint64_t zh = sw128_desc(zaddr(j, 0) + 32u * kk), zl = sw128_desc(zaddr(j, 1) + 32u * kk);
         const uint64_t th = sw128_desc(taddr(j, 0) + 32u * kk), tl = sw128_desc(taddr(j, 1) + 32u * kk);
-        const uint32_t acc = (j > 0 || kk > 0) ? 1u : 0u;
-        umma_tf32_ss(tmem, zh, th, idesc, acc);
-        umma_tf32_ss(tmem + 128u, zh, tl, idesc, acc);
-        umma_tf32_ss(tmem + 128u, zl, th, idesc, 1u);
+        umma_tf32_ss(d, zh, tl, idesc, kk > 0 ? 1u : 0u);
+        umma_tf32_ss(d, zl, th, idesc, 1u);
       }
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)
+        umma_tf32_ss(d, sw128_desc(zaddr(j, 0) + 32u * kk), sw128_desc(taddr(j, 0) + 32u * kk), idesc, 1u);
       if (j == 0 && kch > SC_RING) umma_commit(empty0);
       if (j == 1 && kch > SC_RING) {  // the fourth chunk takes the first one's ring slot
         if (!(ok = wait(empty0))) break;
@@ -199,11 +236,10 @@ __global__ void __launch_bounds__(SC_NT, 1)
     for (int cc = 0; cc < 64; cc += 16) {
       const int col = 64 * g + cc;
       if (col < 32 * kch) {
-        float v[16], w[16], h[16], l[16];
-        tmem_ld16(tmem + lanes + (uint32_t)col, v);
-        tmem_ld16(tmem + lanes + 128u + (uint32_t)col, w);
+        float v[16], h[16], l[16];
+        sum_blocks(tmem + lanes + (uint32_t)col, kch, v);
 #pragma unroll
-        for (int q = 0; q < 16; ++q) split(v[q] + w[q], h[q], l[q]);
+        for (int q = 0; q < 16; ++q) split(v[q], h[q], l[q]);
         tmem_st16(tmem + lanes + 256u + (uint32_t)col, h);
         tmem_st16(tmem + lanes + 384u + (uint32_t)col, l);
       }
@@ -218,12 +254,15 @@ __global__ void __launch_bounds__(SC_NT, 1)
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
         const uint64_t zh = sw128_desc(zaddr(j, 0) + 32u * kk), zl = sw128_desc(zaddr(j, 1) + 32u * kk);
-        const uint32_t ah = tmem + 256u + (uint32_t)(32 * j + 8 * kk), al = ah + 128u;
-        const uint32_t acc = (j > 0 || kk > 0) ? 1u : 0u;
-        umma_tf32_ts(tmem, ah, zh, idesc, acc);
-        umma_tf32_ts(tmem + 128u, ah, zl, idesc, acc);
-        umma_tf32_ts(tmem + 128u, al, zh, idesc, 1u);
+        const uint32_t ah = tmem + 256u + (uint32_t)(32 * j + 8 * kk), al = ah + 128u, d = tmem + 128u * (j & 1);
+        umma_tf32_ts(d, ah, zl, idesc, (j > 1 || kk > 0) ? 1u : 0u);
+        umma_tf32_ts(d, al, zh, idesc, 1u);
       }
+    for (int j = 0; j < kch; ++j)
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)
+        umma_tf32_ts(tmem + 128u * (j & 1), tmem + 256u + (uint32_t)(32 * j + 8 * kk),
+                     sw128_desc(zaddr(j, 0) + 32u * kk), idesc, 1u);
     umma_commit(done2);
     mma2 = true;
   }
@@ -254,15 +293,14 @@ __global__ void __launch_bounds__(SC_NT, 1)
     for (int cc = 0; cc < 64; cc += 16) {
       const int col = 64 * g + cc;
       if (col < 32 * kch) {
-        float v[16], w[16];
-        tmem_ld16(tmem + lanes + (uint32_t)col, v);
-        tmem_ld16(tmem + lanes + 128u + (uint32_t)col, w);
+        float v[16];
+        sum_blocks(tmem + lanes + (uint32_t)col, min(kch, 2), v);
 #pragma unroll
         for (int q = 0; q < 16; ++q) {
           const int p = col + q;
           if (p <= row && row < ka) {
             float h, l;
-            split(v[q] + w[q], h, l);
+            split(v[q], h, l);
             const int o = sc_start(p, ka) + row - p;
             gh[o] = h;
             gl[o] = l;
@@ -314,7 +352,7 @@ __global__ void __launch_bounds__(SC_NT, 1) __cluster_dims__(SC_WG_CL, 1, 1)
   }
   if (warp == 0) {
     asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)),
-                 "r"(256u)
+                 "r"(512u)
                  : "memory");
     asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
   }
@@ -341,16 +379,17 @@ __global__ void __launch_bounds__(SC_NT, 1) __cluster_dims__(SC_WG_CL, 1, 1)
     for (int j = 0; j < nk && ok; ++j) {
       if (!(ok = wait(full(j)))) break;
       tc_fence_after();
-      const uint32_t s = st + (uint32_t)(4 * j) * SC_TILE;
+      const uint32_t s = st + (uint32_t)(4 * j) * SC_TILE, d = tmem + 128u * j;
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk) {
         const uint64_t wh = sw128_desc(s + 32u * kk), wl = sw128_desc(s + SC_TILE + 32u * kk);
         const uint64_t gh = sw128_desc(s + 2 * SC_TILE + 32u * kk), gl = sw128_desc(s + 3 * SC_TILE + 32u * kk);
-        const uint32_t acc = (j > 0 || kk > 0) ? 1u : 0u;
-        umma_tf32_ss(tmem, wh, gh, idesc, acc);
-        umma_tf32_ss(tmem + 128u, wh, gl, idesc, acc);
-        umma_tf32_ss(tmem + 128u, wl, gh, idesc, 1u);
+        umma_tf32_ss(d, wh, gl, idesc, kk > 0 ? 1u : 0u);
+        umma_tf32_ss(d, wl, gh, idesc, 1u);
       }
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)
+        umma_tf32_ss(d, sw128_desc(s + 32u * kk), sw128_desc(s + 2 * SC_TILE + 32u * kk), idesc, 1u);
     }
     umma_commit(done);
     if (*abort_flag) {
@@ -368,19 +407,16 @@ __global__ void __launch_bounds__(SC_NT, 1) __cluster_dims__(SC_WG_CL, 1, 1)
 #pragma unroll
   for (int cc = 0; cc < 64; cc += 16) {
     const int col = 64 * g + cc;
-    float v[16], w[16];
-    if (ok && nk > 0) {
-      tmem_ld16(tmem + lanes + (uint32_t)col, v);
-      tmem_ld16(tmem + lanes + 128u + (uint32_t)col, w);
-    }
+    float v[16];
+    sum_blocks(tmem + lanes + (uint32_t)col, ok ? nk : 0, v);
 #pragma unroll
-    for (int q = 0; q < 16; ++q) tile[(col + q) * SC_W + row] = (ok && nk > 0) ? v[q] + w[q] : 0.0f;
+    for (int q = 0; q < 16; ++q) tile[(col + q) * SC_W + row] = v[q];
   }
   tc_fence_before();
   cl.sync();
   if (warp == 0) {
     tc_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(256u) : "memory");
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
   // this CTA's sixteenth of the columns: the cluster's tiles in rank order
   const int per = SC_W * SC_W / SC_WG_CL / 4;  // float4 per CTA

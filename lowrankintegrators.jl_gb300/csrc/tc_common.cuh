@@ -151,6 +151,23 @@ __device__ __forceinline__ void tmem_ld16(uint32_t taddr, float (&v)[16]) {
   for (int q = 0; q < 16; ++q) v[q] = __uint_as_float(r[q]);
 }
 
+// two blocks of 16 columns behind one wait
+__device__ __forceinline__ void tmem_ld16x2(uint32_t t0, uint32_t t1, float (&v)[16], float (&w)[16]) {
+  asm volatile(
+      "{\n"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%0, %1, %2, %3, %4, %5, %6, %7, "
+      "%8, %9, %10, %11, %12, %13, %14, %15}, [%32];\n"
+      "tcgen05.ld.sync.aligned.32x32b.x16.b32 {%16, %17, %18, %19, %20, %21, %22, %23, "
+      "%24, %25, %26, %27, %28, %29, %30, %31}, [%33];\n"
+      "tcgen05.wait::ld.sync.aligned;\n}"
+      : "=f"(v[0]), "=f"(v[1]), "=f"(v[2]), "=f"(v[3]), "=f"(v[4]), "=f"(v[5]), "=f"(v[6]), "=f"(v[7]),
+        "=f"(v[8]), "=f"(v[9]), "=f"(v[10]), "=f"(v[11]), "=f"(v[12]), "=f"(v[13]), "=f"(v[14]), "=f"(v[15]),
+        "=f"(w[0]), "=f"(w[1]), "=f"(w[2]), "=f"(w[3]), "=f"(w[4]), "=f"(w[5]), "=f"(w[6]), "=f"(w[7]),
+        "=f"(w[8]), "=f"(w[9]), "=f"(w[10]), "=f"(w[11]), "=f"(w[12]), "=f"(w[13]), "=f"(w[14]), "=f"(w[15])
+      : "r"(t0), "r"(t1)
+      : "memory");
+}
+
 __device__ __forceinline__ void tmem_ld64(uint32_t taddr, float (&v)[64]) {
   asm volatile(
       "{\n"
