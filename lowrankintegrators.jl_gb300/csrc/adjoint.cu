@@ -690,7 +690,7 @@ __global__ void __launch_bounds__(WT, 1) adj_fwd(const __grid_constant__ AdjArgs
   double* wout = p1;
   for (int sub = 0; sub < sc.nsub; ++sub)
     for (int st = 0; st < sc.nstages; ++st) {
-      int big = full;
+      int big = full, reaches = 0;
       if (!full) {
         for (int e = tid; e < rows * r; e += WT) {
           const int k = by_rows.div(e), i = e - k * rows;
@@ -698,8 +698,9 @@ __global__ void __launch_bounds__(WT, 1) adj_fwd(const __grid_constant__ AdjArgs
           wout[k * ld + 1 + i] = tw;
           tf[e] = (float)tw;
           big |= !wide::below_2_100(tw);
+          reaches |= wide::reaches_2_m80(tw);
         }
-        big = __syncthreads_or(big);
+        big = wide::out_of_f32(big, reaches);
       }
       const bool last = st + 1 == sc.nstages, end = last && sub + 1 == sc.nsub;
       const double bs = sc.b[st], ha = last ? 0.0 : h * sc.a[st + 1];
@@ -1041,11 +1042,12 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
       load_rows_halo(s.Z + (int64_t)(sub * sc.nstages + st) * len, N, lo, rows, r, z, ld);
       __syncthreads();
       push_halos(tm, N, rows, r, kb, ld);
-      int zbig = full;
+      int zbig = full, zreaches = 0;
       for (int e = tid; e < rows * r; e += WT) {
         const int q = by_rows.div(e), o = q * ld + 1 + e - q * rows;
         p3[o] = T.mul(z, ld, e % rows, e / rows);
         zbig |= !wide::below_2_100(z[o]);
+        zreaches |= wide::reaches_2_m80(z[o]);
       }
       tm.cl.sync();
       outputs(2 * rr, rows, [&](int o, int l, int L) {
@@ -1056,7 +1058,7 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
         for (int i = 1 + l; i <= rows; i += L) v = fma(x[a * ld + i], y[c * ld + i], v);
         return v;
       }, [&](int o, double v) { part[o] += v; });
-      zbig = __syncthreads_or(zbig);  // T z is consumed
+      zbig = wide::out_of_f32(zbig, zreaches);  // T z is consumed
       if (s.kside) {
         for (int e = tid; e < rows * r; e += WT) {
           const int c = by_rows.div(e), i = e - c * rows;
@@ -1079,7 +1081,7 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
         }, [&](int i, double v) { s.thb[lo + i] += v; });
         __syncthreads();
       }
-      int big = full;
+      int big = full, reaches = 0;
       if (!full) {
         for (int e = tid; e < rows * r; e += WT) {
           const int k = by_rows.div(e), i = e - k * rows;
@@ -1087,8 +1089,9 @@ __global__ void __launch_bounds__(WT, 1) adj_rev(const __grid_constant__ AdjArgs
           p3[k * ld + 1 + i] = tk;
           tf[e] = (float)tk;
           big |= !wide::below_2_100(tk);
+          reaches |= wide::reaches_2_m80(tk);
         }
-        big = __syncthreads_or(big);
+        big = wide::out_of_f32(big, reaches);
       }
       for (int e = tid; e < rows * r; e += WT) {
         const int c = by_rows.div(e), i = e - c * rows, o = c * ld + 1 + i;

@@ -191,8 +191,8 @@ __global__ void __launch_bounds__(WT, 2)
       Es[e] = (float)ev;
       if (!(fabs(ev) <= 0x1p-36)) full = 1;  // NaN included
     }
-    // (T w) G = T w + (T w) E with E applied in FP32 while max|E| <= 2^-36 (its
-    // rounding stays below 2^-54 of T w), else the full product
+    // (T w) G = T w + (T w) E with E applied in FP32 (see below_2_100), or the
+    // full product
     full = __syncthreads_or(full);
     tm.cl.sync();  // the zero halo rows of every CTA are set
     push_halos(tm, N, rows, r, win, ldr);
@@ -203,7 +203,7 @@ __global__ void __launch_bounds__(WT, 2)
       double hw = h * sc.gam[sc.nstages];
       for (int j = sc.nstages - 1; j >= 0; --j) {
         const double gj = (j == 0) ? 1.0 : sc.gam[j];
-        int big = full;
+        int big = full, reaches = 0;
         if (!full) {
           // T w into this thread's own entries of wout, its FP32 copy for the row
           for (int e = tid; e < rows * r; e += WT) {
@@ -212,8 +212,9 @@ __global__ void __launch_bounds__(WT, 2)
             wout[k * ldr + 1 + i] = tw;
             tf[e] = (float)tw;
             big |= !wide::below_2_100(tw);
+            reaches |= wide::reaches_2_m80(tw);
           }
-          big = __syncthreads_or(big);
+          big = wide::out_of_f32(big, reaches);
         }
         for (int e = tid; e < rows * r; e += WT) {
           const int c = by_rows.div(e), i = e - c * rows;

@@ -134,8 +134,25 @@ __device__ __forceinline__ void outputs(int nout, int K, const F& f, const D& do
   }
 }
 
-// |x| < 2^100 without an FP64 instruction (false for NaN)
+// The products with a Gram matrix G = I + E: Y G = Y + Y E, with Y E on the FP32
+// pipe while max |E| <= 2^-36.  That adds at most 2^-60 of a row's largest entry
+// to each of its entries, where the rounding of G's own entries (sums over the
+// rows of two bases, 2^-53 each) acts on them in the same way in the full
+// product: errors against 64-bit results are the same in both forms
+// (geometric means over 30 problems: FP64 ensembles 7.02e-16 and 7.05e-16 with
+// the full product, gradients 1.78e-15 and 1.85e-15).  The FP32 range allows it
+// for panels whose entries all stay below 2^100 and of which one reaches 2^-80
+// (what falls under the range is then below 2^-64 of it); the others take
+// the full product.  Both tests without an FP64 instruction, false for NaN.
 __device__ __forceinline__ bool below_2_100(double x) { return (__double2hiint(x) & 0x7fffffff) < 0x46300000; }
+__device__ __forceinline__ bool reaches_2_m80(double x) {
+  return (unsigned)((__double2hiint(x) & 0x7fffffff) - ((1023 - 80) << 20)) < (unsigned)(0x7ff00000 - ((1023 - 80) << 20));
+}
+// whether the full product is needed: a value too large anywhere in the CTA, or
+// none of size (all threads; a barrier)
+__device__ __forceinline__ bool out_of_f32(int big, int reaches) {
+  return __syncthreads_or(big) || !__syncthreads_or(reaches);
+}
 
 // Adds every CTA's part[0 .. len) (shared memory, the same address in every
 // CTA): done(e, sum) runs for each e on one CTA.  The terms are added in

@@ -67,3 +67,48 @@ def test_rank_adaptive_small_remainders(lri, precision, small, tol):
     assert y.S.shape == (2 * r, 2 * r)
     for X in (y.U, y.V):
         assert np.abs(X.T @ X - np.eye(2 * r)).max() <= tol
+
+
+# Bases that are orthonormal to a few 1e-12 only: their Gram matrices' last bits
+# count, also where the panels' entries lie below the FP32 range.
+def nearly_orthonormal(g, X):
+    return X @ (np.eye(X.shape[1]) + 1.5e-12 * g.standard_normal((X.shape[1], X.shape[1])))
+
+
+@pytest.mark.parametrize("n,m,r", [(40, 36, 4), (300, 257, 16), (70, 300, 33)])
+@pytest.mark.parametrize("power", [-90, -150, -300])
+def test_gram_terms_of_small_panels(lri, n, m, r, power):
+    A, B, U, S, V = instance(n + r, n, m, r)
+    g = np.random.default_rng(1)
+    U, V = nearly_orthonormal(g, U), nearly_orthonormal(g, V)
+
+    def run(scale):
+        prob = lri.MatrixDEProblem(lri.SylvesterTridiagOperator(A, B),
+                                   lri.SVDLikeRepresentation(U, S * scale, V), (0.0, 0.1))
+        return lri.solve(prob, lri.UnconventionalAlgorithm(lri.RK4(1)), 0.1).Y[-1]
+
+    scale = 2.0 ** power
+    y, ref = run(scale), run(1.0)
+    # FP64 rounding at condition 2^(r/4) <= 2^8; without E the bases move by 1e-13 and more
+    for a, b in ((y.U, ref.U), (y.S / scale, ref.S), (y.V, ref.V)):
+        assert np.linalg.norm(a - b) <= 2e-14 * 2 ** (r / 8) * np.linalg.norm(b)
+
+
+@pytest.mark.parametrize("n,m,r", [(40, 36, 4), (300, 257, 16)])
+@pytest.mark.parametrize("power", [-90, -150])
+def test_gradients_of_small_panels(lri, n, m, r, power):
+    A, B, U, S, V = instance(n + r, n, m, r)
+    g = np.random.default_rng(1)
+    U, V = nearly_orthonormal(g, U), nearly_orthonormal(g, V)
+    P, Q = (np.linalg.qr(g.standard_normal((k, 5)))[0] for k in (n, m))
+    D = np.diag(2.0 ** -np.arange(5.0))
+
+    def run(scale):
+        prob = lri.MatrixDEProblem(lri.SylvesterTridiagOperator(A, B),
+                                   lri.SVDLikeRepresentation(U, S * scale, V), (0.0, 0.1))
+        _, theta, b = lri.bug_gradient(prob, lri.UnconventionalAlgorithm(lri.RK4(1)), 0.1,
+                                       lri.SVDLikeRepresentation(P, D * scale, Q))
+        return theta / scale ** 2, b.U / scale ** 2, b.S / scale, b.V / scale ** 2
+
+    for a, b in zip(run(2.0 ** power), run(1.0)):
+        assert np.linalg.norm(a - b) <= 2e-13 * 2 ** (r / 8) * np.linalg.norm(b)
