@@ -455,7 +455,8 @@ class Batch:
         for k in self._sizes:
             self._starts.append(self._starts[-1] + -(-k // al) * al)
         self._flat = torch.zeros(self._starts[-1], dtype=self.dtype, device=dev)
-        self.U, self.S, self.V, self.opA, self.opB = self._split(self._flat)
+        self._parts = self._split(self._flat)
+        self.U, self.S, self.V, self.opA, self.opB = self._parts
         self._stage = None
         self.offY = None
         self.has_data = op_kind == _native.LRI_OP_DATA or isinstance(alg, GreedyIntegrator)
@@ -517,7 +518,13 @@ class Batch:
                 hA[self.offA[i]:self.offA[i] + len(a)] = a
                 hB[self.offB[i]:self.offB[i] + len(b)] = b
             end = self._starts[5]
-        self._flat[:end].copy_(t.from_numpy(flat[:end]))
+        mine = (self.U, self.S, self.V, self.opA, self.opB)
+        if all(x is y for x, y in zip(mine, self._parts)):
+            self._flat[:end].copy_(t.from_numpy(flat[:end]))
+        else:  # buffers that the caller put in their place
+            for x, part, start in zip(mine, parts, self._starts):
+                if start < end:
+                    x.zero_()[:part.size].copy_(t.from_numpy(part))
         if operators is not None and self.op_kind in (_native.LRI_OP_BURGERS_PERIODIC, _native.LRI_OP_LOCAL_FLOW):
             hB = np.zeros(int(self.opB.numel()), self.np_dtype)
             for i, op in enumerate(operators):
