@@ -488,6 +488,13 @@ int wide_cluster(int count, int64_t tall, int sms) {
 // where the batch leaves SMs idle, larger clusters, down to four rows per CTA
 // (below that the barriers outweigh the split).  Cores: a cluster only where
 // SMs are idle.
+// There is no rule by cost: FP64 issue bounds either form and the panels' way
+// through L2 hides no other work, so sides win wherever they fit.  Per step,
+// step kernel against sides: n, m 256 to 1024 with r 23 to 32, 350: 20.5, 12.6 ms;
+// 700: 30.0, 25.7; 1400: 53.7, 49.9; n, m to 512 with r 4 to 24, 1000: 8.5, 4.5; n, m
+// 40 to 100 with r 2 to 6, 4000: 3.6, 1.2; data instances of 100 to 512 with r 4 to
+// 32, 64: 11.4, 3.5; 256: 13.7, 9.9; 1024: 24.3, 21.2; of 40 to 80 with r 2 to 8,
+// 4000: 5.3, 1.8; of 1000 to 2000 with r 8 to 32, 20: 144, 25.
 bool wide_plan(WidePlan* w, int count, const int64_t* n, const int64_t* m, const int64_t* r, bool data, int sms,
                std::vector<int32_t>* items) {
   std::vector<SideItem> v;

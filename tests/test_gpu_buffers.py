@@ -41,3 +41,43 @@ def test_upload_into_replaced_buffers(lri, names, precision):
         assert not x.any()
     ref.close()
     b.close()
+
+
+@pytest.mark.parametrize("how", ["no page-locked memory", "too large to stage"])
+def test_snapshots_from_pageable_memory(lri, how, monkeypatch):
+    import torch
+    g = np.random.default_rng(6)
+    n, m, r = 45, 37, 5
+    data = [g.standard_normal((n, m)) for _ in range(4)]
+    U, s, Vt = np.linalg.svd(data[0], full_matrices=False)
+    Y0 = lri.SVDLikeRepresentation(U[:, :r], np.diag(s[:r]), Vt[:r].T)
+
+    def run():
+        b = lri.Batch([n], [m], [r], lri.UnconventionalAlgorithm(lri.RK4(1)), lri._native.LRI_OP_DATA, "fp64")
+        b.upload([Y0])
+        b.data_init([data[0]])
+        for k in (1, 2, 3):
+            mine = data[k].copy()
+            b.step(0.0, 1.0, 1, [mine] if k % 2 else mine.ravel(order="F"))
+            mine[:] = np.nan
+        y = b.download()[0]
+        staged = bool(b._stage)
+        b.close()
+        return y, staged
+
+    ref, staged = run()
+    assert staged
+    if how == "too large to stage":
+        monkeypatch.setattr(lri.Batch, "STAGE_BYTES", 8 * n * m - 1)
+    else:
+        zeros = torch.zeros
+
+        def refuse(*args, pin_memory=False, **kw):
+            if pin_memory:
+                raise RuntimeError("CUDA error: out of memory")
+            return zeros(*args, **kw)
+
+        monkeypatch.setattr(torch, "zeros", refuse)
+    y, staged = run()
+    assert not staged
+    assert np.array_equal(y.U, ref.U) and np.array_equal(y.S, ref.S) and np.array_equal(y.V, ref.V)
