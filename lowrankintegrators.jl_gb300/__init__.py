@@ -472,7 +472,12 @@ class Batch:
     # -- helpers -----------------------------------------------------------
     def _stream(self):
         t = self.torch
-        return C.c_void_p(t._C._cuda_getCurrentRawStream(t.cuda.current_device()))
+        # 0.3 us against 2.9 through a Stream object, in every call of a step
+        # loop; not a public function, so it may be missing
+        raw = getattr(t._C, "_cuda_getCurrentRawStream", None)
+        if raw is None:
+            return C.c_void_p(t.cuda.current_stream().cuda_stream)
+        return C.c_void_p(raw(t.cuda.current_device()))
 
     def close(self):
         if getattr(self, "handle", None) is not None and self.handle.value:

@@ -81,3 +81,14 @@ def test_snapshots_from_pageable_memory(lri, how, monkeypatch):
     y, staged = run()
     assert not staged
     assert np.array_equal(y.U, ref.U) and np.array_equal(y.S, ref.S) and np.array_equal(y.V, ref.V)
+
+
+def test_stream_without_the_raw_lookup(lri, monkeypatch):
+    import torch
+    b = lri.Batch([20], [20], [2], lri.UnconventionalAlgorithm(lri.RK4(1)), lri._native.LRI_OP_ZERO, "fp64")
+    st = torch.cuda.Stream()
+    with torch.cuda.stream(st):
+        assert b._stream().value == st.cuda_stream
+        monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
+        assert b._stream().value == st.cuda_stream
+    b.close()
