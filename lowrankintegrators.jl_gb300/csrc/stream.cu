@@ -1627,6 +1627,7 @@ struct lri_stream {
   void* th = nullptr;
   void* tw = nullptr;   // W' of Uhat (the S flow on the core)
   void* kgp = nullptr;  // split partials of the tensor sums (ceil(max(n, m) / KR_ROWS) x PP x 2R) and of gram_act
+  // (kap, kap2nd, pw2: only where a flow can take the per-stage form with them)
   void* kap = nullptr;  // pair-split partials of the Khatri-Rao products: 2 x kZmax x max(n, m) x 2R
   void* pw = nullptr;   // 3 work panels of max(n, m) x 2R
   void* pw2 = nullptr;     // the side stream's L-flow product panel, max(n, m) x 2R
@@ -2376,10 +2377,7 @@ lri_status lri_burgers_create(lri_stream** out, int32_t dtype, int64_t n, int64_
   // (also the split partials of the S substep's Gram: ceil(n / GA_ROWS) x (2R)^2 FP64)
   alloc(&s->kgp, std::max<int64_t>(s->es * ((nm + KR_ROWS - 1) / KR_ROWS) * PP * 2 * R,
                                    (int64_t)sizeof(double) * ((n + GA_ROWS - 1) / GA_ROWS) * 4 * R * R));
-  alloc(&s->kap, s->es * 2 * kZmax * nm * 2 * R);
   alloc(&s->pw, s->es * 3 * nm * 2 * R);
-  alloc(&s->pw2, s->es * nm * 2 * R);
-  alloc(&s->kap2nd, s->es * kZmax * nm * 2 * R);
   if (e == cudaSuccess && dtype == LRI_F32 && 2 * R > lri::FLOW_KMAX && lri::s_core_supported((int)R)) {
     e = lri::s_core_init(&s->score, (int)R);
     s->core_ok = (e == cudaSuccess);
@@ -2390,6 +2388,16 @@ lri_status lri_burgers_create(lri_stream** out, int32_t dtype, int64_t n, int64_
     e = lri::panel_flow_init(&s->panel);
     s->panel_ok = (e == cudaSuccess);
   }
+  // Buffers of the flows that run one launch per stage: FP64 engines, engines
+  // without a quadratic term, and FP32 ones without the driver's tensor-map
+  // encoder, above the ranks of the flow kernels (n = 4096, m = 16384, r_max =
+  // 64: 210 MB that the other engines do without)
+  const bool nonlin = alpha != 0.0 || beta != 0.0;
+  const bool kl_stages = R > lri::FLOW_KMAX && !(s->panel_ok && nonlin);
+  const bool s_stages = 2 * R > lri::FLOW_KMAX && !(s->core_ok && nonlin);
+  if (nonlin && (kl_stages || s_stages)) alloc(&s->kap, s->es * 2 * kZmax * nm * 2 * R);
+  if (nonlin && kl_stages) alloc(&s->kap2nd, s->es * kZmax * nm * 2 * R);
+  if (kl_stages) alloc(&s->pw2, s->es * nm * 2 * R);
   if (e != cudaSuccess) {
     lri_stream_destroy(s);
     *out = nullptr;
