@@ -548,12 +548,15 @@ class Batch:
         return self._pack_data_into(snapshots, np.zeros(self.totY, self.np_dtype))
 
     def _pack_data_into(self, snapshots, h):
+        end = 0
         for i, Y in enumerate(snapshots):
             n, m = int(self.n[i]), int(self.m[i])
             Y = np.asarray(Y)
             if Y.shape != (n, m):
                 raise ValueError(f"instance {i}: snapshot shape {Y.shape} != {(n, m)}")
-            h[self.offY[i]:self.offY[i] + n * m].reshape((n, m), order="F")[...] = Y
+            end = int(self.offY[i]) + n * m
+            h[end - n * m:end].reshape((n, m), order="F")[...] = Y
+        h[end:] = 0  # instances without a snapshot (the buffer holds an earlier one)
         return h
 
     # Snapshots up to this size are staged in page-locked memory (two of them

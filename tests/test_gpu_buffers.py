@@ -92,3 +92,27 @@ def test_stream_without_the_raw_lookup(lri, monkeypatch):
         monkeypatch.delattr(torch._C, "_cuda_getCurrentRawStream")
         assert b._stream().value == st.cuda_stream
     b.close()
+
+
+def test_instances_without_a_snapshot_see_zeros(lri):
+    """A list shorter than the batch: zeros for the rest, in every step."""
+    g = np.random.default_rng(8)
+    shapes = [(33, 31, 3), (20, 24, 2)]
+    data = [[g.standard_normal(s[:2]) for s in shapes] for _ in range(5)]
+    Y0 = [lri.SVDLikeRepresentation(*(lambda U, s, Vt, r: (U[:, :r], np.diag(s[:r]), Vt[:r].T))(
+        *np.linalg.svd(Y, full_matrices=False), r)) for Y, (_, _, r) in zip(data[0], shapes)]
+
+    def run(last):
+        b = lri.Batch(*(list(x) for x in zip(*shapes)), lri.UnconventionalAlgorithm(lri.RK4(1)),
+                      lri._native.LRI_OP_DATA, "fp64")
+        b.upload(Y0)
+        b.data_init(data[0])
+        for k in (1, 2, 3):
+            b.step(0.0, 1.0, 1, data[k])
+        b.step(0.0, 1.0, 1, last)
+        y = b.download()[1]
+        b.close()
+        return y
+
+    y, ref = run(data[4][:1]), run([data[4][0], np.zeros(shapes[1][:2])])
+    assert np.array_equal(y.U, ref.U) and np.array_equal(y.S, ref.S) and np.array_equal(y.V, ref.V)
