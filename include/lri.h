@@ -209,7 +209,9 @@ LRI_API lri_status lri_batch_prepare(lri_batch* b, double dt, int32_t nsteps);
 /* Register budget of the batch's step kernel, the autotuner's knob for the
  * instance engine: 3 CTAs per SM (at most 80 registers per thread; the
  * default) or 2 (at most 128 registers: fewer spills, less latency hiding).
- * FP64 batches take 3 only.  No counterpart in the reference. */
+ * FP64 batches take 3 only, and double-float BUG batches that run by sides
+ * (lri_batch_launches_per_step above 4) take either without an effect.  No
+ * counterpart in the reference. */
 LRI_API lri_status lri_batch_set_occupancy(lri_batch* b, int32_t ctas_per_sm);
 
 /* Current ranks (host array of length count; synchronises the stream). */
@@ -224,8 +226,9 @@ LRI_API lri_status lri_batch_status(lri_batch* b, void* stream);
  * allocator, or their time loop must not trigger the device-wide
  * synchronisation of cudaMalloc/cudaFree - this advances ONE instance of
  * F(X) = A X + X B^T (tridiagonal A, B as in LRI_OP_SYLVESTER_TRIDIAG) by
- * nsteps BUG steps with the step kernel of lri_batch_step, using a fixed
- * 4 MiB scratch array compiled into the library (held by every GPU that loads
+ * nsteps BUG steps with the one-CTA-per-instance step kernel (FP64 batches of
+ * lri_batch_step run by sides where those fit, so the two differ by the order
+ * of their sums), using a fixed 4 MiB scratch array compiled into the library (held by every GPU that loads
  * it until the process exits) instead of allocated workspace.
  *   dtype   LRI_F64 or LRI_F32 (LRI_DF: LRI_ERR_UNSUPPORTED)
  *   U (n x r), S (r x r), V (m x r)  caller's device buffers, column-major,
@@ -264,10 +267,13 @@ LRI_API lri_status lri_bug_step_noalloc(int32_t dtype, int64_t n, int64_t m, int
  *                   accumulates d loss / d theta
  * Each instance recomputes its step in stage form (RK stage inputs, both
  * QRs, basis changes, projections, S stages) and sweeps back through it;
- * the thin-QR adjoint is (Q_bar + Q copyltu(-Q_bar^T Q)) R^{-T}.  While
- * twice the instance count fits the device's SMs, each instance runs on a
- * 2-CTA thread-block cluster (the K side on one SM, the L side on another);
- * larger batches take one CTA per instance.  The
+ * the thin-QR adjoint is (Q_bar + Q copyltu(-Q_bar^T Q)) R^{-T}.  Batches
+ * that leave SMs idle take a step in four launches, each side of an instance
+ * (and its core) on a thread-block cluster of 2 to 16 CTAs: the largest size
+ * that gives two clusters per instance SMs of their own and every CTA at least
+ * four rows.  Batches with more instances than that, or with panels that do not
+ * fit the cluster's shared memory, take one kernel: a 2-CTA cluster per
+ * instance while twice the count fits the SMs, else one CTA.  The
  * workspace comes from lri_batch_adjoint_prepare (LRI_ERR_STATE without it);
  * the step allocates nothing.  Schemes with nstages * nsub > 16 and other
  * batch kinds return LRI_ERR_UNSUPPORTED. */

@@ -628,7 +628,9 @@ class Batch:
 
     def apply_tuning(self, table=None):
         """Takes the tuned register budget of this batch's precision and
-        dominant rank bucket (``tuning.json``); returns what was chosen."""
+        dominant rank bucket (``tuning.json``); returns what was chosen.  It
+        acts on the step kernel: double-float BUG batches that run by sides
+        take and report it without an effect."""
         ctas, bucket = _tuning.ensemble_occupancy(self.precision, self.n, self.m, self.rcap, table)
         if self.precision != "fp64":
             self.set_occupancy(ctas)

@@ -5,8 +5,8 @@ double-float engines sized for two CTAs per SM, the FP64 steps of small batches
 on clusters, the BUG steps by sides, host C ABI,
 the allocation-free entry point, the discrete adjoint, the large-stream
 engine, its tensor-core snapshot passes, its cluster core SVD, the large
-Burgers engine's tensor-core Khatri-Rao products and its flow kernels
-and tensor-core S flow) compile in parallel with nvcc and
+Burgers engine's flow kernels, its tensor-core panel flows and its
+tensor-core S flow) compile in parallel with nvcc and
 link into one shared library.  The library is rebuilt
 when a source or the public header is newer than it.
 """

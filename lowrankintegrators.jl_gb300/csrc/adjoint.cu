@@ -518,8 +518,8 @@ __global__ void __launch_bounds__(NT, 3) adjoint_step_kernel(AdjArgs g) {
 // launches, the phases above.  adj_fwd, adj_rev and adj_out give each side of
 // an instance a cluster whose CTAs split its rows (panels in shared memory,
 // the stage inputs in the workspace); adj_core splits the core's entries over
-// one cluster.  The products (T z) G use G = I + E with E applied in FP32
-// while max|E| <= 2^-36, as the forward steps do.  One reverse step at n = m =
+// one cluster.  The products with a Gram matrix take its FP32 form where the
+// forward steps do (below_2_100 in wide.cuh).  One reverse step at n = m =
 // 2048, r = 32: 37.0 ms on a 2-CTA pair, 2.0 ms here (adj_fwd 0.63, adj_core
 // 0.18, adj_rev 1.02, adj_out 0.15), bound by FP64 issue on 32 SMs.
 // ---------------------------------------------------------------------------

@@ -596,9 +596,10 @@ lri_status lri_batch_set_occupancy(lri_batch* b, int32_t ctas_per_sm) {
 
 int32_t lri_batch_launches_per_step(const lri_batch* b) {
   if (!b) return 0;
-  // one engine launch; double-float batches add the three write-back
-  // conversions (and one snapshot conversion for data problems) per call
-  const int step = b->sides().nclass ? b->sides().nclass + 1 : 1;  // the sides' classes, then the core
+  // one launch of the step kernel, or one per class of sides and one of the
+  // cores; double-float batches add the three write-back conversions (and one
+  // snapshot conversion for data problems) per call
+  const int step = b->sides().nclass ? b->sides().nclass + 1 : 1;
   if (b->desc.dtype == LRI_DF) return step + 3 + (b->totY > 0 ? 1 : 0);
   return step;
 }

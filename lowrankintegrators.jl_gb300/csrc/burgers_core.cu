@@ -418,7 +418,7 @@ __global__ void __launch_bounds__(SC_NT, 1) __cluster_dims__(SC_WG_CL, 1, 1)
     tc_fence_after();
     asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem), "r"(512u) : "memory");
   }
-  // this CTA's sixteenth of the columns: the cluster's tiles in rank order
+  // this CTA's eighth of the columns: the cluster's tiles in rank order
   const int per = SC_W * SC_W / SC_WG_CL / 4;  // float4 per CTA
   float4* dst = reinterpret_cast<float4*>(part) + (int64_t)(blockIdx.x / SC_WG_CL) * (SC_W * SC_W / 4);
   for (int e = tid; e < per; e += SC_NT) {

@@ -2,7 +2,7 @@
 // of a side in shared memory.
 //
 // A step is two launches: sides_kernel takes every (instance, side) pair - the
-// K and L steps read only the old factors - and core_kernel (engine_impl.cuh)
+// K and L steps read only the old factors - and core_kernel (engine_df.cu)
 // every instance's S step.  A side runs on one CTA, or on a cluster of 2 to 16
 // CTAs that split its rows where its three panels would not leave room for
 // two CTAs on an SM.  The work is grouped into classes by cluster size and

@@ -14,7 +14,7 @@
 //   wide_core   one cluster per instance: S~0 = M S0 N^T and the S step, the
 //               core's columns split over the CTAs.
 // One instance, per step: 256 x 256, r = 8, 20 RK4 substeps 1056 us on a 2-CTA
-// pair, 270 us here (sides 161, core 109; what is left are the 160 dependent
+// pair, 275 us here (sides 165, core 109; what is left are the 160 dependent
 // stages' barriers and FP64 chains); 2048 x 2048, r = 32, 12.0 ms against 0.57
 // ms (FP64 issue on 32 SMs); a 100 x 100 data step, r = 12, 754 us on one CTA,
 // 86 us here.

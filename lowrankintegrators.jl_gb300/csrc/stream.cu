@@ -982,9 +982,11 @@ __device__ __forceinline__ void pair_ab(int p, int ka, int& a, int& b) {
 // A CTA takes 16 TU pairs x 16 TV columns, TU x TV of them per thread: 128 x 128
 // for the widest panels, where forming the products and reading both
 // operands from shared memory would otherwise bound it.  The stores into
-// the chunk take 8 rows x 4 pairs per warp (a row stride of 4 banks: no
-// conflicts; 64-wide tiles with rows across the lanes had 32-way ones).  At
-// m = 16384: 128 columns 2.70 -> 1.21 ms, 64 columns 0.39 -> 0.21 ms.
+// the chunk take 8 rows x 4 pairs per warp (FP32: a row stride of 4 banks, no
+// conflicts, where 64-wide tiles with rows across the lanes had 32-way ones;
+// FP64: a stride of 8 banks, two-way ones beside FP64 multiply-adds at 1/64 of
+// the FP32 rate).  FP32, m = 16384: 128 columns 2.70 -> 1.21 ms, 64 columns
+// 0.39 -> 0.21 ms.
 template <typename T, int TU, int TV>
 __global__ void __launch_bounds__(256) kr_gram_part(int N, int R, int aug, const int32_t* __restrict__ rank,
                                                      const T* __restrict__ P, const T* __restrict__ Q,
@@ -1929,7 +1931,6 @@ struct StreamOps {
                      [&](const StreamOps<T>& o) { return side(o, m, tp(s->Xl), V, tp(s->Vh), blk(4)); });
   }
 
-  // TF32 split of flow tensor k for the tensor-core products
   // the whole L substep flow (Lp holds L0 and its RK panels): one launch, or
   // (FP64 above rank FLOW_KMAX, or no quadratic term) per stage the product
   // panel, the Khatri-Rao partials and the combine (with the side stream's

@@ -263,7 +263,8 @@ __device__ __forceinline__ float lead(double x) { return (float)x; }
 // Square root and reciprocal of the reflector's scalars.  FP64: Newton steps
 // from the FP32 estimates (about 12 and 5 FP64 instructions, where the library
 // calls take some 25 and 12; one warp's chain of them is on the critical path
-// of every column), within the FP32 exponent range, else the library's.
+// of every column), within the FP32 exponent range, else the library's.  At
+// most one unit in the last place from the correctly rounded values.
 __device__ __forceinline__ float root(float x) { return sqrtf(x); }
 __device__ __forceinline__ dfloat root(dfloat x) { return lri_df::sqrt(x); }
 __device__ __forceinline__ double root(double x) {
